@@ -69,12 +69,14 @@ typedef struct rtg_progress {
  * device counters behind the roofline figures. */
 typedef struct rtg_stats {
   uint64_t camera_samples, rays, shadow_rays, rr_terminated, invalid_samples, passes;
-  uint64_t iterations, node_visits, prim_tests, sphere_tests, extend_launches; /* closest-hit kernel */
+  uint64_t iterations, node_visits, prim_tests, sphere_tests, extend_launches; /* closest-hit walks */
   uint64_t shadow_node_visits, shadow_prim_tests, shadow_sphere_tests;         /* any-hit kernel */
   uint64_t kernel_launches; /* every kernel of this library launched by the render */
   double elapsed_ms;        /* host wall time of the render call */
   double device_ms;         /* CUDA-event time on the context's stream, first to last launch */
-  double extend_ms, shade_ms, shadow_ms, accumulate_ms, direct_ms; /* per-kernel event time (time_kernels) */
+  /* Per-kernel event time (time_kernels). extend_ms is the path kernel's, which shades and traces
+   * shadow rays too; shade_ms and shadow_ms stay 0. */
+  double extend_ms, shade_ms, shadow_ms, accumulate_ms, direct_ms;
   double plan_ms;           /* generation-plan kernel (time_kernels) */
 } rtg_stats;
 
@@ -300,10 +302,12 @@ int rtg_probe_read_bandwidth(rtg_context* ctx, uint64_t bytes, int32_t reps, int
 
 /* ---- engine tuning (no reference counterpart) ---- */
 typedef struct rtg_tuning {
-  uint32_t pool_paths;       /* wavefront path slots (default 1 << 20) */
-  uint32_t block;            /* threads per block of the wavefront kernels: 64, 128, 256 */
+  uint32_t pool_paths;       /* paths of one wavefront iteration while requests are open; a render's
+                              * iterations take four times as many (default 1 << 20) */
+  uint32_t block;            /* threads per block of the path kernel: 64, 128, 256 */
   uint64_t max_pass_samples; /* radiance slots shared by all passes in flight (default 1 << 27) */
-  int32_t extend_blocks, shade_blocks, shadow_blocks; /* 0 = occupancy-derived persistent grid */
+  int32_t extend_blocks; /* grid of the path kernel; 0 = every resident block */
+  int32_t shade_blocks, shadow_blocks; /* accepted, without effect */
   int32_t time_kernels;      /* CUDA events around each kernel (rtg_stats.*_ms) */
   int32_t count_traversal;   /* node / primitive counters (rtg_stats.node_visits, prim_tests) */
   uint32_t backlog_pools;    /* samples kept open for generation, in pools (default 3) */

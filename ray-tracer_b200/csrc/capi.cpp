@@ -747,7 +747,7 @@ int rtg_get_tuning(rtg_context* ctx, rtg_tuning* out) {
     const rtg::EngineConfig& c = ctx->engine->config();
     *out = rtg_tuning{};
     out->pool_paths = c.pool_paths;
-    out->block = static_cast<uint32_t>(c.shape.extend_block);
+    out->block = static_cast<uint32_t>(c.shape.block);
     out->max_pass_samples = c.max_pass_samples;
     out->extend_blocks = c.shape.extend_blocks;
     out->shade_blocks = c.shape.shade_blocks;
@@ -784,7 +784,7 @@ int rtg_set_tuning(rtg_context* ctx, const rtg_tuning* in) {
       return RTG_ERR_BUSY;
     }
     c.pool_paths = in->pool_paths;
-    c.shape.extend_block = static_cast<int>(in->block);
+    c.shape.block = static_cast<int>(in->block);
     c.max_pass_samples = in->max_pass_samples;
     c.shape.extend_blocks = in->extend_blocks;
     c.shape.shade_blocks = in->shade_blocks;

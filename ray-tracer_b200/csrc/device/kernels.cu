@@ -1,33 +1,23 @@
 // Wavefront path tracer for sm_100a.
 //
-// One iteration of the wavefront over a pool of path slots:
-//   k_plan    — one block: decides which open segments (passes of renders) the
-//               free slots go to, in the host's priority order, and copies the
-//               counters and segment progress to the pinned snapshot ring;
-//   k_extend  — fills free slots with new camera paths (thin-lens generation,
-//               src/rendering/renderer.cpp:33-37 + include/raytracer/core/camera.hpp:54-62)
-//               and finds every live path's closest hit (Scene::intersect).
-//   k_shade   — emission, material sampling, next-event estimation and Russian
-//               roulette for each hit (src/rendering/integrator.cpp:97-139); continuing
-//               paths are stream-compacted into the other state buffer and shadow
-//               rays into the shadow queue with one atomic per warp (ballot + popc).
-//   k_shadow  — any-hit test of each shadow ray (Scene::occluded); unoccluded ones
-//               add their contribution to the sample's radiance slot.
-// Every path owns one radiance slot addressed by (segment, pixel, sample-in-pass);
-// all adds to it happen in path order from kernels that are stream-ordered, so
-// the result does not depend on queue order, batch composition or timing. Paths
-// that end count themselves done in their segment's progress record; once a
-// segment is done, k_accumulate folds each pixel's samples into the double
-// framebuffer in sample order (Framebuffer::add,
+// One iteration over a list of at most `capacity` paths:
+//   k_plan — one block: decides which open segments (passes of renders) the new
+//            paths come from, in the host's priority order, and copies the
+//            counters and segment progress to the pinned snapshot ring;
+//   k_path — generates the camera paths (thin-lens generation,
+//            src/rendering/renderer.cpp:33-37 + include/raytracer/core/camera.hpp:54-62)
+//            and traces them: closest hits (Scene::intersect), emission, material
+//            sampling, next-event estimation and Russian roulette
+//            (src/rendering/integrator.cpp:97-139) and shadow rays
+//            (Scene::occluded). Each warp is a small wavefront of its own (see
+//            there); when the list is used up and more work is open, the paths
+//            in flight are left for the next iteration.
+// Every path owns one radiance slot addressed by (segment, pixel, sample-in-pass)
+// and adds to its radiance in path order, so the result does not depend on
+// scheduling, batch composition or timing. Paths that end count themselves done in
+// their segment's progress record; once a segment is done, k_accumulate folds each
+// pixel's samples into the double framebuffer in sample order (Framebuffer::add,
 // include/raytracer/rendering/framebuffer.hpp:31), passes of one render in order.
-//
-// Path state, hits and shadow rays are written and read once per iteration and
-// outgrow L2 at the pool sizes used, so they go through cache-streaming loads and
-// stores (__ldcs / __stcs) and leave L1/L2 to the BVH nodes and primitives.
-//
-// Work distribution: persistent warps fetch 32 items at a time from a cursor in
-// WaveCounters (Aila & Laine, "Understanding the Efficiency of Ray Traversal on
-// GPUs", HPG 2009), so uneven traversal costs balance across SMs.
 #include <cfloat>
 #include <type_traits>
 
@@ -40,6 +30,8 @@ namespace {
 
 constexpr float kRayTMin = 1e-6f;  // include/raytracer/math/ray.hpp:45
 constexpr int kStackSmem = 8;  // stack entries per thread in shared memory (8 measured 1% faster than 16 or 24)
+constexpr int kPathStack = 6;  // the same for the path kernel, whose path slots need the room (6 and 8 measure alike)
+constexpr int kPathThreads = 896;  // threads per SM the path kernel is compiled for (72 registers)
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 __device__ __forceinline__ std::uint64_t ld_u64(std::uint32_t lo, std::uint32_t hi) {
@@ -57,13 +49,6 @@ __device__ __forceinline__ void warp_add_u64(std::uint64_t v, std::uint64_t* dst
 __device__ __forceinline__ void chain_to_previous_grid() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// Warp-wide fetch of the next 32 work items from `cursor`.
-__device__ __forceinline__ std::uint32_t warp_fetch(std::uint32_t* cursor) {
-  std::uint32_t base = 0;
-  if ((threadIdx.x & 31) == 0) base = atomicAdd(cursor, 32u);
-  return __shfl_sync(kFull, base, 0);
 }
 
 struct CameraSample {
@@ -110,34 +95,36 @@ __device__ __forceinline__ CameraSample camera_sample(const RtgSceneDev& J, cons
 // ---------------------------------------------------------------------------
 // Inclusive scan over one block of kMaxGen threads (warp shuffles, then the warp
 // totals); `tot` is a kMaxGen / 32 scratch array and receives the block total.
-__device__ __forceinline__ std::uint32_t plan_scan(std::uint32_t v, std::uint32_t* tot, std::uint32_t& total) {
+template <class T>
+__device__ __forceinline__ T plan_scan(T v, T* tot, T& total) {
   constexpr int kWarps = kMaxGen / 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const std::uint32_t y = __shfl_up_sync(kFull, v, off);
+    const T y = __shfl_up_sync(kFull, v, off);
     if (lane >= off) v += y;
   }
   if (lane == 31) tot[w] = v;
   __syncthreads();
   if (w == 0) {
-    std::uint32_t x = lane < kWarps ? tot[lane] : 0u;
+    T x = lane < kWarps ? tot[lane] : 0;
 #pragma unroll
     for (int off = 1; off < kWarps; off <<= 1) {
-      const std::uint32_t y = __shfl_up_sync(kFull, x, off);
+      const T y = __shfl_up_sync(kFull, x, off);
       if (lane >= off) x += y;
     }
     if (lane < kWarps) tot[lane] = x;
   }
   __syncthreads();
   total = tot[kWarps - 1];
-  return v + (w > 0 ? tot[w - 1] : 0u);
+  return v + (w > 0 ? tot[w - 1] : 0);
 }
 
 // Generation plan: free slots go to the open segments greedily in the host's
 // order. One block of kMaxGen threads, one table entry each.
 __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
-  __shared__ std::uint32_t tot_rem[kMaxGen / 32], tot_flag[kMaxGen / 32];
+  __shared__ unsigned long long tot_rem[kMaxGen / 32];
+  __shared__ std::uint32_t tot_flag[kMaxGen / 32];
   chain_to_previous_grid();
   WaveCounters* C = wb.cnt;
   const int t = threadIdx.x;
@@ -164,12 +151,13 @@ __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
       C->error_info = slot;
     }
   }
-  // Inclusive scan of rem (each <= room <= 2^23, so the sum fits 32 bits).
-  std::uint32_t total = 0, n_plan = 0;
-  const std::uint32_t excl = plan_scan(rem, tot_rem, total) - rem;
-  const std::uint32_t take = excl >= room ? 0u : min(rem, room - excl);
+  unsigned long long total = 0;
+  std::uint32_t n_plan = 0;
+  const unsigned long long before = plan_scan<unsigned long long>(rem, tot_rem, total) - rem;
+  const std::uint32_t excl = before < room ? static_cast<std::uint32_t>(before) : room;
+  const std::uint32_t take = min(rem, room - excl);
   const std::uint32_t flag = take > 0 ? 1u : 0u;
-  const std::uint32_t fpos = plan_scan(flag, tot_flag, n_plan);
+  const std::uint32_t fpos = plan_scan<std::uint32_t>(flag, tot_flag, n_plan);
   if (flag) {
     const std::uint32_t k = fpos - 1;
     wb.plan->end[k] = excl + take;
@@ -178,304 +166,450 @@ __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
     wb.seg_prog[slot].generated = gen0 + take;
   }
   if (t == 0) {
-    const std::uint32_t n_new = total < room ? total : room;
+    const std::uint32_t n_new = total < room ? static_cast<std::uint32_t>(total) : room;
     wb.plan->n = n_plan;
     wb.plan->n_new = n_new;
-    C->n_extend = live + n_new;
+    C->n_items = live + n_new;
+    // Fewer new paths than there is room for: nothing else is open, so this
+    // iteration runs its paths to their end.
+    C->finish = total < room ? 1u : 0u;
     C->live[par ^ 1] = 0;
-    C->n_shadow = 0;
-    C->fetch[0] = 0;
-    C->fetch[1] = 0;
-    C->fetch[2] = 0;
+    C->fetch = 0;
     C->generated += n_new;
     C->iteration = iter + 1;
   }
 }
 
 // ---------------------------------------------------------------------------
-// Closest hit of one ray: the eight-wide tree (kWide8) or the binary tree, or
-// brute force when the job asks for it.
-template <int kBlock, bool kCount, bool kWide8, class Stack>
-__device__ __forceinline__ RayHit trace_closest(const RtgSceneDev& J, float3 o, float3 d, float tmin, Stack* stack,
-                                                TraceCount& tc) {
-  if (!J.use_bvh) return closest_brute<kCount>(J, o, d, tmin, FLT_MAX, tc);
-  if constexpr (kWide8) return closest_hit8<kStackSmem, kBlock, kCount>(J, o, d, tmin, FLT_MAX, stack, tc);
-  else return closest_hit<kStackSmem, kBlock, kCount>(J, o, d, tmin, FLT_MAX, stack, tc);
+// The path kernel: a wavefront per warp.
+//
+// Every warp owns kWarpPaths path slots in shared memory and sorts them into three
+// queues: `idle` (no path), `ready` (a ray to trace) and `lit` (a shadow ray to
+// trace). A step takes up to 32 entries of one queue:
+//   new     idle slots get the next items of the iteration's list (paths left by
+//           the previous iteration, then new camera paths), and go on as
+//   bounce  closest hit, emission, material sampling, next-event estimation and
+//           Russian roulette of each path; its slot then moves to `lit`, `ready`
+//           or `idle`;
+//   shadow  any-hit test of each shadow ray, then on to `ready` or `idle`.
+// The warp takes the first queue that can fill its lanes, so the walks and the
+// shading run 29 to 31 of 32 lanes wide (one path per lane, refilled when it ends,
+// leaves 40% of the lanes without a shadow ray and measured 1.4 to 1.6 times
+// slower). There is no barrier, and path state stays on the SM. A path in `lit` is
+// in no other queue, so the adds to its radiance keep their order.
+//
+// It replaces one kernel per stage over a pool of paths in HBM, where every bounce
+// of every path moved some 300 bytes and every stage waited for its slowest warp
+// (36 us of fixed cost an iteration on the sphere field, 160 us on the mesh). On
+// B200, device time before and after, default pool: Cornell 256x256x64 2595 and
+// 1960 us, sphere field 640x360x64 4446 and 2850 us; pool of 2^23: sphere field
+// 512x512x128 8250 and 5970 us, mesh 1024x1024x64 52.9 and 50.5 ms, 16 scenes of the
+// mix 123.2 and 115.0 ms.
+//
+// What bounds it: instruction issue (73% of the slots on Cornell) under divergence
+// (11 to 16 of 32 lanes active in the walks), then the walks' dependent loads.
+// - 56 slots a warp and 72 registers (7 blocks of 128 per SM) measured best: 48
+//   slots fill 27 lanes (3 to 6% slower), 64 leave less L1 (1 to 2%), 96 only 16
+//   warps an SM (18 to 25%); at 64 registers the shading spills (5 to 8%).
+// - Instruction cache: closest-hit and shadow rays share one copy of the walk, and
+//   what only some jobs need is in other instances. With a copy each (and the
+//   four-wide walk for shadow rays), warps in different steps evict each other's
+//   loops: 2.1 of 9.5 cycles per instruction went to fetching, now 0.4.
+constexpr int kWarpPaths = 56;
+
+constexpr std::uint32_t kPathSpecular = 1u << 12;   // last bounce was specular (or the path is new)
+constexpr std::uint32_t kPathContinues = 1u << 13;  // goes on after its shadow ray
+constexpr int kPathSegShift = 16;                   // low 12 bits: depth; 16 and up: segment slot
+static_assert(kMaxSegments <= 1 << 16, "the segment slot does not fit the path word");
+
+// One warp's path slots, one 4-byte column per field.
+template <bool kMis>
+struct alignas(16) WarpPaths {
+  float o[3][kWarpPaths];       // ray origin (and the shadow ray's: both leave the hit on the same side)
+  float d[3][kWarpPaths];
+  float beta[3][kWarpPaths];    // throughput
+  float light[3][kWarpPaths];   // radiance so far
+  std::uint32_t rng[4][kWarpPaths];  // PCG32 state (lo, hi), increment (lo, hi)
+  std::uint32_t sample[kWarpPaths];  // radiance slot
+  std::uint32_t meta[kWarpPaths];
+  float sh_d[3][kWarpPaths];    // shadow ray direction, length, contribution
+  float sh_tmax[kWarpPaths];
+  float sh_c[3][kWarpPaths];
+  float pdf[kMis ? kWarpPaths : 1];  // pdf of the last diffuse bounce
+  std::uint16_t job[kWarpPaths];
+  std::uint8_t idle[kWarpPaths], ready[kWarpPaths], lit[kWarpPaths];
+};
+
+__device__ __forceinline__ float3 get3(const float (&v)[3][kWarpPaths], int p) { return f3(v[0][p], v[1][p], v[2][p]); }
+__device__ __forceinline__ void set3(float (&v)[3][kWarpPaths], int p, float3 x) {
+  v[0][p] = x.x;
+  v[1][p] = x.y;
+  v[2][p] = x.z;
+}
+__device__ __forceinline__ void add3(float (&v)[3][kWarpPaths], int p, float3 x) {
+  v[0][p] += x.x;
+  v[1][p] += x.y;
+  v[2][p] += x.z;
 }
 
-// Any hit of one shadow ray below tmax: the eight-wide or the four-wide tree.
-template <int kBlock, bool kCount, bool kWide8, class Stack>
-__device__ __forceinline__ bool trace_any(const RtgSceneDev& J, float3 o, float3 d, float tmin, float tmax,
-                                          Stack* stack, TraceCount& tc) {
-  if (!J.use_bvh) return any_brute(J, o, d, tmin, tmax);
-  if constexpr (kWide8) return any_hit8<kStackSmem, kBlock, kCount>(J, o, d, tmin, tmax, stack, tc);
-  else return any_hit4<kStackSmem, kBlock, kCount>(J, o, d, tmin, tmax, stack, tc);
-}
+// The walk of an instance. The common instance walks the binary tree; the general
+// one also counts, walks the eight-wide tree and tests every primitive of jobs that
+// ask for it. Kept out of the common instance, that code frees instruction cache: 3%
+// (mesh) to 6% (Cornell).
+template <bool kGeneral>
+struct Walk;
 
-// Per-thread traversal stack entries in shared memory: groups (two words) for
-// the eight-wide walk, node links for the binary and four-wide walks.
-template <bool kWide8>
-using StackEntry = std::conditional_t<kWide8, uint2, int>;
-
-template <int kBlock, bool kCount, bool kWide8>
-__global__ void __launch_bounds__(kBlock) k_extend(WaveBuffers wb, int par) {
-  __shared__ StackEntry<kWide8> stack[kStackSmem * kBlock];
-  chain_to_previous_grid();
-  WaveCounters* C = wb.cnt;
-  const std::uint32_t live = C->live[par];
-  const std::uint32_t n = C->n_extend;
-  const GenPlan& P = *wb.plan;
-  float4* const A = wb.st_a[par];
-  float4* const B = wb.st_b[par];
-  TraceCount tc;
-  std::uint64_t rays = 0;
-  while (true) {
-    const std::uint32_t base = warp_fetch(&C->fetch[0]);
-    if (base >= n) break;
-    const std::uint32_t i = base + (threadIdx.x & 31);
-    if (i >= n) continue;
-    float3 o, d;
-    std::uint32_t job;
-    if (i >= live) {
-      // New path j: plan entry k is the first with end[k] > j.
-      const std::uint32_t j = i - live;
-      int lo = 0, hi = static_cast<int>(P.n) - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (P.end[mid] > j) hi = mid;
-        else lo = mid + 1;
-      }
-      const std::uint32_t seg = P.seg[lo];
-      const std::uint64_t local = P.start[lo] + (j - (lo > 0 ? P.end[lo - 1] : 0u));
-      const DevSegment S = wb.segs[seg];
-      job = S.job;
-      const CameraSample cs = camera_sample(wb.jobs[job], S, local);
-      o = cs.o;
-      d = cs.d;
-      __stcs(&A[i], make_float4(o.x, o.y, o.z, __uint_as_float(cs.sample)));
-      // Camera rays count as a specular bounce (no NEE double-count guard).
-      __stcs(&B[i], make_float4(d.x, d.y, d.z, __uint_as_float(kFlagSpecular | (job << kMetaSceneShift))));
-      __stcs(&wb.st_c[par][i], make_float4(1.f, 1.f, 1.f, __uint_as_float(seg)));
-      __stcs(&wb.st_d[par][i], make_uint4(static_cast<std::uint32_t>(cs.rng.state), static_cast<std::uint32_t>(cs.rng.state >> 32),
-                                   static_cast<std::uint32_t>(cs.rng.inc), static_cast<std::uint32_t>(cs.rng.inc >> 32)));
-      wb.radiance[cs.sample] = make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-      const float4 a = __ldcs(&A[i]);
-      const float4 b = __ldcs(&B[i]);
-      o = f3(a);
-      d = f3(b);
-      job = __float_as_uint(b.w) >> kMetaSceneShift;
-    }
-    const RtgSceneDev& J = wb.jobs[job];
-    const RayHit h = trace_closest<kBlock, kCount, kWide8>(J, o, d, kRayTMin, stack, tc);
-    __stcs(&wb.hits[i], make_float4(h.t, __uint_as_float(h.word), h.b1, h.b2));
-    ++rays;
+template <>
+struct Walk<false> {
+  using Entry = int;
+  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* column,
+                                               int, TraceCount& tc) {
+    return walk_binary<kPathStack, 32, false>(J, o, d, kRayTMin, tmax, any, column, tc);
   }
-  warp_add_u64(rays, &C->rays);
-  if (kCount) {
+};
+
+template <>
+struct Walk<true> {
+  using Entry = uint2;
+  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* column,
+                                               int tree, TraceCount& tc) {
+    RayHit found{tmax, 0u, 0.f, 0.f};
+    if (!J.use_bvh) {
+      if (!any) return closest_brute<true>(J, o, d, kRayTMin, tmax, tc);
+      if (!any_brute(J, o, d, kRayTMin, tmax)) found.word = kHitMiss;
+      return found;
+    }
+    if (tree == 8) {
+      if (!any) return closest_hit8<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, column, tc);
+      if (!any_hit8<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, column, tc)) found.word = kHitMiss;
+      return found;
+    }
+    return walk_binary<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, any, reinterpret_cast<int*>(column), tc);
+  }
+};
+
+template <bool kMis, bool kGeneral>
+constexpr std::size_t kWarpSmem = sizeof(WarpPaths<kMis>) + sizeof(typename Walk<kGeneral>::Entry) * 32 * kPathStack;
+
+// kMis: some open job uses multiple importance sampling. Without one, that code is
+// compiled out. closest_tree and shadow_tree matter to the general instance only.
+template <int kBlock, bool kMis, bool kGeneral>
+__global__ void __launch_bounds__(kBlock, kPathThreads / kBlock)
+k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned long long s_total[3];
+  using Entry = typename Walk<kGeneral>::Entry;
+  const int lane = threadIdx.x & 31;
+  unsigned char* const mine = smem + (threadIdx.x >> 5) * kWarpSmem<kMis, kGeneral>;
+  WarpPaths<kMis>& S = *reinterpret_cast<WarpPaths<kMis>*>(mine);
+  // This thread's stack column: entry k at column[k * 32].
+  Entry* const column = reinterpret_cast<Entry*>(mine + sizeof(WarpPaths<kMis>)) + lane;
+  if (threadIdx.x < 3) s_total[threadIdx.x] = 0;
+#pragma unroll 1
+  for (int k = lane; k < kWarpPaths; k += 32) S.idle[k] = static_cast<std::uint8_t>(k);
+  __syncthreads();
+  chain_to_previous_grid();
+  WaveCounters* const C = wb.cnt;
+  const std::uint32_t live = C->live[par], n = C->n_items;
+  const bool finish = C->finish != 0;
+  const unsigned below = (1u << lane) - 1u;
+  Walk<kGeneral> walk;
+  TraceCount tc, sh_tc;
+  std::uint32_t rays = 0, shadow_rays = 0, rr_killed = 0;     // of the warp
+  std::uint32_t done_seg = 0xFFFFFFFFu, done_count = 0;       // finished paths not yet counted in their segment
+  int n_idle = kWarpPaths, n_ready = 0, n_lit = 0;
+  bool more = true;  // the iteration's list may have items left
+  while (true) {
+    const int n_new = more ? n_idle : 0;
+    enum { kShadow, kBounce, kNew } step;
+    if (!more && !finish) {
+      // The list is used up and more will follow: leave the paths for the next
+      // iteration, once no shadow ray is pending.
+      if (n_lit == 0) break;
+      step = kShadow;
+    } else if (n_lit >= 32) {
+      step = kShadow;
+    } else if (n_ready >= 32) {
+      step = kBounce;
+    } else if (n_new >= 32) {
+      step = kNew;
+    } else {
+      if ((n_lit | n_ready | n_new) == 0) break;
+      step = n_lit >= n_ready && n_lit >= n_new ? kShadow : (n_ready >= n_new ? kBounce : kNew);
+    }
+    bool on = false, cont = false, shadow = false, killed = false;
+    int p = 0;
+    float3 o = f3(0.f, 0.f, 0.f), d = o;
+    float tmax = FLT_MAX;
+    std::uint32_t job = 0;
+    if (step == kShadow) {
+      const int take = min(n_lit, 32);
+      n_lit -= take;
+      shadow_rays += take;
+      on = lane < take;
+      if (on) {
+        p = S.lit[n_lit + lane];
+        o = get3(S.o, p);
+        d = get3(S.sh_d, p);
+        tmax = S.sh_tmax[p];
+        job = S.job[p];
+      }
+    } else if (step == kBounce) {
+      const int take = min(n_ready, 32);
+      n_ready -= take;
+      rays += take;
+      on = lane < take;
+      if (on) {
+        p = S.ready[n_ready + lane];
+        o = get3(S.o, p);
+        d = get3(S.d, p);
+        job = S.job[p];
+      }
+    } else {
+      int take = min(n_idle, 32);
+      std::uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&C->fetch, static_cast<std::uint32_t>(take));
+      base = __shfl_sync(kFull, base, 0);
+      if (base >= n) {
+        more = false;
+        continue;
+      }
+      if (n - base < static_cast<std::uint32_t>(take)) {
+        take = static_cast<int>(n - base);
+        more = false;
+      }
+      n_idle -= take;
+      rays += take;
+      on = lane < take;
+      if (on) {
+        p = S.idle[n_idle + lane];
+        const std::uint32_t i = base + lane;
+        if (i < live) {
+          // A path the previous iteration left.
+          const float4 a = __ldcs(&wb.st_a[par][i]), b = __ldcs(&wb.st_b[par][i]), c = __ldcs(&wb.st_c[par][i]);
+          const uint4 r = __ldcs(&wb.st_d[par][i]);
+          const float4 l = __ldcs(&wb.st_e[par][i]);
+          o = f3(a);
+          d = f3(b);
+          S.sample[p] = __float_as_uint(a.w);
+          S.meta[p] = __float_as_uint(b.w);
+          set3(S.beta, p, f3(c));
+          job = __float_as_uint(c.w);
+          S.rng[0][p] = r.x;
+          S.rng[1][p] = r.y;
+          S.rng[2][p] = r.z;
+          S.rng[3][p] = r.w;
+          set3(S.light, p, f3(l));
+          if (kMis) S.pdf[p] = l.w;
+        } else {
+          const std::uint32_t j = i - live;
+          // New path j: plan entry k is the first with end[k] > j.
+          const GenPlan& P = *wb.plan;
+          int lo = 0, hi = static_cast<int>(P.n) - 1;
+#pragma unroll 1
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (P.end[mid] > j) hi = mid;
+            else lo = mid + 1;
+          }
+          const std::uint32_t seg = P.seg[lo];
+          const std::uint64_t local = P.start[lo] + (j - (lo > 0 ? P.end[lo - 1] : 0u));
+          const DevSegment sg = wb.segs[seg];
+          job = sg.job;
+          const CameraSample cs = camera_sample(wb.jobs[job], sg, local);
+          o = cs.o;
+          d = cs.d;
+          S.sample[p] = cs.sample;
+          // Camera rays count as a specular bounce (no NEE double-count guard).
+          S.meta[p] = kPathSpecular | (seg << kPathSegShift);
+          set3(S.beta, p, f3(1.f, 1.f, 1.f));
+          S.rng[0][p] = static_cast<std::uint32_t>(cs.rng.state);
+          S.rng[1][p] = static_cast<std::uint32_t>(cs.rng.state >> 32);
+          S.rng[2][p] = static_cast<std::uint32_t>(cs.rng.inc);
+          S.rng[3][p] = static_cast<std::uint32_t>(cs.rng.inc >> 32);
+          set3(S.light, p, f3(0.f, 0.f, 0.f));
+        }
+        S.job[p] = static_cast<std::uint16_t>(job);
+      }
+    }
+    __syncwarp();
+    if (on) {
+      const RtgSceneDev& J = wb.jobs[job];
+      // One copy of the walk serves both kinds of rays.
+      const bool any = step == kShadow;
+      const RayHit h = walk(J, o, d, tmax, any, column, any ? shadow_tree : closest_tree, any ? sh_tc : tc);
+      const std::uint32_t meta = S.meta[p];
+      if (any) {
+        if (h.word == kHitMiss) add3(S.light, p, get3(S.sh_c, p));
+        cont = (meta & kPathContinues) != 0;
+      } else if (h.word == kHitMiss) {
+        // The normals view shows misses black.
+        if (J.integrator != 2) add3(S.light, p, get3(S.beta, p) * background(J, d));
+      } else {
+        const Surface s = make_surface(J, o, d, h);
+        if (J.integrator == 2) {
+          // Normals view: outward shading normal mapped to [0, 1].
+          const float3 nn = s.front ? s.n : -s.n;
+          set3(S.light, p, f3(0.5f * (nn.x + 1.f), 0.5f * (nn.y + 1.f), 0.5f * (nn.z + 1.f)));
+        } else {
+          const DevMaterial m = J.materials[s.material];
+          const float3 le = emitted(m, s.front);
+          // A light reached by a diffuse bounce was already counted by NEE. With
+          // MIS both count, each weighted by the power heuristic against the other.
+          if (!is_zero3(le)) {
+            float w = 1.f;
+            if (!(meta & kPathSpecular) && J.light_sampling && !s.is_plane)
+              w = kMis && J.light_sampling == 2
+                      ? power_heuristic(S.pdf[kMis ? p : 0],
+                                        light_pdf_of_hit(J, o, d, h, s) / static_cast<float>(J.n_lights))
+                      : 0.f;
+            if (w > 0.f) add3(S.light, p, get3(S.beta, p) * le * w);
+          }
+          Pcg rng{ld_u64(S.rng[0][p], S.rng[1][p]), ld_u64(S.rng[2][p], S.rng[3][p])};
+          Scatter sr;
+          if (scatter(m, d, s, rng, sr)) {
+            // The next ray goes to shared memory before the light sample, which
+            // needs the registers.
+            set3(S.o, p, spawn_towards(s.p, s.gn, sr.dir));
+            set3(S.d, p, sr.dir);
+            if (J.light_sampling && !sr.specular && J.n_lights > 0) {
+              const std::uint32_t nl = static_cast<std::uint32_t>(J.n_lights);
+              const LightSample ls = sample_light(J.lights + rng.below(nl), s, rng);
+              if (ls.valid) {
+                // Only a Lambertian scatter is non-specular: its weight is the albedo.
+                const float3 f = lambert_cos(sr.weight, s, ls.wi);
+                if (!is_zero3(f) && !is_zero3(ls.li_over_pdf)) {
+                  // Its origin is the one stored above: a Lambertian scatter leaves,
+                  // and lambert_cos is non-zero, on the side of s.gn only.
+                  const ShadowRay sray = shadow_ray(s, ls);
+                  float w = 1.f;  // a point light (pdf 0) cannot be hit by BSDF sampling
+                  if (kMis && J.light_sampling == 2 && ls.pdf > 0.f)
+                    w = power_heuristic(ls.pdf / static_cast<float>(nl), dot3(s.n, ls.wi) * kInvPiF);
+                  set3(S.sh_d, p, sray.d);
+                  S.sh_tmax[p] = sray.tmax;
+                  set3(S.sh_c, p, get3(S.beta, p) * (f * ls.li_over_pdf) * (static_cast<float>(nl) * w));
+                  shadow = true;
+                }
+              }
+            }
+            float3 beta = get3(S.beta, p) * sr.weight;
+            const std::uint32_t depth = (meta & kMetaDepthMask) + 1;
+            bool alive = !is_zero3(beta);
+            if (alive && depth >= static_cast<std::uint32_t>(J.rr_min_depth)) {
+              const float q = fminf(fmaxf(max3(beta), 0.05f), 0.95f);
+              if (rng.uniform() >= q) {
+                alive = false;
+                killed = true;
+              } else {
+                beta = beta * (1.f / q);
+              }
+            }
+            cont = alive && depth < static_cast<std::uint32_t>(J.max_depth);
+            if (cont) {
+              set3(S.beta, p, beta);
+              S.rng[0][p] = static_cast<std::uint32_t>(rng.state);
+              S.rng[1][p] = static_cast<std::uint32_t>(rng.state >> 32);
+              // Cosine-hemisphere pdf of this bounce, for the MIS weight at the next hit.
+              if (kMis && J.light_sampling == 2 && !sr.specular) S.pdf[kMis ? p : 0] = dot3(s.n, sr.dir) * kInvPiF;
+            }
+            S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u);
+          }
+        }
+      }
+    }
+    const bool ready = cont && !shadow, end = on && !cont && !shadow;
+    const unsigned m_lit = __ballot_sync(kFull, shadow), m_ready = __ballot_sync(kFull, ready);
+    const unsigned m_end = __ballot_sync(kFull, end);
+    rr_killed += __popc(__ballot_sync(kFull, killed));
+    if (shadow) S.lit[n_lit + __popc(m_lit & below)] = static_cast<std::uint8_t>(p);
+    if (ready) S.ready[n_ready + __popc(m_ready & below)] = static_cast<std::uint8_t>(p);
+    if (m_end) {
+      std::uint32_t seg = 0;
+      if (end) {
+        S.idle[n_idle + __popc(m_end & below)] = static_cast<std::uint8_t>(p);
+        const float3 l = get3(S.light, p);
+        wb.radiance[S.sample[p]] = make_float4(l.x, l.y, l.z, 0.f);
+        seg = S.meta[p] >> kPathSegShift;
+      }
+      // Finished paths are counted in their segment: the warp keeps a count while
+      // they belong to one segment, as they mostly do.
+      const std::uint32_t seg0 = __shfl_sync(kFull, seg, __ffs(m_end) - 1);
+      if (__any_sync(kFull, end && seg != seg0)) {
+        const unsigned same = __match_any_sync(kFull, end ? seg : 0xFFFFFFFFu);
+        if (end && lane == __ffs(same) - 1) atomicAdd(&wb.seg_prog[seg].done, static_cast<std::uint32_t>(__popc(same)));
+      } else {
+        if (seg0 != done_seg) {
+          if (lane == 0 && done_count) atomicAdd(&wb.seg_prog[done_seg].done, done_count);
+          done_seg = seg0;
+          done_count = 0;
+        }
+        done_count += __popc(m_end);
+      }
+    }
+    n_lit += __popc(m_lit);
+    n_ready += __popc(m_ready);
+    n_idle += __popc(m_end);
+    __syncwarp();
+  }
+  if (lane == 0 && done_count) atomicAdd(&wb.seg_prog[done_seg].done, done_count);
+  if (n_ready) {
+    std::uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&C->live[par ^ 1], static_cast<std::uint32_t>(n_ready));
+    base = __shfl_sync(kFull, base, 0);
+#pragma unroll 1
+    for (int k = lane; k < n_ready; k += 32) {
+      const int p = S.ready[k];
+      const std::uint32_t i = base + k;
+      const float3 o = get3(S.o, p), d = get3(S.d, p), b = get3(S.beta, p), l = get3(S.light, p);
+      __stcs(&wb.st_a[par ^ 1][i], make_float4(o.x, o.y, o.z, __uint_as_float(S.sample[p])));
+      __stcs(&wb.st_b[par ^ 1][i], make_float4(d.x, d.y, d.z, __uint_as_float(S.meta[p])));
+      __stcs(&wb.st_c[par ^ 1][i], make_float4(b.x, b.y, b.z, __uint_as_float(S.job[p])));
+      __stcs(&wb.st_d[par ^ 1][i], make_uint4(S.rng[0][p], S.rng[1][p], S.rng[2][p], S.rng[3][p]));
+      __stcs(&wb.st_e[par ^ 1][i], make_float4(l.x, l.y, l.z, kMis ? S.pdf[kMis ? p : 0] : 0.f));
+    }
+  }
+  // Counters: one atomic per block and counter.
+  if (lane == 0) {
+    atomicAdd(&s_total[0], static_cast<unsigned long long>(rays));
+    atomicAdd(&s_total[1], static_cast<unsigned long long>(shadow_rays));
+    atomicAdd(&s_total[2], static_cast<unsigned long long>(rr_killed));
+  }
+  __syncthreads();
+  if (threadIdx.x < 3 && s_total[threadIdx.x]) {
+    std::uint64_t* const to = threadIdx.x == 0 ? &C->rays : (threadIdx.x == 1 ? &C->shadow_rays : &C->rr_terminated);
+    atomicAdd(reinterpret_cast<unsigned long long*>(to), s_total[threadIdx.x]);
+  }
+  if (kGeneral) {
     warp_add_u64(tc.nodes, &C->node_visits);
     warp_add_u64(tc.prims, &C->prim_tests);
     warp_add_u64(tc.spheres, &C->sphere_tests);
+    warp_add_u64(sh_tc.nodes, &C->shadow_node_visits);
+    warp_add_u64(sh_tc.prims, &C->shadow_prim_tests);
+    warp_add_u64(sh_tc.spheres, &C->shadow_sphere_tests);
   }
 }
 
 // ---------------------------------------------------------------------------
-// 64 registers (8 blocks of 128 per SM) with a few spills measured 4% faster than 80.
-// kMis: some open job uses multiple importance sampling. Without one, the MIS code
-// is compiled out and the kernel keeps its registers for the common path.
-template <int kBlock, bool kMis>
-__global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_shade(WaveBuffers wb, int par) {
-  constexpr int kWarps = kBlock / 32;
-  // Per-round queue counts and bases, double-buffered by round parity: a round
-  // writes one buffer while the other may still be read, so no barrier is needed
-  // at the end of a round.
-  __shared__ std::uint32_t s_cnt[2][2][kWarps];
-  __shared__ std::uint32_t s_base[2][2];
-  int rb = 0;
-  chain_to_previous_grid();
-  WaveCounters* C = wb.cnt;
-  const std::uint32_t n = C->n_extend;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float4* const A = wb.st_a[par];
-  const float4* const B = wb.st_b[par];
-  const float4* const Cc = wb.st_c[par];
-  const uint4* const D = wb.st_d[par];
-  std::uint64_t rr_killed = 0;
-  // Uniform work per path: blocks stride over the hits in order (no fetch atomics).
-  for (std::uint32_t base = blockIdx.x * kBlock; base < n; base += gridDim.x * kBlock) {
-    const std::uint32_t i = base + threadIdx.x;
-    bool cont = false, shadow = false;
-    float3 o_next = f3(0.f, 0.f, 0.f), d_next = o_next, beta = o_next, sh_o = o_next, sh_d = o_next, sh_c = o_next;
-    float sh_tmax = 0.f;
-    std::uint32_t sample = 0, meta_next = 0, job = 0, seg = 0;
-    float pdf_next = -1.f;  // set when the next hit may need a MIS weight
-    Pcg rng{0, 0};
-    if (i < n) {
-      const float4 a = __ldcs(&A[i]), b = __ldcs(&B[i]), c = __ldcs(&Cc[i]), hv = __ldcs(&wb.hits[i]);
-      const uint4 r = __ldcs(&D[i]);
-      const float3 o = f3(a), d = f3(b);
-      sample = __float_as_uint(a.w);
-      const std::uint32_t meta = __float_as_uint(b.w);
-      const std::uint32_t depth = meta & kMetaDepthMask;
-      const bool specular_bounce = (meta & kFlagSpecular) != 0;
-      job = meta >> kMetaSceneShift;
-      seg = __float_as_uint(c.w);
-      beta = f3(c);
-      rng.state = ld_u64(r.x, r.y);
-      rng.inc = ld_u64(r.z, r.w);
-      const RtgSceneDev& J = wb.jobs[job];
-      const RayHit h{hv.x, __float_as_uint(hv.y), hv.z, hv.w};
-      float4* const slot = &wb.radiance[sample];
-      if (J.integrator == 2) {
-        // Normals view: outward shading normal mapped to [0, 1]; black on a miss.
-        if (h.word != kHitMiss) {
-          const Surface s = make_surface(J, o, d, h);
-          const float3 nn = s.front ? s.n : -s.n;
-          *slot = make_float4(0.5f * (nn.x + 1.f), 0.5f * (nn.y + 1.f), 0.5f * (nn.z + 1.f), 0.f);
-        }
-      } else if (h.word == kHitMiss) {
-        const float3 bg = beta * background(J, d);
-        const float4 acc = *slot;
-        *slot = make_float4(acc.x + bg.x, acc.y + bg.y, acc.z + bg.z, 0.f);
-      } else {
-        const Surface s = make_surface(J, o, d, h);
-        const DevMaterial m = J.materials[s.material];
-        const float3 le = emitted(m, s.front);
-        // A light reached by a diffuse bounce was already counted by NEE. With
-        // MIS both count, each weighted by the power heuristic against the other.
-        if (!is_zero3(le)) {
-          float w = 1.f;
-          if (!specular_bounce && J.light_sampling && !s.is_plane)
-            w = kMis && J.light_sampling == 2
-                    ? power_heuristic(__ldcs(&wb.st_e[par][i]),
-                                      light_pdf_of_hit(J, o, d, h, s) / static_cast<float>(J.n_lights))
-                    : 0.f;
-          if (w > 0.f) {
-            const float3 add = beta * le * w;
-            const float4 acc = *slot;
-            *slot = make_float4(acc.x + add.x, acc.y + add.y, acc.z + add.z, 0.f);
-          }
-        }
-        Scatter sr;
-        if (scatter(m, d, s, rng, sr)) {
-          if (J.light_sampling && !sr.specular && J.n_lights > 0) {
-            const std::uint32_t nl = static_cast<std::uint32_t>(J.n_lights);
-            const LightSample ls = sample_light(J.lights + rng.below(nl), s, rng);
-            if (ls.valid) {
-              // Only a Lambertian scatter is non-specular: its weight is the albedo.
-              const float3 f = lambert_cos(sr.weight, s, ls.wi);
-              if (!is_zero3(f) && !is_zero3(ls.li_over_pdf)) {
-                const ShadowRay sray = shadow_ray(s, ls);
-                sh_o = sray.o;
-                sh_d = sray.d;
-                sh_tmax = sray.tmax;
-                float w = 1.f;  // a point light (pdf 0) cannot be hit by BSDF sampling
-                if (kMis && J.light_sampling == 2 && ls.pdf > 0.f)
-                  w = power_heuristic(ls.pdf / static_cast<float>(nl), dot3(s.n, ls.wi) * kInvPiF);
-                sh_c = beta * (f * ls.li_over_pdf) * (static_cast<float>(nl) * w);
-                shadow = true;
-              }
-            }
-          }
-          beta = beta * sr.weight;
-          bool alive = !is_zero3(beta);
-          if (alive && depth + 1 >= static_cast<std::uint32_t>(J.rr_min_depth)) {
-            const float q = fminf(fmaxf(max3(beta), 0.05f), 0.95f);
-            if (rng.uniform() >= q) {
-              alive = false;
-              ++rr_killed;
-            } else {
-              beta = beta * (1.f / q);
-            }
-          }
-          if (alive && depth + 1 < static_cast<std::uint32_t>(J.max_depth)) {
-            cont = true;
-            o_next = spawn_towards(s.p, s.gn, sr.dir);
-            d_next = sr.dir;
-            meta_next = (depth + 1) | (sr.specular ? kFlagSpecular : 0u) | (job << kMetaSceneShift);
-            // Cosine-hemisphere pdf of this bounce, for the MIS weight at the next hit.
-            if (kMis && J.light_sampling == 2 && !sr.specular) pdf_next = dot3(s.n, sr.dir) * kInvPiF;
-          }
-        }
-      }
-    }
-    // Appends aggregated per block: one atomic per queue per 256 paths.
-    const unsigned mc = __ballot_sync(kFull, cont), ms = __ballot_sync(kFull, shadow);
-    if (lane == 0) {
-      s_cnt[rb][0][warp] = __popc(mc);
-      s_cnt[rb][1][warp] = __popc(ms);
-    }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-      std::uint32_t total = 0;
-      for (int w = 0; w < kWarps; ++w) {
-        const std::uint32_t c = s_cnt[rb][threadIdx.x][w];
-        s_cnt[rb][threadIdx.x][w] = total;
-        total += c;
-      }
-      s_base[rb][threadIdx.x] = total ? atomicAdd(threadIdx.x == 0 ? &C->live[par ^ 1] : &C->n_shadow, total) : 0u;
-    }
-    __syncthreads();
-    const unsigned below = (1u << lane) - 1u;
-    const std::uint32_t cpos = s_base[rb][0] + s_cnt[rb][0][warp] + __popc(mc & below);
-    const std::uint32_t spos = s_base[rb][1] + s_cnt[rb][1][warp] + __popc(ms & below);
-    // The next round writes the other buffer; the one after writes this one again
-    // only after its first barrier, which every thread reaches after these reads.
-    rb ^= 1;
-    // A path that ends here is done once this iteration's shadow stage has run:
-    // count it in its segment (one atomic per segment present in the warp).
-    const bool fin = i < n && !cont;
-    const unsigned same = __match_any_sync(kFull, fin ? seg : 0xFFFFFFFFu);
-    if (fin && (threadIdx.x & 31) == static_cast<unsigned>(__ffs(same) - 1))
-      atomicAdd(&wb.seg_prog[seg].done, static_cast<std::uint32_t>(__popc(same)));
-    if (cont) {
-      __stcs(&wb.st_a[par ^ 1][cpos], make_float4(o_next.x, o_next.y, o_next.z, __uint_as_float(sample)));
-      __stcs(&wb.st_b[par ^ 1][cpos], make_float4(d_next.x, d_next.y, d_next.z, __uint_as_float(meta_next)));
-      __stcs(&wb.st_c[par ^ 1][cpos], make_float4(beta.x, beta.y, beta.z, __uint_as_float(seg)));
-      __stcs(&wb.st_d[par ^ 1][cpos], make_uint4(static_cast<std::uint32_t>(rng.state), static_cast<std::uint32_t>(rng.state >> 32),
-                                          static_cast<std::uint32_t>(rng.inc), static_cast<std::uint32_t>(rng.inc >> 32)));
-      if (kMis && pdf_next >= 0.f) __stcs(&wb.st_e[par ^ 1][cpos], pdf_next);
-    }
-    if (shadow) {
-      __stcs(&wb.sh_a[spos], make_float4(sh_o.x, sh_o.y, sh_o.z, __uint_as_float(sample)));
-      __stcs(&wb.sh_b[spos], make_float4(sh_d.x, sh_d.y, sh_d.z, sh_tmax));
-      __stcs(&wb.sh_c[spos], make_float4(sh_c.x, sh_c.y, sh_c.z, __uint_as_float(job)));
-    }
-  }
-  warp_add_u64(rr_killed, &C->rr_terminated);
+// The walks of the direct integrator: the eight-wide tree (kWide8) or the binary
+// (closest hit) and four-wide (any hit) trees, or brute force when the job asks for
+// it. `column` is this thread's stack.
+template <bool kWide8>
+using StackEntry = std::conditional_t<kWide8, uint2, int>;
+
+template <int kBlock, bool kWide8>
+__device__ __forceinline__ RayHit trace_closest(const RtgSceneDev& J, float3 o, float3 d, StackEntry<kWide8>* column,
+                                                TraceCount& tc) {
+  if (!J.use_bvh) return closest_brute<false>(J, o, d, kRayTMin, FLT_MAX, tc);
+  if constexpr (kWide8) return closest_hit8<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, column, tc);
+  else return closest_hit<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, column, tc);
 }
 
-// ---------------------------------------------------------------------------
-template <int kBlock, bool kCount, bool kWide8>
-__global__ void __launch_bounds__(kBlock) k_shadow(WaveBuffers wb) {
-  __shared__ StackEntry<kWide8> stack[kStackSmem * kBlock];
-  chain_to_previous_grid();
-  WaveCounters* C = wb.cnt;
-  const std::uint32_t n = C->n_shadow;
-  TraceCount tc;
-  std::uint64_t rays = 0;
-  while (true) {
-    const std::uint32_t base = warp_fetch(&C->fetch[2]);
-    if (base >= n) break;
-    const std::uint32_t i = base + (threadIdx.x & 31);
-    if (i >= n) continue;
-    const float4 a = __ldcs(&wb.sh_a[i]), b = __ldcs(&wb.sh_b[i]), c = __ldcs(&wb.sh_c[i]);
-    const RtgSceneDev& J = wb.jobs[__float_as_uint(c.w)];
-    const float3 o = f3(a), d = f3(b);
-    const bool blocked = trace_any<kBlock, kCount, kWide8>(J, o, d, kRayTMin, b.w, stack, tc);
-    ++rays;
-    if (!blocked) {
-      float4* const slot = &wb.radiance[__float_as_uint(a.w)];
-      const float4 acc = *slot;
-      *slot = make_float4(acc.x + c.x, acc.y + c.y, acc.z + c.z, 0.f);
-    }
-  }
-  warp_add_u64(rays, &C->shadow_rays);
-  if (kCount) {
-    warp_add_u64(tc.nodes, &C->shadow_node_visits);
-    warp_add_u64(tc.prims, &C->shadow_prim_tests);
-    warp_add_u64(tc.spheres, &C->shadow_sphere_tests);
-  }
+template <int kBlock, bool kWide8>
+__device__ __forceinline__ bool trace_any(const RtgSceneDev& J, float3 o, float3 d, float tmax,
+                                          StackEntry<kWide8>* column, TraceCount& tc) {
+  if (!J.use_bvh) return any_brute(J, o, d, kRayTMin, tmax);
+  if constexpr (kWide8) return any_hit8<kStackSmem, kBlock, false>(J, o, d, kRayTMin, tmax, column, tc);
+  else return any_hit4<kStackSmem, kBlock, false>(J, o, d, kRayTMin, tmax, column, tc);
 }
 
 // ---------------------------------------------------------------------------
@@ -502,7 +636,7 @@ __device__ __forceinline__ float3 direct_light_all(const RtgSceneDev& J, const D
     if (is_zero3(f) || is_zero3(ls.li_over_pdf)) continue;
     const ShadowRay sr = shadow_ray(s, ls);
     ++shadow_rays;
-    const bool blocked = trace_any<kBlock, false, kWide8>(J, sr.o, sr.d, kRayTMin, sr.tmax, stack, tc);
+    const bool blocked = trace_any<kBlock, kWide8>(J, sr.o, sr.d, sr.tmax, stack, tc);
     if (!blocked) sum = sum + f * ls.li_over_pdf;
   }
   return sum;
@@ -512,6 +646,7 @@ template <int kBlock, bool kWide8>
 __global__ void __launch_bounds__(kBlock) k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance,
                                                    WaveCounters* C) {
   __shared__ StackEntry<kWide8> stack[kStackSmem * kBlock];
+  StackEntry<kWide8>* const column = stack + threadIdx.x;
   TraceCount tc;
   std::uint64_t rays = 0, shadow_rays = 0;
   const RtgSceneDev& J = *job;
@@ -525,7 +660,7 @@ __global__ void __launch_bounds__(kBlock) k_direct(const RtgSceneDev* __restrict
     bool overflow = false;
     while (true) {
       ++rays;
-      const RayHit h = trace_closest<kBlock, false, kWide8>(J, cur.o, cur.d, kRayTMin, stack, tc);
+      const RayHit h = trace_closest<kBlock, kWide8>(J, cur.o, cur.d, column, tc);
       bool next = false;
       if (h.word == kHitMiss) {
         L = L + cur.w * background(J, cur.d);
@@ -536,7 +671,7 @@ __global__ void __launch_bounds__(kBlock) k_direct(const RtgSceneDev* __restrict
         if (cur.depth < J.max_depth) {
           const std::uint32_t kind = kind_of(m);
           if (kind == kLambertian) {
-            L = L + cur.w * direct_light_all<kBlock, kWide8>(J, m, s, cs.rng, stack, tc, shadow_rays);
+            L = L + cur.w * direct_light_all<kBlock, kWide8>(J, m, s, cs.rng, column, tc, shadow_rays);
           } else if (kind == kMetal) {
             Scatter sr;
             if (scatter(m, cur.d, s, cs.rng, sr)) {
@@ -661,8 +796,8 @@ __global__ void __launch_bounds__(kBlock) k_ray_closest(const RtgSceneDev* __res
   TraceCount tc;
   RayHit h;
   if (brute) h = closest_brute<false>(*job, f3(a), f3(b), a.w, b.w, tc);
-  else if (tree == 8) h = closest_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack, tc);
-  else h = closest_hit<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack), tc);
+  else if (tree == 8) h = closest_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack + threadIdx.x, tc);
+  else h = closest_hit<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack) + threadIdx.x, tc);
   refine_hit(*job, f3(a), f3(b), h);
   out[i] = make_float4(h.t, __uint_as_float(h.word), h.b1, h.b2);
 }
@@ -677,8 +812,8 @@ __global__ void __launch_bounds__(kBlock) k_ray_any(const RtgSceneDev* __restric
   TraceCount tc;
   bool hit;
   if (brute) hit = any_brute(*job, f3(a), f3(b), a.w, b.w);
-  else if (tree == 8) hit = any_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack, tc);
-  else hit = any_hit4<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack), tc);
+  else if (tree == 8) hit = any_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack + threadIdx.x, tc);
+  else hit = any_hit4<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack) + threadIdx.x, tc);
   out[i] = hit ? 1u : 0u;
 }
 
@@ -693,39 +828,15 @@ int persistent_blocks(K kernel, int block) {
   return sms * per_sm;
 }
 
-// Persistent grid sizes per kernel variant: [counting][eight-wide].
-struct BlockCounts {
-  int extend[2][2] = {}, shadow[2][2] = {}, shade = 0, shade_mis = 0;
-};
-
-template <int kBlock>
-const BlockCounts& block_counts() {
-  static BlockCounts bc = [] {
-    BlockCounts b;
-    b.extend[0][0] = persistent_blocks(k_extend<kBlock, false, false>, kBlock);
-    b.extend[0][1] = persistent_blocks(k_extend<kBlock, false, true>, kBlock);
-    b.extend[1][0] = persistent_blocks(k_extend<kBlock, true, false>, kBlock);
-    b.extend[1][1] = persistent_blocks(k_extend<kBlock, true, true>, kBlock);
-    b.shade = persistent_blocks(k_shade<kBlock, false>, kBlock);
-    b.shade_mis = persistent_blocks(k_shade<kBlock, true>, kBlock);
-    b.shadow[0][0] = persistent_blocks(k_shadow<kBlock, false, false>, kBlock);
-    b.shadow[0][1] = persistent_blocks(k_shadow<kBlock, false, true>, kBlock);
-    b.shadow[1][0] = persistent_blocks(k_shadow<kBlock, true, false>, kBlock);
-    b.shadow[1][1] = persistent_blocks(k_shadow<kBlock, true, true>, kBlock);
-    return b;
-  }();
-  return bc;
-}
-
 // Launch with programmatic stream serialization (when enabled) so the kernel's
 // blocks are scheduled while the previous wavefront kernel drains.
 template <class... KArgs, class... Args>
-cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block, bool pdl, cudaStream_t stream,
-                           Args... args) {
+cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block, std::size_t smem, bool pdl,
+                           cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(static_cast<unsigned>(block));
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -735,67 +846,55 @@ cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block, bool p
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <int kBlock, bool kCount, bool kWide8>
-cudaError_t launch_extend(int blocks, bool pdl, cudaStream_t stream, const WaveBuffers& wb, int par) {
-  return launch_chained(k_extend<kBlock, kCount, kWide8>, blocks, kBlock, pdl, stream, wb, par);
-}
-
-template <int kBlock, bool kCount, bool kWide8>
-cudaError_t launch_shadow(int blocks, bool pdl, cudaStream_t stream, const WaveBuffers& wb) {
-  return launch_chained(k_shadow<kBlock, kCount, kWide8>, blocks, kBlock, pdl, stream, wb);
+// Grid of one instance of the path kernel on the current device: every block
+// resident. At most kMaxPathsPerSm path slots per SM, whatever `blocks` asks for.
+template <int kBlock, bool kMis, bool kGeneral>
+cudaError_t launch_path(const WaveBuffers& wb, int par, const LaunchShape& shape, cudaStream_t stream) {
+  constexpr std::size_t smem = kBlock / 32 * kWarpSmem<kMis, kGeneral>;
+  constexpr int kMaxBlocksPerSm = kMaxPathsPerSm / kWarpPaths / (kBlock / 32);
+  struct Grid {
+    cudaError_t err = cudaSuccess;
+    int sms = 0, per_sm = 0;
+  };
+  static const Grid grid = [] {
+    Grid g;
+    int dev = 0;
+    g.err = cudaFuncSetAttribute(k_path<kBlock, kMis, kGeneral>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem));
+    if (g.err == cudaSuccess) g.err = cudaGetDevice(&dev);
+    if (g.err == cudaSuccess) g.err = cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (g.err == cudaSuccess)
+      g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g.per_sm, k_path<kBlock, kMis, kGeneral>, kBlock, smem);
+    g.per_sm = g.per_sm < 1 ? 1 : (g.per_sm > kMaxBlocksPerSm ? kMaxBlocksPerSm : g.per_sm);
+    return g;
+  }();
+  if (grid.err != cudaSuccess) return grid.err;
+  int blocks = shape.extend_blocks > 0 ? shape.extend_blocks : grid.sms * grid.per_sm;
+  blocks = blocks < grid.sms * kMaxBlocksPerSm ? blocks : grid.sms * kMaxBlocksPerSm;
+  return launch_chained(k_path<kBlock, kMis, kGeneral>, blocks, kBlock, smem, shape.chained, stream, wb, par,
+                        shape.closest_tree, shape.shadow_tree);
 }
 
 template <int kBlock>
-cudaError_t stage_impl(Stage stage, const WaveBuffers& wb, int par, const LaunchShape& shape, bool count,
-                       cudaStream_t stream) {
-  const BlockCounts& bc = block_counts<kBlock>();
-  const bool pdl = shape.chained;
-  switch (stage) {
-    case Stage::Plan:
-      return launch_chained(k_plan, 1, kMaxGen, pdl, stream, wb, par);
-    case Stage::Extend: {
-      const bool w8 = shape.closest_tree == 8;
-      const int blocks = shape.extend_blocks ? shape.extend_blocks : bc.extend[count][w8];
-      if (count) return w8 ? launch_extend<kBlock, true, true>(blocks, pdl, stream, wb, par)
-                           : launch_extend<kBlock, true, false>(blocks, pdl, stream, wb, par);
-      return w8 ? launch_extend<kBlock, false, true>(blocks, pdl, stream, wb, par)
-                : launch_extend<kBlock, false, false>(blocks, pdl, stream, wb, par);
-    }
-    case Stage::Shade: {
-      const int blocks = shape.shade_blocks ? shape.shade_blocks : (shape.mis ? bc.shade_mis : bc.shade);
-      return shape.mis ? launch_chained(k_shade<kBlock, true>, blocks, kBlock, pdl, stream, wb, par)
-                       : launch_chained(k_shade<kBlock, false>, blocks, kBlock, pdl, stream, wb, par);
-    }
-    case Stage::Shadow: {
-      const bool w8 = shape.shadow_tree == 8;
-      const int blocks = shape.shadow_blocks ? shape.shadow_blocks : bc.shadow[count][w8];
-      if (count) return w8 ? launch_shadow<kBlock, true, true>(blocks, pdl, stream, wb)
-                           : launch_shadow<kBlock, true, false>(blocks, pdl, stream, wb);
-      return w8 ? launch_shadow<kBlock, false, true>(blocks, pdl, stream, wb)
-                : launch_shadow<kBlock, false, false>(blocks, pdl, stream, wb);
-    }
-  }
-  return cudaErrorInvalidValue;
+cudaError_t launch_path(const WaveBuffers& wb, int par, const LaunchShape& shape, cudaStream_t stream) {
+  if (shape.general) return shape.mis ? launch_path<kBlock, true, true>(wb, par, shape, stream)
+                                      : launch_path<kBlock, false, true>(wb, par, shape, stream);
+  return shape.mis ? launch_path<kBlock, true, false>(wb, par, shape, stream)
+                   : launch_path<kBlock, false, false>(wb, par, shape, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_stage(Stage stage, const WaveBuffers& wb, int parity, const LaunchShape& shape, bool count_traversal,
-                         cudaStream_t stream) {
-  switch (shape.extend_block) {
-    case 64: return stage_impl<64>(stage, wb, parity, shape, count_traversal, stream);
-    case 256: return stage_impl<256>(stage, wb, parity, shape, count_traversal, stream);
-    default: return stage_impl<128>(stage, wb, parity, shape, count_traversal, stream);
-  }
+cudaError_t launch_plan(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream) {
+  return launch_chained(k_plan, 1, kMaxGen, 0, shape.chained, stream, wb, parity);
 }
 
-cudaError_t launch_iteration(const WaveBuffers& wb, int parity, const LaunchShape& shape, bool count_traversal,
-                             cudaStream_t stream) {
-  for (Stage st : {Stage::Plan, Stage::Extend, Stage::Shade, Stage::Shadow}) {
-    const cudaError_t e = launch_stage(st, wb, parity, shape, count_traversal, stream);
-    if (e != cudaSuccess) return e;
+cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream) {
+  switch (shape.block) {
+    case 64: return launch_path<64>(wb, parity, shape, stream);
+    case 256: return launch_path<256>(wb, parity, shape, stream);
+    default: return launch_path<128>(wb, parity, shape, stream);
   }
-  return cudaSuccess;
 }
 
 cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const DevSegment& seg,

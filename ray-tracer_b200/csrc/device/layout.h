@@ -209,31 +209,31 @@ struct alignas(16) GenPlan {
   std::uint64_t start[kMaxGen];
 };
 
-// Path-state stream record, four float4 (SoA): one element per live path.
-//  a = (origin, sample id bits)         b = (direction, meta bits)
-//  c = (throughput, segment slot bits)  d = PCG32 state (lo, hi) and increment (lo, hi)
-// meta: depth (bits 0-11) | flags (bits 12-15) | job (bits 16-31)
-constexpr std::uint32_t kFlagSpecular = 1u << 12;
+// A path left from one iteration to the next, five float4 (SoA):
+//  a = (origin, radiance slot bits)     b = (direction, path word bits)
+//  c = (throughput, job bits)           d = PCG32 state (lo, hi) and increment (lo, hi)
+//  e = (radiance so far, pdf of the last diffuse bounce (MIS jobs only))
+// The path word's low 12 bits are the depth; the path kernel defines the rest.
 constexpr std::uint32_t kMetaDepthMask = 0xFFFu;
-constexpr int kMetaSceneShift = 16;
 constexpr int kMaxJobs = 65536;  // job descriptors addressable from the path record
 
 // Wavefront counters in device memory.
 struct alignas(16) WaveCounters {
-  std::uint32_t live[2];      // live paths at the start of an iteration (parity)
-  std::uint32_t n_extend;     // paths traced this iteration (live + new)
-  std::uint32_t n_shadow;     // shadow rays queued this iteration
-  std::uint32_t fetch[4];     // persistent-kernel work-fetch cursors
+  std::uint32_t live[2];      // paths left from the previous iteration (parity)
+  std::uint32_t n_items;      // paths of this iteration (left over + new)
+  std::uint32_t finish;       // 1: this iteration runs its paths to their end
+  std::uint32_t fetch;        // next item of this iteration's list
+  std::uint32_t pad[3];
   std::uint64_t iteration;    // plan launches so far (selects the snapshot ring slot)
   std::uint64_t generated;    // camera samples generated so far
   std::uint64_t rays;         // closest-hit rays traced
   std::uint64_t shadow_rays;
   std::uint64_t rr_terminated;
   std::uint64_t invalid_samples;
-  std::uint64_t node_visits;  // closest-hit kernel; filled only by the counting kernel variants
+  std::uint64_t node_visits;  // closest-hit walks; filled only by the general kernel instances
   std::uint64_t prim_tests;
   std::uint64_t sphere_tests; // of which spheres (32-byte reads; triangles read 48)
-  std::uint64_t shadow_node_visits;  // any-hit kernel, same meaning
+  std::uint64_t shadow_node_visits;  // any-hit walks, same meaning
   std::uint64_t shadow_prim_tests;
   std::uint64_t shadow_sphere_tests;
   std::uint32_t error;        // non-zero: a bounds check failed (index recorded in error_info)

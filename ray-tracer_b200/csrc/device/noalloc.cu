@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(kBlock) k_ray_closest_scratch(unsigned char* s
   TraceCount tc;
   RayHit h;
   if (brute) h = closest_brute<false>(job, f3(a), f3(b), a.w, b.w, tc);
-  else if (tree == 8) h = closest_hit8<kStack, kBlock, false>(job, f3(a), f3(b), a.w, b.w, stack, tc);
-  else h = closest_hit<kStack, kBlock, false>(job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack), tc);
+  else if (tree == 8) h = closest_hit8<kStack, kBlock, false>(job, f3(a), f3(b), a.w, b.w, stack + threadIdx.x, tc);
+  else h = closest_hit<kStack, kBlock, false>(job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack) + threadIdx.x, tc);
   refine_hit(job, f3(a), f3(b), h);
   const bool miss = h.word == kHitMiss;
   const bool plane = !miss && (h.word & kHitPlaneBit);

@@ -9,18 +9,20 @@
 
 namespace rtg {
 
-// Device buffers of one continuous wavefront (a pool of `capacity` path slots)
-// and the segment tables it draws new paths from.
+// Path slots resident per SM, at most: the paths left over by an iteration are no
+// more than this times the SMs.
+constexpr int kMaxPathsPerSm = 4096;
+
+// Device buffers of one continuous wavefront (iterations of at most `capacity`
+// paths) and the segment tables it draws new paths from.
 struct WaveBuffers {
+  // Paths left from one iteration to the next, by parity: min(capacity,
+  // kMaxPathsPerSm * SMs) records.
   float4* st_a[2];
   float4* st_b[2];
   float4* st_c[2];
   uint4* st_d[2];
-  float* st_e[2];  // pdf of the direction a diffuse bounce sampled (read only by MIS jobs)
-  float4* hits;
-  float4* sh_a;
-  float4* sh_b;
-  float4* sh_c;
+  float4* st_e[2];
   float4* radiance;            // one float4 per sample of every open segment
   WaveCounters* cnt;
   const RtgSceneDev* jobs;     // job descriptors, indexed by job slot
@@ -30,28 +32,24 @@ struct WaveBuffers {
   GenPlan* plan;               // this iteration's generation plan
   WaveSnapshot* ring;          // pinned, host-mapped snapshot ring
   std::uint32_t ring_size;
-  std::uint32_t capacity;      // at most 2^23 path slots
+  std::uint32_t capacity;      // paths an iteration may hold
 };
 
 struct LaunchShape {
-  int extend_blocks = 0, shade_blocks = 0, shadow_blocks = 0;  // 0 = derived from the SM count
-  int extend_block = 128;  // 64, 128 or 256
+  int extend_blocks = 0;   // grid of the path kernel (0 = every resident block)
+  int shade_blocks = 0, shadow_blocks = 0;  // kept for rtg_tuning; no kernel uses them
+  int block = 128;         // threads per block of the path kernel: 64, 128 or 256
   bool chained = true;     // programmatic dependent launch between the wavefront kernels
-  bool mis = false;        // a job with multiple importance sampling is open (shade kernel variant)
+  bool mis = false;        // a job with multiple importance sampling is open (kernel variant)
+  bool general = false;    // counting, an eight-wide walk, or a brute-force job: the general variant
   int closest_tree = 2;    // closest-hit walk: 2 the binary tree, 8 the compressed eight-wide tree
   int shadow_tree = 4;     // any-hit walk: 4 the four-wide tree, 8 the compressed eight-wide tree
 };
 
-enum class Stage { Plan, Extend, Shade, Shadow };
-
-// One stage of a wavefront iteration on `stream`; `parity` alternates 0/1
-// between iterations. The stages must run in the order plan, extend, shade, shadow.
-cudaError_t launch_stage(Stage stage, const WaveBuffers& wb, int parity, const LaunchShape& shape, bool count_traversal,
-                         cudaStream_t stream);
-
-// One wavefront iteration (plan, generate+extend, shade, shadow) on `stream`.
-cudaError_t launch_iteration(const WaveBuffers& wb, int parity, const LaunchShape& shape, bool count_traversal,
-                             cudaStream_t stream);
+// The two launches of a wavefront iteration on `stream`, in this order; `parity`
+// alternates 0/1 between iterations.
+cudaError_t launch_plan(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream);
+cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream);
 
 // Per-pixel reduction of a finished segment into its job's framebuffer.
 cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const DevSegment& seg,

@@ -87,7 +87,7 @@ AutotuneResult autotune(Engine& e, const std::vector<Engine::BatchJob>& jobs, co
       cfg.pool_paths = pool;
       e.reset_wave();
     }
-    cfg.shape.extend_block = block;
+    cfg.shape.block = block;
   };
   if (use_cache && cache_lookup(best.key, best)) {
     best.key = workload_signature(e, jobs);

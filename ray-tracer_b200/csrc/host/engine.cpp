@@ -75,6 +75,10 @@ constexpr int kLag = 2;    // iterations queued ahead of the snapshot being read
 constexpr std::size_t kStageBytes = std::size_t(1) << 20;  // host->device staging per iteration
 constexpr std::size_t kStagePiece = std::size_t(1) << 20;  // batch upload: bytes per host copy task
 constexpr int kJobSlots = 4096;  // job descriptors resident at once
+// Paths of one iteration, in pools: renders take several, since every iteration
+// ends with a wait for its slowest warps (0.03 ms on the sphere field, 0.1 ms on the
+// mix, 0.2 ms on the mesh); requests take one, so a preview waits less for its turn.
+constexpr std::uint32_t kRenderItems = 4;
 
 }  // namespace
 
@@ -192,7 +196,7 @@ void Engine::reset_wave() {
   if (wave_) {
     WaveBuffers& b = wave_->wb;
     for (int i = 0; i < 2; ++i) { dev_free(b.st_a[i]); dev_free(b.st_b[i]); dev_free(b.st_c[i]); dev_free(b.st_d[i]); dev_free(b.st_e[i]); }
-    dev_free(b.hits); dev_free(b.sh_a); dev_free(b.sh_b); dev_free(b.sh_c); dev_free(b.radiance); dev_free(b.cnt);
+    dev_free(b.radiance); dev_free(b.cnt);
     dev_free(wave_->jobs_dev); dev_free(wave_->segs_dev); dev_free(wave_->prog_dev);
     dev_free(wave_->gen_dev); dev_free(wave_->plan_dev);
     if (wave_->ring) cudaFreeHost(wave_->ring);
@@ -655,18 +659,17 @@ void Engine::ensure_wave() {
   Wave& W = *wave_;
   WaveBuffers& b = W.wb;
   const std::uint32_t P = cfg_.pool_paths;
-  b.capacity = P;
+  b.capacity = P * kRenderItems;
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  const std::uint32_t left = std::min<std::uint32_t>(P * kRenderItems, static_cast<std::uint32_t>(sms) * kMaxPathsPerSm);
   for (int i = 0; i < 2; ++i) {
-    b.st_a[i] = dev_alloc<float4>(P);
-    b.st_b[i] = dev_alloc<float4>(P);
-    b.st_c[i] = dev_alloc<float4>(P);
-    b.st_d[i] = dev_alloc<uint4>(P);
-    b.st_e[i] = dev_alloc<float>(P);
+    b.st_a[i] = dev_alloc<float4>(left);
+    b.st_b[i] = dev_alloc<float4>(left);
+    b.st_c[i] = dev_alloc<float4>(left);
+    b.st_d[i] = dev_alloc<uint4>(left);
+    b.st_e[i] = dev_alloc<float4>(left);
   }
-  b.hits = dev_alloc<float4>(P);
-  b.sh_a = dev_alloc<float4>(P);
-  b.sh_b = dev_alloc<float4>(P);
-  b.sh_c = dev_alloc<float4>(P);
   W.rad_cap = std::max<std::uint64_t>(1, std::min<std::uint64_t>(cfg_.max_pass_samples, 0xFFFFFFFFull));
   b.radiance = dev_alloc<float4>(W.rad_cap);
   W.rad_free.emplace(0, W.rad_cap);
@@ -840,6 +843,7 @@ int Engine::open_job(const JobSpec& spec, bool serving, PassCallback cb) {
   stage(W.jobs_dev + j.desc_slot, &d, sizeof(d));
   sc.jobs_open++;
   if (j.settings.light_sampling && j.settings.mis) ++mis_jobs_;
+  if (!j.settings.use_bvh) ++brute_jobs_;
   const int h = j.handle;
   jobs_.emplace(h, std::move(j));
   return h;
@@ -849,6 +853,7 @@ void Engine::close_job(Job& j) {
   Wave& W = *wave_;
   W.free_jobs.push_back(j.desc_slot);
   if (j.settings.light_sampling && j.settings.mis) --mis_jobs_;
+  if (!j.settings.use_bvh) --brute_jobs_;
   auto it = scenes_.find(j.scene_id);
   if (it != scenes_.end()) it->second->jobs_open--;
 }
@@ -955,7 +960,7 @@ void Engine::refill() {
     if (!s.used || s.complete || s.abandoned) continue;
     backlog[jobs_.at(s.job).priority] += s.d.count - std::min<std::uint64_t>(s.done, s.d.count);
   }
-  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * W.wb.capacity;
+  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderItems);
   while (true) {
     Job* best = nullptr;
     for (auto& kv : jobs_) {
@@ -1083,30 +1088,29 @@ void Engine::launch_one_iteration() {
   const int par = static_cast<int>(W.it & 1);
   const int r = static_cast<int>(W.it % kRing);
   const bool timed = cfg_.time_kernels;
-  const bool count = cfg_.count_traversal;
-  const Stage stages[4] = {Stage::Plan, Stage::Extend, Stage::Shade, Stage::Shadow};
+  W.wb.capacity = cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderItems);
   LaunchShape shape = cfg_.shape;
   shape.mis = mis_jobs_ > 0;
-  for (int k = 0; k < 4; ++k) {
-    if (timed) CK(cudaEventRecord(W.tev[2 * k], stream_));
-    CK(launch_stage(stages[k], W.wb, par, shape, count, stream_));
-    if (timed) CK(cudaEventRecord(W.tev[2 * k + 1], stream_));
-  }
+  shape.general = cfg_.count_traversal || brute_jobs_ > 0 || shape.closest_tree == 8 || shape.shadow_tree == 8;
+  if (timed) CK(cudaEventRecord(W.tev[0], stream_));
+  CK(launch_plan(W.wb, par, shape, stream_));
+  if (timed) CK(cudaEventRecord(W.tev[1], stream_));
+  CK(launch_paths(W.wb, par, shape, stream_));
   // After the whole iteration, so no event sits between chained kernels; the
   // plan's snapshot and this slot's staged copies are complete once it fires.
+  if (timed) CK(cudaEventRecord(W.tev[2], stream_));
   CK(cudaEventRecord(W.plan_ev[r], stream_));
   W.plan_recorded[r] = true;
   if (timed) {
-    CK(cudaEventSynchronize(W.tev[7]));
-    float ms[4] = {0, 0, 0, 0};
-    for (int k = 0; k < 4; ++k) CK(cudaEventElapsedTime(&ms[k], W.tev[2 * k], W.tev[2 * k + 1]));
-    stats_.plan_ms += ms[0];
-    stats_.extend_ms += ms[1];
-    stats_.shade_ms += ms[2];
-    stats_.shadow_ms += ms[3];
+    CK(cudaEventSynchronize(W.tev[2]));
+    float plan_ms = 0, path_ms = 0;
+    CK(cudaEventElapsedTime(&plan_ms, W.tev[0], W.tev[1]));
+    CK(cudaEventElapsedTime(&path_ms, W.tev[1], W.tev[2]));
+    stats_.plan_ms += plan_ms;
+    stats_.extend_ms += path_ms;
   }
   stats_.extend_launches++;
-  stats_.kernel_launches += 4;
+  stats_.kernel_launches += 2;
   stats_.iterations++;
   W.it++;
 }
@@ -1135,7 +1139,7 @@ void Engine::abort_all() {
   WaveCounters c{};
   CK(cudaMemcpy(&c, W.wb.cnt, sizeof(c), cudaMemcpyDeviceToHost));
   c.live[0] = c.live[1] = 0;
-  c.n_extend = c.n_shadow = 0;
+  c.n_items = 0;
   CK(cudaMemcpy(W.wb.cnt, &c, sizeof(c), cudaMemcpyHostToDevice));
   for (int k = 0; k < kMaxSegments; ++k)
     if (segs_[k].used) {

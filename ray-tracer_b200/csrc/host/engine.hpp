@@ -59,7 +59,8 @@ struct RenderStats {
   std::uint64_t shadow_node_visits = 0, shadow_prim_tests = 0, shadow_sphere_tests = 0;
   double elapsed_ms = 0;
   double device_ms = 0;  // CUDA events on the engine stream around the whole render
-  // Summed CUDA-event time of each kernel family (when kernel timing is on).
+  // Summed CUDA-event time of each kernel family (when kernel timing is on); the
+  // path kernel's is extend_ms, with the shading and the shadow rays in it.
   double extend_ms = 0, shade_ms = 0, shadow_ms = 0, accumulate_ms = 0, direct_ms = 0, plan_ms = 0;
   std::uint64_t extend_launches = 0;
 };
@@ -105,7 +106,7 @@ struct GpuFrame {
 using PassCallback = std::function<void(const RenderProgress&)>;
 
 struct EngineConfig {
-  std::uint32_t pool_paths = 1u << 20;          // wavefront path slots (<= 2^23)
+  std::uint32_t pool_paths = 1u << 20;          // paths of one wavefront iteration (<= 2^23)
   std::uint64_t max_pass_samples = 1ull << 27;  // radiance slots shared by the open segments
   std::uint32_t backlog_pools = 3;              // keep this many pools of samples open for generation
   LaunchShape shape;
@@ -333,6 +334,7 @@ class Engine {
   std::uint64_t job_seq_ = 0;
   std::size_t serve_open_ = 0;
   int mis_jobs_ = 0;               // open jobs with multiple importance sampling
+  int brute_jobs_ = 0;             // open jobs without a BVH (use_bvh = false)
   bool gen_dirty_ = false;
   WaveCounters last_counters_{};   // from the latest snapshot
   WaveCounters base_counters_{};   // at the start of the current render
