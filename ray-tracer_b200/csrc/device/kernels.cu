@@ -19,7 +19,6 @@
 // pixel's samples into the double framebuffer in sample order (Framebuffer::add,
 // include/raytracer/rendering/framebuffer.hpp:31), passes of one render in order.
 #include <cfloat>
-#include <type_traits>
 
 #include "device/shade.cuh"
 #include "device/wave.h"
@@ -240,13 +239,16 @@ struct alignas(16) WarpPaths {
   std::uint8_t idle[kWarpPaths], ready[kWarpPaths], lit[kWarpPaths];
 };
 
-__device__ __forceinline__ float3 get3(const float (&v)[3][kWarpPaths], int p) { return f3(v[0][p], v[1][p], v[2][p]); }
-__device__ __forceinline__ void set3(float (&v)[3][kWarpPaths], int p, float3 x) {
+template <int kSlots>
+__device__ __forceinline__ float3 get3(const float (&v)[3][kSlots], int p) { return f3(v[0][p], v[1][p], v[2][p]); }
+template <int kSlots>
+__device__ __forceinline__ void set3(float (&v)[3][kSlots], int p, float3 x) {
   v[0][p] = x.x;
   v[1][p] = x.y;
   v[2][p] = x.z;
 }
-__device__ __forceinline__ void add3(float (&v)[3][kWarpPaths], int p, float3 x) {
+template <int kSlots>
+__device__ __forceinline__ void add3(float (&v)[3][kSlots], int p, float3 x) {
   v[0][p] += x.x;
   v[1][p] += x.y;
   v[2][p] += x.z;
@@ -590,97 +592,202 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
 }
 
 // ---------------------------------------------------------------------------
-// The walks of the direct integrator: the eight-wide tree (kWide8) or the binary
-// (closest hit) and four-wide (any hit) trees, or brute force when the job asks for
-// it. `column` is this thread's stack.
-template <bool kWide8>
-using StackEntry = std::conditional_t<kWide8, uint2, int>;
-
-template <int kBlock, bool kWide8>
-__device__ __forceinline__ RayHit trace_closest(const RtgSceneDev& J, float3 o, float3 d, StackEntry<kWide8>* column,
-                                                TraceCount& tc) {
-  if (!J.use_bvh) return closest_brute<false>(J, o, d, kRayTMin, FLT_MAX, tc);
-  if constexpr (kWide8) return closest_hit8<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, column, tc);
-  else return closest_hit<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, column, tc);
-}
-
-template <int kBlock, bool kWide8>
-__device__ __forceinline__ bool trace_any(const RtgSceneDev& J, float3 o, float3 d, float tmax,
-                                          StackEntry<kWide8>* column, TraceCount& tc) {
-  if (!J.use_bvh) return any_brute(J, o, d, kRayTMin, tmax);
-  if constexpr (kWide8) return any_hit8<kStackSmem, kBlock, false>(J, o, d, kRayTMin, tmax, column, tc);
-  else return any_hit4<kStackSmem, kBlock, false>(J, o, d, kRayTMin, tmax, column, tc);
-}
-
-// ---------------------------------------------------------------------------
 // Whitted-style direct integrator (src/rendering/integrator.cpp:141-174): every
 // light at diffuse hits, recursion through metal, and a deterministic Fresnel
-// split at dielectrics. The recursion becomes a depth-first walk with an explicit
-// stack of pending refraction branches, which keeps the reference's RNG draw order.
+// split at dielectrics. The recursion becomes a depth-first walk of each sample's
+// tree with a stack of pending refraction branches, which keeps the reference's RNG
+// draw order.
+//
+// Scheduled like the path kernel: each warp holds kDirectPaths samples in shared
+// memory; `ready` ones have a ray to trace, `lit` ones the next light of a diffuse
+// hit to sample and test. The surface of a lit sample is made again from its hit for
+// each light, which costs less than keeping it. Pending branches are in device
+// memory: at most one per level, so min(max depth, kDirectStack) records a sample.
+// Bound by the serial walk of the largest trees: of the 7.3 ms that the mesh takes
+// at 640x360x16, depth 8, some 4.3 ms are the longest sample's chain (that is also
+// what one sample a pixel takes), 2.5 ms the throughput. One thread per whole sample,
+// where lanes wait for the longest tree of their warp, measured 8.4 ms with the same
+// walk. First in, first out queues, which advance the long samples sooner, measured
+// 7.6 ms: they lose more coherence than tail.
 constexpr int kDirectStack = 48;
+constexpr int kDirectPaths = 48;
+constexpr int kPendingRows = 3;  // float4 rows of a pending branch: (o, d.x), (d.yz, w.xy), (w.z, depth)
 
-struct Pending {
-  float3 o, d, w;
-  int depth;
+struct alignas(16) DirectPaths {
+  float o[3][kDirectPaths], d[3][kDirectPaths], w[3][kDirectPaths];  // ray and its weight
+  float light[3][kDirectPaths];                                      // radiance so far
+  float sum[3][kDirectPaths];                                        // of the lights at the current hit
+  float f[3][kDirectPaths], li[3][kDirectPaths];                     // BRDF and light of the shadow ray in flight
+  float hit[4][kDirectPaths];
+  std::uint32_t rng[4][kDirectPaths];
+  std::uint32_t sample[kDirectPaths];
+  std::uint16_t depth[kDirectPaths];
+  std::int32_t light_index[kDirectPaths];
+  std::uint8_t pending[kDirectPaths];                                // refraction branches on the stack
+  std::uint8_t idle[kDirectPaths], ready[kDirectPaths], lit[kDirectPaths];
 };
 
-template <int kBlock, bool kWide8>
-__device__ __forceinline__ float3 direct_light_all(const RtgSceneDev& J, const DevMaterial& m, const Surface& s,
-                                                   Pcg& rng, StackEntry<kWide8>* stack, TraceCount& tc,
-                                                   std::uint64_t& shadow_rays) {
-  float3 sum = f3(0.f, 0.f, 0.f);
-  for (int li = 0; li < J.n_lights; ++li) {
-    const LightSample ls = sample_light(J.lights + li, s, rng);
-    if (!ls.valid) continue;
-    const float3 f = brdf_cos(m, s, ls.wi);
-    if (is_zero3(f) || is_zero3(ls.li_over_pdf)) continue;
-    const ShadowRay sr = shadow_ray(s, ls);
-    ++shadow_rays;
-    const bool blocked = trace_any<kBlock, kWide8>(J, sr.o, sr.d, sr.tmax, stack, tc);
-    if (!blocked) sum = sum + f * ls.li_over_pdf;
-  }
-  return sum;
-}
+template <bool kGeneral>
+constexpr std::size_t kDirectWarpSmem = sizeof(DirectPaths) + sizeof(typename Walk<kGeneral>::Entry) * 32 * kPathStack;
 
-template <int kBlock, bool kWide8>
-__global__ void __launch_bounds__(kBlock) k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance,
-                                                   WaveCounters* C) {
-  __shared__ StackEntry<kWide8> stack[kStackSmem * kBlock];
-  StackEntry<kWide8>* const column = stack + threadIdx.x;
-  TraceCount tc;
-  std::uint64_t rays = 0, shadow_rays = 0;
+template <int kBlock, bool kGeneral>
+__global__ void __launch_bounds__(kBlock, kPathThreads / kBlock)
+k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, WaveCounters* C, float4* stack_rows,
+         int stack_depth, int tree) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using Entry = typename Walk<kGeneral>::Entry;
+  const int lane = threadIdx.x & 31;
+  unsigned char* const mine = smem + (threadIdx.x >> 5) * kDirectWarpSmem<kGeneral>;
+  DirectPaths& S = *reinterpret_cast<DirectPaths*>(mine);
+  Entry* const column = reinterpret_cast<Entry*>(mine + sizeof(DirectPaths)) + lane;
+  // Pending branches of this warp's slot p start at row (first_slot + p) * stack_depth * kPendingRows.
+  const std::size_t first_slot =
+      (static_cast<std::size_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5)) * kDirectPaths;
+#pragma unroll 1
+  for (int k = lane; k < kDirectPaths; k += 32) S.idle[k] = static_cast<std::uint8_t>(k);
+  __syncwarp();
   const RtgSceneDev& J = *job;
-  const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * kBlock;
-  for (std::uint64_t w = static_cast<std::uint64_t>(blockIdx.x) * kBlock + threadIdx.x; w < seg.count; w += stride) {
-    CameraSample cs = camera_sample(J, seg, w);
-    Pending todo[kDirectStack];
-    int sp = 0;
-    Pending cur{cs.o, cs.d, f3(1.f, 1.f, 1.f), 0};
-    float3 L = f3(0.f, 0.f, 0.f);
-    bool overflow = false;
-    while (true) {
-      ++rays;
-      const RayHit h = trace_closest<kBlock, kWide8>(J, cur.o, cur.d, column, tc);
-      bool next = false;
+  const std::uint32_t count = static_cast<std::uint32_t>(seg.count);  // under 2^32 (the radiance slots are)
+  const unsigned below = (1u << lane) - 1u;
+  Walk<kGeneral> walk;
+  TraceCount tc;
+  std::uint32_t rays = 0, shadow_rays = 0;  // of the warp
+  bool overflow = false, more = true;
+  int n_idle = kDirectPaths, n_ready = 0, n_lit = 0;
+  while (true) {
+    const int n_new = more ? n_idle : 0;
+    enum { kLight, kTrace, kNew } step;
+    if (n_lit >= 32) step = kLight;
+    else if (n_ready >= 32) step = kTrace;
+    else if (n_new >= 32) step = kNew;
+    else {
+      if ((n_lit | n_ready | n_new) == 0) break;
+      step = n_lit >= n_ready && n_lit >= n_new ? kLight : (n_ready >= n_new ? kTrace : kNew);
+    }
+    bool on = false, ray = false;  // the lane has a sample; the sample has a ray to trace in this step
+    int p = 0;
+    float3 o = f3(0.f, 0.f, 0.f), d = o;
+    float tmax = FLT_MAX;
+    if (step == kLight) {
+      const int take = min(n_lit, 32);
+      n_lit -= take;
+      on = lane < take;
+      if (on) {
+        p = S.lit[n_lit + lane];
+        const Surface s = make_surface(J, get3(S.o, p), get3(S.d, p),
+                                       RayHit{S.hit[0][p], __float_as_uint(S.hit[1][p]), S.hit[2][p], S.hit[3][p]});
+        Pcg rng{ld_u64(S.rng[0][p], S.rng[1][p]), ld_u64(S.rng[2][p], S.rng[3][p])};
+        const LightSample ls = sample_light(J.lights + S.light_index[p], s, rng);
+        S.rng[0][p] = static_cast<std::uint32_t>(rng.state);
+        S.rng[1][p] = static_cast<std::uint32_t>(rng.state >> 32);
+        if (ls.valid) {
+          const float3 f = brdf_cos(J.materials[s.material], s, ls.wi);
+          if (!is_zero3(f) && !is_zero3(ls.li_over_pdf)) {
+            const ShadowRay sr = shadow_ray(s, ls);
+            o = sr.o;
+            d = sr.d;
+            tmax = sr.tmax;
+            set3(S.f, p, f);
+            set3(S.li, p, ls.li_over_pdf);
+            ray = true;
+          }
+        }
+      }
+      shadow_rays += __popc(__ballot_sync(kFull, ray));
+    } else if (step == kTrace) {
+      const int take = min(n_ready, 32);
+      n_ready -= take;
+      on = ray = lane < take;
+      rays += take;
+      if (on) {
+        p = S.ready[n_ready + lane];
+        o = get3(S.o, p);
+        d = get3(S.d, p);
+      }
+    } else {
+      int take = min(n_idle, 32);
+      std::uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&C->direct_fetch, static_cast<std::uint32_t>(take));
+      base = __shfl_sync(kFull, base, 0);
+      if (base >= count) {
+        more = false;
+        continue;
+      }
+      if (count - base < static_cast<std::uint32_t>(take)) {
+        take = static_cast<int>(count - base);
+        more = false;
+      }
+      n_idle -= take;
+      on = ray = lane < take;
+      rays += take;
+      if (on) {
+        p = S.idle[n_idle + lane];
+        const CameraSample cs = camera_sample(J, seg, base + lane);
+        o = cs.o;
+        d = cs.d;
+        set3(S.o, p, o);
+        set3(S.d, p, d);
+        set3(S.w, p, f3(1.f, 1.f, 1.f));
+        set3(S.light, p, f3(0.f, 0.f, 0.f));
+        S.rng[0][p] = static_cast<std::uint32_t>(cs.rng.state);
+        S.rng[1][p] = static_cast<std::uint32_t>(cs.rng.state >> 32);
+        S.rng[2][p] = static_cast<std::uint32_t>(cs.rng.inc);
+        S.rng[3][p] = static_cast<std::uint32_t>(cs.rng.inc >> 32);
+        S.sample[p] = cs.sample;
+        S.depth[p] = 0;
+        S.pending[p] = 0;
+      }
+    }
+    __syncwarp();
+    RayHit h{tmax, kHitMiss, 0.f, 0.f};
+    if (ray) h = walk(J, o, d, tmax, step == kLight, column, tree, tc);
+    // What the sample does next: trace S.o, S.d; sample a light; or neither, and then
+    // a pending branch is next, or the sample is done.
+    bool go = false, lit = false;
+    if (on && step == kLight) {
+      if (ray && h.word == kHitMiss) {
+        const float3 sum = get3(S.sum, p) + get3(S.f, p) * get3(S.li, p);
+        set3(S.sum, p, sum);
+      }
+      const int next = S.light_index[p] + 1;
+      S.light_index[p] = next;
+      lit = next < J.n_lights;
+      if (!lit) set3(S.light, p, get3(S.light, p) + get3(S.w, p) * get3(S.sum, p));
+    } else if (on) {
+      const float3 w = get3(S.w, p);
       if (h.word == kHitMiss) {
-        L = L + cur.w * background(J, cur.d);
+        set3(S.light, p, get3(S.light, p) + w * background(J, d));
       } else {
-        const Surface s = make_surface(J, cur.o, cur.d, h);
+        const Surface s = make_surface(J, o, d, h);
         const DevMaterial m = J.materials[s.material];
-        L = L + cur.w * emitted(m, s.front);
-        if (cur.depth < J.max_depth) {
+        set3(S.light, p, get3(S.light, p) + w * emitted(m, s.front));
+        const int depth = S.depth[p];
+        if (depth < J.max_depth) {
           const std::uint32_t kind = kind_of(m);
           if (kind == kLambertian) {
-            L = L + cur.w * direct_light_all<kBlock, kWide8>(J, m, s, cs.rng, column, tc, shadow_rays);
+            if (J.n_lights > 0) {
+              S.hit[0][p] = h.t;
+              S.hit[1][p] = __uint_as_float(h.word);
+              S.hit[2][p] = h.b1;
+              S.hit[3][p] = h.b2;
+              set3(S.sum, p, f3(0.f, 0.f, 0.f));
+              S.light_index[p] = 0;
+              lit = true;
+            }
           } else if (kind == kMetal) {
+            Pcg rng{ld_u64(S.rng[0][p], S.rng[1][p]), ld_u64(S.rng[2][p], S.rng[3][p])};
             Scatter sr;
-            if (scatter(m, cur.d, s, cs.rng, sr)) {
-              cur = Pending{spawn_towards(s.p, s.gn, sr.dir), sr.dir, cur.w * f3(m.colour_a), cur.depth + 1};
-              next = true;
+            go = scatter(m, d, s, rng, sr);
+            S.rng[0][p] = static_cast<std::uint32_t>(rng.state);
+            S.rng[1][p] = static_cast<std::uint32_t>(rng.state >> 32);
+            if (go) {
+              set3(S.o, p, spawn_towards(s.p, s.gn, sr.dir));
+              set3(S.d, p, sr.dir);
+              set3(S.w, p, w * f3(m.colour_a));
             }
           } else if (kind == kDielectric) {
             const float ior = m.head.z;
-            const float3 in = unit_or(cur.d, f3(0.f, 0.f, 0.f));
+            const float3 in = unit_or(d, f3(0.f, 0.f, 0.f));
             const float eta = s.front ? 1.f / ior : ior;
             const float cos_i = fminf(-dot3(in, s.n), 1.f);
             float3 refr;
@@ -688,28 +795,59 @@ __global__ void __launch_bounds__(kBlock) k_direct(const RtgSceneDev* __restrict
             const float F = can ? schlick(cos_i, eta) : 1.f;
             const float3 tint = f3(m.colour_a);
             if (can) {
-              if (sp < kDirectStack) {
+              const int sp = S.pending[p];
+              if (sp < stack_depth) {
                 const float3 td = unit_or(refr, f3(0.f, 0.f, 0.f));
-                todo[sp++] = Pending{spawn_towards(s.p, s.gn, td), td, cur.w * tint * (1.f - F), cur.depth + 1};
+                const float3 to = spawn_towards(s.p, s.gn, td), tw = w * tint * (1.f - F);
+                float4* const row = stack_rows + ((first_slot + p) * stack_depth + sp) * kPendingRows;
+                row[0] = make_float4(to.x, to.y, to.z, td.x);
+                row[1] = make_float4(td.y, td.z, tw.x, tw.y);
+                row[2] = make_float4(tw.z, __int_as_float(depth + 1), 0.f, 0.f);
+                S.pending[p] = static_cast<std::uint8_t>(sp + 1);
               } else {
                 overflow = true;
               }
             }
             const float3 rd = reflect3(in, s.n);
-            cur = Pending{spawn_towards(s.p, s.gn, rd), rd, cur.w * tint * F, cur.depth + 1};
-            next = true;
+            set3(S.o, p, spawn_towards(s.p, s.gn, rd));
+            set3(S.d, p, rd);
+            set3(S.w, p, w * tint * F);
+            go = true;
           }
+          if (go) S.depth[p] = static_cast<std::uint16_t>(depth + 1);
         }
       }
-      if (next) continue;
-      if (sp == 0) break;
-      cur = todo[--sp];
     }
-    if (overflow) atomicExch(&C->error, 2u);
-    radiance[cs.sample] = make_float4(L.x, L.y, L.z, 0.f);
+    if (on && !go && !lit && S.pending[p] > 0) {
+      const int sp = S.pending[p] - 1;
+      const float4* const row = stack_rows + ((first_slot + p) * stack_depth + sp) * kPendingRows;
+      const float4 a = row[0], b = row[1], c = row[2];
+      set3(S.o, p, f3(a.x, a.y, a.z));
+      set3(S.d, p, f3(a.w, b.x, b.y));
+      set3(S.w, p, f3(b.z, b.w, c.x));
+      S.depth[p] = static_cast<std::uint16_t>(__float_as_int(c.y));
+      S.pending[p] = static_cast<std::uint8_t>(sp);
+      go = true;
+    }
+    const bool end = on && !go && !lit;
+    if (end) {
+      const float3 l = get3(S.light, p);
+      radiance[S.sample[p]] = make_float4(l.x, l.y, l.z, 0.f);
+    }
+    const unsigned m_lit = __ballot_sync(kFull, lit), m_ready = __ballot_sync(kFull, go), m_end = __ballot_sync(kFull, end);
+    if (lit) S.lit[n_lit + __popc(m_lit & below)] = static_cast<std::uint8_t>(p);
+    if (go) S.ready[n_ready + __popc(m_ready & below)] = static_cast<std::uint8_t>(p);
+    if (end) S.idle[n_idle + __popc(m_end & below)] = static_cast<std::uint8_t>(p);
+    n_lit += __popc(m_lit);
+    n_ready += __popc(m_ready);
+    n_idle += __popc(m_end);
+    __syncwarp();
   }
-  warp_add_u64(rays, &C->rays);
-  warp_add_u64(shadow_rays, &C->shadow_rays);
+  if (overflow) atomicExch(&C->error, 2u);
+  if (lane == 0) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(&C->rays), static_cast<unsigned long long>(rays));
+    atomicAdd(reinterpret_cast<unsigned long long*>(&C->shadow_rays), static_cast<unsigned long long>(shadow_rays));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -817,17 +955,6 @@ __global__ void __launch_bounds__(kBlock) k_ray_any(const RtgSceneDev* __restric
   out[i] = hit ? 1u : 0u;
 }
 
-// Blocks per SM the persistent kernels are launched with (occupancy-derived, cached).
-template <class K>
-int persistent_blocks(K kernel, int block) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
-  if (per_sm < 1) per_sm = 1;
-  return sms * per_sm;
-}
-
 // Launch with programmatic stream serialization (when enabled) so the kernel's
 // blocks are scheduled while the previous wavefront kernel drains.
 template <class... KArgs, class... Args>
@@ -846,28 +973,30 @@ cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block, std::s
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Grid of one instance of the path kernel on the current device: every block
-// resident. At most kMaxPathsPerSm path slots per SM, whatever `blocks` asks for.
+// Persistent grid of a kernel on the current device: every resident block, at most
+// `cap` an SM.
+struct Grid {
+  cudaError_t err = cudaSuccess;
+  int sms = 0, per_sm = 0;
+};
+template <class K>
+Grid resident_grid(K kernel, int block, std::size_t smem, int cap) {
+  Grid g;
+  int dev = 0;
+  g.err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (g.err == cudaSuccess) g.err = cudaGetDevice(&dev);
+  if (g.err == cudaSuccess) g.err = cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, dev);
+  if (g.err == cudaSuccess) g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g.per_sm, kernel, block, smem);
+  g.per_sm = g.per_sm < 1 ? 1 : (g.per_sm > cap ? cap : g.per_sm);
+  return g;
+}
+
+// At most kMaxPathsPerSm path slots per SM, whatever extend_blocks asks for.
 template <int kBlock, bool kMis, bool kGeneral>
 cudaError_t launch_path(const WaveBuffers& wb, int par, const LaunchShape& shape, cudaStream_t stream) {
   constexpr std::size_t smem = kBlock / 32 * kWarpSmem<kMis, kGeneral>;
   constexpr int kMaxBlocksPerSm = kMaxPathsPerSm / kWarpPaths / (kBlock / 32);
-  struct Grid {
-    cudaError_t err = cudaSuccess;
-    int sms = 0, per_sm = 0;
-  };
-  static const Grid grid = [] {
-    Grid g;
-    int dev = 0;
-    g.err = cudaFuncSetAttribute(k_path<kBlock, kMis, kGeneral>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem));
-    if (g.err == cudaSuccess) g.err = cudaGetDevice(&dev);
-    if (g.err == cudaSuccess) g.err = cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g.err == cudaSuccess)
-      g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g.per_sm, k_path<kBlock, kMis, kGeneral>, kBlock, smem);
-    g.per_sm = g.per_sm < 1 ? 1 : (g.per_sm > kMaxBlocksPerSm ? kMaxBlocksPerSm : g.per_sm);
-    return g;
-  }();
+  static const Grid grid = resident_grid(k_path<kBlock, kMis, kGeneral>, kBlock, smem, kMaxBlocksPerSm);
   if (grid.err != cudaSuccess) return grid.err;
   int blocks = shape.extend_blocks > 0 ? shape.extend_blocks : grid.sms * grid.per_sm;
   blocks = blocks < grid.sms * kMaxBlocksPerSm ? blocks : grid.sms * kMaxBlocksPerSm;
@@ -904,17 +1033,38 @@ cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance, WaveCounters* cnt,
-                          bool wide8, cudaStream_t stream) {
-  static int blocks[2] = {0, 0};
-  if (wide8) {
-    if (!blocks[1]) blocks[1] = persistent_blocks(k_direct<128, true>, 128);
-    k_direct<128, true><<<blocks[1], 128, 0, stream>>>(job_dev, seg, radiance, cnt);
-  } else {
-    if (!blocks[0]) blocks[0] = persistent_blocks(k_direct<128, false>, 128);
-    k_direct<128, false><<<blocks[0], 128, 0, stream>>>(job_dev, seg, radiance, cnt);
-  }
+namespace {
+constexpr int kDirectBlock = 128;
+template <bool kGeneral>
+const Grid& direct_grid() {
+  static const Grid grid = resident_grid(k_direct<kDirectBlock, kGeneral>, kDirectBlock,
+                                         kDirectBlock / 32 * kDirectWarpSmem<kGeneral>, kPathThreads / kDirectBlock);
+  return grid;
+}
+
+template <bool kGeneral>
+cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance,
+                                   WaveCounters* cnt, float4* pending, int pending_depth, int tree, cudaStream_t stream) {
+  const Grid& grid = direct_grid<kGeneral>();
+  if (grid.err != cudaSuccess) return grid.err;
+  const cudaError_t e = cudaMemsetAsync(&cnt->direct_fetch, 0, sizeof(cnt->direct_fetch), stream);
+  if (e != cudaSuccess) return e;
+  k_direct<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, kDirectBlock / 32 * kDirectWarpSmem<kGeneral>,
+                                     stream>>>(job_dev, seg, radiance, cnt, pending, pending_depth, tree);
   return cudaGetLastError();
+}
+}  // namespace
+
+int direct_pending_depth(int max_depth) { return max_depth < kDirectStack ? max_depth : kDirectStack; }
+
+std::size_t direct_pending_bytes(int sms, int pending_depth) {
+  return static_cast<std::size_t>(sms) * (kPathThreads / 32) * kDirectPaths * pending_depth * kPendingRows * sizeof(float4);
+}
+
+cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance, WaveCounters* cnt,
+                          float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream) {
+  return general ? launch_direct_instance<true>(job_dev, seg, radiance, cnt, pending, pending_depth, tree, stream)
+                 : launch_direct_instance<false>(job_dev, seg, radiance, cnt, pending, pending_depth, tree, stream);
 }
 
 cudaError_t launch_resolve(const double* fb_sum, const std::uint32_t* fb_count, std::uint64_t pixels, int tone_map,

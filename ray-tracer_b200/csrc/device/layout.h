@@ -223,7 +223,8 @@ struct alignas(16) WaveCounters {
   std::uint32_t n_items;      // paths of this iteration (left over + new)
   std::uint32_t finish;       // 1: this iteration runs its paths to their end
   std::uint32_t fetch;        // next item of this iteration's list
-  std::uint32_t pad[3];
+  std::uint32_t direct_fetch; // next sample of a direct-integrator pass
+  std::uint32_t pad[2];
   std::uint64_t iteration;    // plan launches so far (selects the snapshot ring slot)
   std::uint64_t generated;    // camera samples generated so far
   std::uint64_t rays;         // closest-hit rays traced

@@ -1,6 +1,7 @@
 #pragma once
 // Host-visible launch interface of the sm_100a kernels (kernels.cu). Plain C++:
 // no CUDA syntax, so the C++20 host code can include it.
+#include <cstddef>
 #include <cstdint>
 
 #include <cuda_runtime_api.h>
@@ -55,10 +56,15 @@ cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& s
 cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const DevSegment& seg,
                               const float4* radiance, cudaStream_t stream);
 
-// Direct (Whitted) integrator over one whole segment: whole samples per thread
-// (depth-first with an explicit stack). Writes each sample's radiance slot.
+// Direct (Whitted) integrator over one whole segment. Writes each sample's radiance
+// slot. `pending` holds direct_pending_bytes(SMs, pending_depth) bytes for the
+// samples' pending refraction branches, pending_depth of them a sample
+// (direct_pending_depth of the job's maximum depth; 0 for a scene without dielectrics,
+// whose samples have none). `general`: an eight-wide walk (tree 8) or brute force.
+int direct_pending_depth(int max_depth);
+std::size_t direct_pending_bytes(int sms, int pending_depth);
 cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance, WaveCounters* cnt,
-                          bool wide8, cudaStream_t stream);
+                          float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream);
 
 // Framebuffer means (mean_out, 3 doubles per pixel) and/or their tone-mapped
 // sRGB encoding (rgb8, 3 bytes per pixel); either output may be null.

@@ -104,6 +104,9 @@ struct Engine::Wave {
   std::vector<int> free_segs;
   std::uint32_t snapshot_slots = 0;
   std::uint32_t hi_slot = 0;           // segment slots ever used are below this
+  int sms = 0;
+  float4* direct_pending = nullptr;    // pending branches of the direct integrator (grown on demand)
+  std::size_t direct_pending_bytes = 0;
   std::uint64_t stall = 0;             // snapshots without a finished sample while work is open
   std::uint64_t last_done_sum = 0;
 
@@ -198,7 +201,7 @@ void Engine::reset_wave() {
     for (int i = 0; i < 2; ++i) { dev_free(b.st_a[i]); dev_free(b.st_b[i]); dev_free(b.st_c[i]); dev_free(b.st_d[i]); dev_free(b.st_e[i]); }
     dev_free(b.radiance); dev_free(b.cnt);
     dev_free(wave_->jobs_dev); dev_free(wave_->segs_dev); dev_free(wave_->prog_dev);
-    dev_free(wave_->gen_dev); dev_free(wave_->plan_dev);
+    dev_free(wave_->gen_dev); dev_free(wave_->plan_dev); dev_free(wave_->direct_pending);
     if (wave_->ring) cudaFreeHost(wave_->ring);
     if (wave_->staging) cudaFreeHost(wave_->staging);
     for (auto& e : wave_->plan_ev) if (e) cudaEventDestroy(e);
@@ -660,9 +663,8 @@ void Engine::ensure_wave() {
   WaveBuffers& b = W.wb;
   const std::uint32_t P = cfg_.pool_paths;
   b.capacity = P * kRenderItems;
-  int sms = 0;
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-  const std::uint32_t left = std::min<std::uint32_t>(P * kRenderItems, static_cast<std::uint32_t>(sms) * kMaxPathsPerSm);
+  CK(cudaDeviceGetAttribute(&W.sms, cudaDevAttrMultiProcessorCount, device_));
+  const std::uint32_t left = std::min<std::uint32_t>(P * kRenderItems, static_cast<std::uint32_t>(W.sms) * kMaxPathsPerSm);
   for (int i = 0; i < 2; ++i) {
     b.st_a[i] = dev_alloc<float4>(left);
     b.st_b[i] = dev_alloc<float4>(left);
@@ -912,6 +914,18 @@ bool Engine::run_direct_pass(Job& j) {
   Wave& W = *wave_;
   const std::uint32_t k = next_pass_size(j);
   const std::uint64_t count = j.pixels * k;
+  int pending_depth = 0;
+  for (const Material& m : scene(j.scene_id).host->materials)
+    if (std::holds_alternative<Dielectric>(m)) pending_depth = direct_pending_depth(j.settings.max_depth);
+  const std::size_t pending_bytes = direct_pending_bytes(W.sms, pending_depth);
+  if (W.direct_pending_bytes < pending_bytes) {
+    CK(cudaStreamSynchronize(stream_));
+    dev_free(W.direct_pending);
+    W.direct_pending = nullptr;
+    W.direct_pending_bytes = 0;
+    W.direct_pending = dev_alloc<float4>(pending_bytes / sizeof(float4));
+    W.direct_pending_bytes = pending_bytes;
+  }
   std::uint64_t at = 0;
   if (!W.rad_alloc(count, at)) return false;  // retried once radiance space frees up
   DevSegment d{};
@@ -922,7 +936,8 @@ bool Engine::run_direct_pass(Job& j) {
   d.sample_base = at;
   const bool timed = cfg_.time_kernels;
   if (timed) CK(cudaEventRecord(W.tev[8], stream_));
-  CK(launch_direct(W.jobs_dev + j.desc_slot, d, W.wb.radiance, W.wb.cnt, cfg_.shape.closest_tree == 8, stream_));
+  CK(launch_direct(W.jobs_dev + j.desc_slot, d, W.wb.radiance, W.wb.cnt, W.direct_pending, pending_depth,
+                   !j.settings.use_bvh || cfg_.shape.closest_tree == 8, cfg_.shape.closest_tree, stream_));
   if (timed) CK(cudaEventRecord(W.tev[9], stream_));
   CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, d, W.wb.radiance, stream_));
   stats_.kernel_launches += 2;
