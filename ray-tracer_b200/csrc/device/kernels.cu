@@ -264,17 +264,19 @@ struct Walk;
 template <>
 struct Walk<false> {
   using Entry = int;
-  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* column,
+  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* stack,
                                                int, TraceCount& tc) {
-    return walk_binary<kPathStack, 32, false>(J, o, d, kRayTMin, tmax, any, column, tc);
+    return walk_binary<kPathStack, 32, false>(J, o, d, kRayTMin, tmax, any, stack + (threadIdx.x & 31), tc);
   }
 };
 
 template <>
 struct Walk<true> {
   using Entry = uint2;
-  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* column,
+  __device__ __forceinline__ RayHit operator()(const RtgSceneDev& J, float3 o, float3 d, float tmax, bool any, Entry* stack,
                                                int tree, TraceCount& tc) {
+    // The columns of the two kinds of walk differ: their entries have different sizes.
+    Entry* const column = stack + (threadIdx.x & 31);
     RayHit found{tmax, 0u, 0.f, 0.f};
     if (!J.use_bvh) {
       if (!any) return closest_brute<true>(J, o, d, kRayTMin, tmax, tc);
@@ -286,7 +288,8 @@ struct Walk<true> {
       if (!any_hit8<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, column, tc)) found.word = kHitMiss;
       return found;
     }
-    return walk_binary<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, any, reinterpret_cast<int*>(column), tc);
+    return walk_binary<kPathStack, 32, true>(J, o, d, kRayTMin, tmax, any, reinterpret_cast<int*>(stack) + (threadIdx.x & 31),
+                                       tc);
   }
 };
 
@@ -304,8 +307,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
   const int lane = threadIdx.x & 31;
   unsigned char* const mine = smem + (threadIdx.x >> 5) * kWarpSmem<kMis, kGeneral>;
   WarpPaths<kMis>& S = *reinterpret_cast<WarpPaths<kMis>*>(mine);
-  // This thread's stack column: entry k at column[k * 32].
-  Entry* const column = reinterpret_cast<Entry*>(mine + sizeof(WarpPaths<kMis>)) + lane;
+  Entry* const stack = reinterpret_cast<Entry*>(mine + sizeof(WarpPaths<kMis>));  // of the warp
   if (threadIdx.x < 3) s_total[threadIdx.x] = 0;
 #pragma unroll 1
   for (int k = lane; k < kWarpPaths; k += 32) S.idle[k] = static_cast<std::uint8_t>(k);
@@ -439,7 +441,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
       const RtgSceneDev& J = wb.jobs[job];
       // One copy of the walk serves both kinds of rays.
       const bool any = step == kShadow;
-      const RayHit h = walk(J, o, d, tmax, any, column, any ? shadow_tree : closest_tree, any ? sh_tc : tc);
+      const RayHit h = walk(J, o, d, tmax, any, stack, any ? shadow_tree : closest_tree, any ? sh_tc : tc);
       const std::uint32_t meta = S.meta[p];
       if (any) {
         if (h.word == kHitMiss) add3(S.light, p, get3(S.sh_c, p));
@@ -639,7 +641,7 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
   const int lane = threadIdx.x & 31;
   unsigned char* const mine = smem + (threadIdx.x >> 5) * kDirectWarpSmem<kGeneral>;
   DirectPaths& S = *reinterpret_cast<DirectPaths*>(mine);
-  Entry* const column = reinterpret_cast<Entry*>(mine + sizeof(DirectPaths)) + lane;
+  Entry* const stack = reinterpret_cast<Entry*>(mine + sizeof(DirectPaths));  // of the warp
   // Pending branches of this warp's slot p start at row (first_slot + p) * stack_depth * kPendingRows.
   const std::size_t first_slot =
       (static_cast<std::size_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5)) * kDirectPaths;
@@ -740,7 +742,7 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
     }
     __syncwarp();
     RayHit h{tmax, kHitMiss, 0.f, 0.f};
-    if (ray) h = walk(J, o, d, tmax, step == kLight, column, tree, tc);
+    if (ray) h = walk(J, o, d, tmax, step == kLight, stack, tree, tc);
     // What the sample does next: trace S.o, S.d; sample a light; or neither, and then
     // a pending branch is next, or the sample is done.
     bool go = false, lit = false;
