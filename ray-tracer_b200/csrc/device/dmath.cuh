@@ -16,36 +16,51 @@ namespace rtg {
 
 __device__ __forceinline__ float3 f3(float a, float b, float c) { return make_float3(a, b, c); }
 __device__ __forceinline__ float3 f3(float4 v) { return make_float3(v.x, v.y, v.z); }
-__device__ __forceinline__ float3 operator+(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
-__device__ __forceinline__ float3 operator-(float3 a, float3 b) { return f3(a.x - b.x, a.y - b.y, a.z - b.z); }
+// Pinned rounding, for everything a sample's value depends on: every product and sum
+// is an explicit fmaf or an __fmul_rn / __fadd_rn / __fsub_rn, which the compiler
+// never fuses, so the bits do not depend on the kernel the code is inlined into, on
+// its register limit or on what else it computes. (Left to contract freely, the same
+// source rounded differently in different instances of a kernel.) The vector operators
+// round each operation; mad3, dot3 and dot3p say which product is fused. Where two forms
+// would do, each place keeps the one its values have always had.
+__device__ __forceinline__ float3 operator+(float3 a, float3 b) {
+  return f3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z));
+}
+__device__ __forceinline__ float3 operator-(float3 a, float3 b) {
+  return f3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z));
+}
 __device__ __forceinline__ float3 operator-(float3 a) { return f3(-a.x, -a.y, -a.z); }
-__device__ __forceinline__ float3 operator*(float3 a, float3 b) { return f3(a.x * b.x, a.y * b.y, a.z * b.z); }
-__device__ __forceinline__ float3 operator*(float3 a, float s) { return f3(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ float3 operator*(float s, float3 a) { return f3(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ float3 operator*(float3 a, float3 b) {
+  return f3(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z));
+}
+__device__ __forceinline__ float3 operator*(float3 a, float s) {
+  return f3(__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s));
+}
+__device__ __forceinline__ float3 operator*(float s, float3 a) { return a * s; }
+// a b + c, fused.
+__device__ __forceinline__ float3 mad3(float a, float3 b, float3 c) {
+  return f3(fmaf(a, b.x, c.x), fmaf(a, b.y, c.y), fmaf(a, b.z, c.z));
+}
+__device__ __forceinline__ float3 mad3(float3 a, float3 b, float3 c) {
+  return f3(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z));
+}
+__device__ __forceinline__ float dot3(float3 a, float3 b) {
+  return fmaf(a.z, b.z, fmaf(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
-  return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+  return f3(fmaf(a.y, b.z, -__fmul_rn(a.z, b.y)), fmaf(a.z, b.x, -__fmul_rn(a.x, b.z)),
+            fmaf(a.x, b.y, -__fmul_rn(a.y, b.x)));
 }
 __device__ __forceinline__ float max3(float3 a) { return fmaxf(a.x, fmaxf(a.y, a.z)); }
 __device__ __forceinline__ bool is_zero3(float3 a) { return a.x == 0.f && a.y == 0.f && a.z == 0.f; }
 
-// Pinned rounding, for the code that decides hits: the hit tests, the slab
-// set-up and the camera ray. Every product and sum is an explicit fmaf or an
-// __fmul_rn / __fadd_rn / __fsub_rn, which the compiler never fuses, so the bits
-// do not depend on the kernel the code is inlined into. (Left to contract freely,
-// the counting and non-counting instances of the closest-hit kernel rounded a few
-// hits differently.)
-__device__ __forceinline__ float3 sub3p(float3 a, float3 b) {
-  return f3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z));
-}
-__device__ __forceinline__ float3 add3p(float3 a, float3 b) {
-  return f3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z));
-}
+// dot3 with the first product unfused instead of the second.
 __device__ __forceinline__ float dot3p(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x))); }
-__device__ __forceinline__ float3 cross3p(float3 a, float3 b) {
-  return f3(fmaf(a.y, b.z, -__fmul_rn(a.z, b.y)), fmaf(a.z, b.x, -__fmul_rn(a.x, b.z)),
-            fmaf(a.x, b.y, -__fmul_rn(a.y, b.x)));
-}
+
+// The hit tests' own forms (dot3p fuses in another order than dot3).
+__device__ __forceinline__ float3 sub3p(float3 a, float3 b) { return a - b; }
+__device__ __forceinline__ float3 add3p(float3 a, float3 b) { return a + b; }
+__device__ __forceinline__ float3 cross3p(float3 a, float3 b) { return cross3(a, b); }
 
 // Normalise (pinned rounding), or return `fallback` for (near-)zero or non-finite input.
 __device__ __forceinline__ float3 unit_or(float3 v, float3 fallback) {
@@ -55,24 +70,24 @@ __device__ __forceinline__ float3 unit_or(float3 v, float3 fallback) {
   return f3(__fmul_rn(v.x, s), __fmul_rn(v.y, s), __fmul_rn(v.z, s));
 }
 
-__device__ __forceinline__ float3 reflect3(float3 v, float3 n) { return v - (2.f * dot3(v, n)) * n; }
+__device__ __forceinline__ float3 reflect3(float3 v, float3 n) { return mad3(-__fmul_rn(2.f, dot3(v, n)), n, v); }
 
 // Snell refraction of unit `v` through unit `n` (facing against v), eta = n_i / n_t.
 __device__ __forceinline__ bool refract3(float3 v, float3 n, float eta, float3& out) {
   const float cos_i = fminf(-dot3(v, n), 1.f);
-  const float sin2_t = eta * eta * (1.f - cos_i * cos_i);
+  const float sin2_t = __fmul_rn(__fmul_rn(eta, eta), fmaf(-cos_i, cos_i, 1.f));
   if (sin2_t > 1.f) return false;
-  const float cos_t = sqrtf(1.f - sin2_t);
-  out = eta * v + (eta * cos_i - cos_t) * n;
+  const float cos_t = sqrtf(__fsub_rn(1.f, sin2_t));
+  out = mad3(eta, v, fmaf(eta, cos_i, -cos_t) * n);
   return true;
 }
 
 __device__ __forceinline__ float schlick(float cos_theta, float eta) {
-  float r0 = (1.f - eta) / (1.f + eta);
-  r0 *= r0;
-  const float m = 1.f - cos_theta;
-  const float m2 = m * m;
-  return r0 + (1.f - r0) * (m2 * m2 * m);
+  float r0 = __fsub_rn(1.f, eta) / __fadd_rn(1.f, eta);
+  r0 = __fmul_rn(r0, r0);
+  const float m = __fsub_rn(1.f, cos_theta);
+  const float m2 = __fmul_rn(m, m);
+  return fmaf(__fsub_rn(1.f, r0), __fmul_rn(__fmul_rn(m2, m2), m), r0);
 }
 
 // ---------------------------------------------------------------------------
@@ -95,7 +110,7 @@ struct Pcg {
     return __funnelshift_r(x, x, r);  // rotate right by r
   }
   // Uniform in [0, 1) from the top 24 bits of one draw.
-  __device__ __forceinline__ float uniform() { return static_cast<float>(next() >> 8) * 0x1p-24f; }
+  __device__ __forceinline__ float uniform() { return __fmul_rn(static_cast<float>(next() >> 8), 0x1p-24f); }
   // Uniform integer in [0, n): floor(u32 * n / 2^32), which equals the CPU's
   // floor(double(u32) / 2^32 * n) exactly for n < 2^21.
   __device__ __forceinline__ std::uint32_t below(std::uint32_t n) {
@@ -126,33 +141,33 @@ __device__ __forceinline__ float2 unit_disk(Pcg& rng) {
 }
 
 __device__ __forceinline__ float3 unit_vector(Pcg& rng) {
-  const float z = 1.f - 2.f * rng.uniform();
-  const float r = sqrtf(fmaxf(0.f, 1.f - z * z));
+  const float z = fmaf(-2.f, rng.uniform(), 1.f);
+  const float r = sqrtf(fmaxf(0.f, fmaf(-z, z, 1.f)));
   float s, c;
   sincospif(2.f * rng.uniform(), &s, &c);
-  return f3(r * c, r * s, z);
+  return f3(__fmul_rn(r, c), __fmul_rn(r, s), z);
 }
 
 __device__ __forceinline__ float3 cosine_hemisphere(Pcg& rng) {
   const float2 d = unit_disk(rng);
-  return f3(d.x, d.y, sqrtf(fmaxf(0.f, 1.f - d.x * d.x - d.y * d.y)));
+  return f3(d.x, d.y, sqrtf(fmaxf(0.f, fmaf(-d.y, d.y, fmaf(-d.x, d.x, 1.f)))));
 }
 
 // Uniform direction in the cone 1 - cos(theta) <= one_minus_cos_max around +Z.
 // Written in terms of 1 - cos so narrow cones keep their precision in fp32.
 __device__ __forceinline__ float3 uniform_cone(Pcg& rng, float one_minus_cos_max) {
-  const float s = rng.uniform() * one_minus_cos_max;  // 1 - cos(theta)
-  const float cos_t = 1.f - s;
-  const float sin_t = sqrtf(fmaxf(0.f, s * (2.f - s)));
+  const float s = __fmul_rn(rng.uniform(), one_minus_cos_max);  // 1 - cos(theta)
+  const float cos_t = __fsub_rn(1.f, s);
+  const float sin_t = sqrtf(fmaxf(0.f, __fmul_rn(s, __fsub_rn(2.f, s))));
   float sp, cp;
   sincospif(2.f * rng.uniform(), &sp, &cp);
-  return f3(sin_t * cp, sin_t * sp, cos_t);
+  return f3(__fmul_rn(sin_t, cp), __fmul_rn(sin_t, sp), cos_t);
 }
 
 // Uniform barycentrics (b1, b2) on a triangle (square-root parameterisation).
 __device__ __forceinline__ float2 uniform_triangle(Pcg& rng) {
   const float su = sqrtf(rng.uniform());
-  return make_float2(1.f - su, rng.uniform() * su);
+  return make_float2(__fsub_rn(1.f, su), __fmul_rn(rng.uniform(), su));
 }
 
 // Orthonormal basis around unit w (Duff et al. 2017, "Building an Orthonormal
@@ -161,12 +176,13 @@ struct Frame {
   float3 u, v, w;
   __device__ __forceinline__ explicit Frame(float3 n) : w(n) {
     const float sign = copysignf(1.f, n.z);
-    const float a = -1.f / (sign + n.z);
-    const float b = n.x * n.y * a;
-    u = f3(1.f + sign * n.x * n.x * a, sign * b, -sign * n.x);
-    v = f3(b, sign + n.y * n.y * a, -n.y);
+    const float a = -1.f / __fadd_rn(sign, n.z);
+    const float b = __fmul_rn(__fmul_rn(n.x, n.y), a);
+    u = f3(fmaf(__fmul_rn(__fmul_rn(sign, n.x), n.x), a, 1.f), __fmul_rn(sign, b), __fmul_rn(-sign, n.x));
+    v = f3(b, fmaf(__fmul_rn(n.y, n.y), a, sign), -n.y);
   }
-  __device__ __forceinline__ float3 to_world(float3 a) const { return a.x * u + a.y * v + a.z * w; }
+  __device__ __forceinline__ float3 to_world(float3 a) const { return f3(fmaf(a.z, w.x, fmaf(a.y, v.x, __fmul_rn(a.x, u.x))), fmaf(a.z, w.y, fmaf(a.y, v.y, __fmul_rn(a.x, u.y))),
+              fmaf(a.z, w.z, fmaf(a.x, u.z, __fmul_rn(a.y, v.z)))); }
 };
 
 // ---------------------------------------------------------------------------
@@ -178,25 +194,26 @@ struct Frame {
 // (include/raytracer/math/ray.hpp:41-58), which is below an fp32 ulp at the
 // 555-unit scale of a Cornell room.
 __device__ __forceinline__ float ulp_step(float p, float n, float scaled_n) {
-  const int step = static_cast<int>(256.f * n);
+  const int step = static_cast<int>(__fmul_rn(256.f, n));
   const float moved = __int_as_float(__float_as_int(p) + (p < 0.f ? -step : step));
-  return fabsf(p) < (1.f / 32.f) ? p + scaled_n : moved;
+  return fabsf(p) < (1.f / 32.f) ? __fadd_rn(p, scaled_n) : moved;
 }
 __device__ __forceinline__ float3 spawn_point(float3 p, float3 n) {
   constexpr float kNearScale = 1.f / 65536.f;
-  return f3(ulp_step(p.x, n.x, kNearScale * n.x), ulp_step(p.y, n.y, kNearScale * n.y),
-            ulp_step(p.z, n.z, kNearScale * n.z));
+  const float3 near = kNearScale * n;  // exact: a power of two
+  return f3(ulp_step(p.x, n.x, near.x), ulp_step(p.y, n.y, near.y), ulp_step(p.z, n.z, near.z));
 }
 // Spawn for direction `dir` from a surface with geometric normal `gn`.
 __device__ __forceinline__ float3 spawn_towards(float3 p, float3 gn, float3 dir) {
   return spawn_point(p, dot3(dir, gn) > 0.f ? gn : -gn);
 }
 
-// The reference's shadow-ray shortening distance, 4 * 1.6e-6 * max(1, |p|inf)
-// (src/rendering/integrator.cpp:69-70), which is ~100 fp32 ulps of |p|.
-__device__ __forceinline__ float shadow_margin(float3 p) {
+// The reference's shadow-ray shortening distance is 4 * 1.6e-6 * max(1, |p|inf)
+// (src/rendering/integrator.cpp:69-70), ~100 fp32 ulps of |p|: kShadowMargin times this.
+constexpr float kShadowMargin = 4.f * 1.6e-6f;
+__device__ __forceinline__ float shadow_scale(float3 p) {
   const float m = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), 1.f));
-  return 4.f * 1.6e-6f * m;
+  return m;
 }
 
 }  // namespace rtg

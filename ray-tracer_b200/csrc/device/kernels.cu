@@ -247,11 +247,14 @@ __device__ __forceinline__ void set3(float (&v)[3][kSlots], int p, float3 x) {
   v[1][p] = x.y;
   v[2][p] = x.z;
 }
+// v[.][p] += x, and += a b, fused.
 template <int kSlots>
-__device__ __forceinline__ void add3(float (&v)[3][kSlots], int p, float3 x) {
-  v[0][p] += x.x;
-  v[1][p] += x.y;
-  v[2][p] += x.z;
+__device__ __forceinline__ void add_to(float (&v)[3][kSlots], int p, float3 x) {
+  set3(v, p, get3(v, p) + x);
+}
+template <int kSlots, class A>
+__device__ __forceinline__ void mad_to(float (&v)[3][kSlots], int p, A a, float3 b) {
+  set3(v, p, mad3(a, b, get3(v, p)));
 }
 
 // The walk of an instance. The common instance walks the binary tree; the general
@@ -444,17 +447,17 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
       const RayHit h = walk(J, o, d, tmax, any, stack, any ? shadow_tree : closest_tree, any ? sh_tc : tc);
       const std::uint32_t meta = S.meta[p];
       if (any) {
-        if (h.word == kHitMiss) add3(S.light, p, get3(S.sh_c, p));
+        if (h.word == kHitMiss) add_to(S.light, p, get3(S.sh_c, p));
         cont = (meta & kPathContinues) != 0;
       } else if (h.word == kHitMiss) {
         // The normals view shows misses black.
-        if (J.integrator != 2) add3(S.light, p, get3(S.beta, p) * background(J, d));
+        if (J.integrator != 2) mad_to(S.light, p, get3(S.beta, p), background(J, d));
       } else {
         const Surface s = make_surface(J, o, d, h);
         if (J.integrator == 2) {
           // Normals view: outward shading normal mapped to [0, 1].
           const float3 nn = s.front ? s.n : -s.n;
-          set3(S.light, p, f3(0.5f * (nn.x + 1.f), 0.5f * (nn.y + 1.f), 0.5f * (nn.z + 1.f)));
+          set3(S.light, p, (nn + f3(1.f, 1.f, 1.f)) * 0.5f);
         } else {
           const DevMaterial m = J.materials[s.material];
           const float3 le = emitted(m, s.front);
@@ -467,7 +470,11 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
                       ? power_heuristic(S.pdf[kMis ? p : 0],
                                         light_pdf_of_hit(J, o, d, h, s) / static_cast<float>(J.n_lights))
                       : 0.f;
-            if (w > 0.f) add3(S.light, p, get3(S.beta, p) * le * w);
+            if (kMis && J.light_sampling == 2) {
+              if (w > 0.f) mad_to(S.light, p, w, get3(S.beta, p) * le);
+            } else if (w > 0.f) {
+              mad_to(S.light, p, get3(S.beta, p), le);
+            }
           }
           Pcg rng{ld_u64(S.rng[0][p], S.rng[1][p]), ld_u64(S.rng[2][p], S.rng[3][p])};
           Scatter sr;
@@ -488,10 +495,10 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
                   const ShadowRay sray = shadow_ray(s, ls);
                   float w = 1.f;  // a point light (pdf 0) cannot be hit by BSDF sampling
                   if (kMis && J.light_sampling == 2 && ls.pdf > 0.f)
-                    w = power_heuristic(ls.pdf / static_cast<float>(nl), dot3(s.n, ls.wi) * kInvPiF);
+                    w = power_heuristic(ls.pdf / static_cast<float>(nl), __fmul_rn(dot3(s.n, ls.wi), kInvPiF));
                   set3(S.sh_d, p, sray.d);
                   S.sh_tmax[p] = sray.tmax;
-                  set3(S.sh_c, p, get3(S.beta, p) * (f * ls.li_over_pdf) * (static_cast<float>(nl) * w));
+                  set3(S.sh_c, p, get3(S.beta, p) * (f * ls.li_over_pdf) * __fmul_rn(static_cast<float>(nl), w));
                   shadow = true;
                 }
               }
@@ -514,7 +521,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
               S.rng[0][p] = static_cast<std::uint32_t>(rng.state);
               S.rng[1][p] = static_cast<std::uint32_t>(rng.state >> 32);
               // Cosine-hemisphere pdf of this bounce, for the MIS weight at the next hit.
-              if (kMis && J.light_sampling == 2 && !sr.specular) S.pdf[kMis ? p : 0] = dot3(s.n, sr.dir) * kInvPiF;
+              if (kMis && J.light_sampling == 2 && !sr.specular) S.pdf[kMis ? p : 0] = __fmul_rn(dot3p(s.n, sr.dir), kInvPiF);
             }
             S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u);
           }
@@ -747,22 +754,19 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
     // a pending branch is next, or the sample is done.
     bool go = false, lit = false;
     if (on && step == kLight) {
-      if (ray && h.word == kHitMiss) {
-        const float3 sum = get3(S.sum, p) + get3(S.f, p) * get3(S.li, p);
-        set3(S.sum, p, sum);
-      }
+      if (ray && h.word == kHitMiss) mad_to(S.sum, p, get3(S.f, p), get3(S.li, p));
       const int next = S.light_index[p] + 1;
       S.light_index[p] = next;
       lit = next < J.n_lights;
-      if (!lit) set3(S.light, p, get3(S.light, p) + get3(S.w, p) * get3(S.sum, p));
+      if (!lit) mad_to(S.light, p, get3(S.w, p), get3(S.sum, p));
     } else if (on) {
       const float3 w = get3(S.w, p);
       if (h.word == kHitMiss) {
-        set3(S.light, p, get3(S.light, p) + w * background(J, d));
+        mad_to(S.light, p, w, background(J, d));
       } else {
         const Surface s = make_surface(J, o, d, h);
         const DevMaterial m = J.materials[s.material];
-        set3(S.light, p, get3(S.light, p) + w * emitted(m, s.front));
+        mad_to(S.light, p, w, emitted(m, s.front));
         const int depth = S.depth[p];
         if (depth < J.max_depth) {
           const std::uint32_t kind = kind_of(m);
@@ -800,7 +804,7 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
               const int sp = S.pending[p];
               if (sp < stack_depth) {
                 const float3 td = unit_or(refr, f3(0.f, 0.f, 0.f));
-                const float3 to = spawn_towards(s.p, s.gn, td), tw = w * tint * (1.f - F);
+                const float3 to = spawn_towards(s.p, s.gn, td), tw = w * tint * __fsub_rn(1.f, F);
                 float4* const row = stack_rows + ((first_slot + p) * stack_depth + sp) * kPendingRows;
                 row[0] = make_float4(to.x, to.y, to.z, td.x);
                 row[1] = make_float4(td.y, td.z, tw.x, tw.y);

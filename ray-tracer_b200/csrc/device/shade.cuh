@@ -31,12 +31,12 @@ struct Surface {
 // surface-accurate point).
 __device__ __forceinline__ Surface make_surface(const RtgSceneDev& sc, float3 o, float3 d, const RayHit& h) {
   Surface s;
-  s.p = o + h.t * d;
+  s.p = mad3(h.t, d, o);
   s.is_plane = (h.word & kHitPlaneBit) != 0 && h.word != kHitMiss;
   if (s.is_plane) {
     const DevPlane pl = sc.planes[h.word & ~kHitPlaneBit];
     const float3 nrm = f3(pl.normal);
-    s.p = s.p - dot3(s.p - f3(pl.point), nrm) * nrm;
+    s.p = mad3(-dot3(s.p - f3(pl.point), nrm), nrm, s.p);
     s.front = dot3(d, nrm) < 0.f;
     s.gn = s.front ? nrm : -nrm;
     s.n = s.gn;
@@ -51,13 +51,13 @@ __device__ __forceinline__ Surface make_surface(const RtgSceneDev& sc, float3 o,
   s.material = mword & 0x7FFFFFFFu;
   if (__float_as_uint(p0.w) & kSphereBit) {
     const float3 outward = unit_or((s.p - f3(p0)) * (1.f / p1.x), f3(0.f, 1.f, 0.f));
-    s.p = f3(p0) + p1.x * outward;
+    s.p = mad3(p1.x, outward, f3(p0));
     s.front = dot3(d, outward) < 0.f;
     s.gn = s.front ? outward : -outward;
     s.n = s.gn;
     return s;
   }
-  s.p = f3(p0) + h.b1 * f3(p1) + h.b2 * f3(p2);
+  s.p = mad3(h.b2, f3(p2), mad3(h.b1, f3(p1), f3(p0)));
   const float3 ng = unit_or(cross3(f3(p1), f3(p2)), f3(0.f, 0.f, 0.f));
   s.front = dot3(d, ng) < 0.f;
   s.gn = s.front ? ng : -ng;
@@ -66,8 +66,8 @@ __device__ __forceinline__ Surface make_surface(const RtgSceneDev& sc, float3 o,
     const float4 n0 = __ldg(&sc.slot_normals[3 * slot]);
     const float4 n1 = __ldg(&sc.slot_normals[3 * slot + 1]);
     const float4 n2 = __ldg(&sc.slot_normals[3 * slot + 2]);
-    const float w0 = 1.f - h.b1 - h.b2;
-    const float3 ns = unit_or(w0 * f3(n0) + h.b1 * f3(n1) + h.b2 * f3(n2), ng);
+    const float w0 = __fsub_rn(__fsub_rn(1.f, h.b1), h.b2);
+    const float3 ns = unit_or(mad3(h.b2, f3(n2), mad3(w0, f3(n0), h.b1 * f3(n1))), ng);
     s.n = s.front ? ns : -ns;
     // Keep the shading normal in the geometric normal's hemisphere.
     if (dot3(s.n, s.gn) <= 0.f) s.n = s.gn;
@@ -77,16 +77,16 @@ __device__ __forceinline__ Surface make_surface(const RtgSceneDev& sc, float3 o,
 
 __device__ __forceinline__ float3 background(const RtgSceneDev& sc, float3 d) {
   if (sc.bg_solid) return sc.bg_top * sc.bg_intensity;
-  const float t = 0.5f * (unit_or(d, f3(0.f, 0.f, 0.f)).y + 1.f);
-  return (sc.bg_bottom * (1.f - t) + sc.bg_top * t) * sc.bg_intensity;
+  const float t = __fmul_rn(0.5f, __fadd_rn(unit_or(d, f3(0.f, 0.f, 0.f)).y, 1.f));
+  return mad3(__fsub_rn(1.f, t), sc.bg_bottom, sc.bg_top * t) * sc.bg_intensity;
 }
 
 __device__ __forceinline__ float3 albedo_at(const DevMaterial& m, float3 p) {
   const float scale = m.head.y;
   if (scale <= 0.f) return f3(m.colour_a);
   // The 1e-4 offset keeps surfaces lying on a cell boundary from flickering.
-  const int parity = static_cast<int>(floorf(p.x * scale + 1e-4f)) + static_cast<int>(floorf(p.y * scale + 1e-4f)) +
-                     static_cast<int>(floorf(p.z * scale + 1e-4f));
+  const int parity = static_cast<int>(floorf(fmaf(p.x, scale, 1e-4f))) + static_cast<int>(floorf(fmaf(p.y, scale, 1e-4f))) +
+                     static_cast<int>(floorf(fmaf(p.z, scale, 1e-4f)));
   return (parity & 1) ? f3(m.colour_b) : f3(m.colour_a);
 }
 
@@ -118,7 +118,7 @@ __device__ __forceinline__ bool scatter(const DevMaterial& m, float3 d, const Su
     const float rough = m.head.z;
     if (rough > 0.f) {
       const float3 fuzz = unit_vector(rng);
-      r = unit_or(unit_or(r, f3(0.f, 0.f, 0.f)) + rough * fuzz, f3(0.f, 0.f, 0.f));
+      r = unit_or(mad3(rough, fuzz, unit_or(r, f3(0.f, 0.f, 0.f))), f3(0.f, 0.f, 0.f));
     }
     if (dot3(r, s.gn) <= 0.f) return false;
     out.dir = r;
@@ -148,7 +148,7 @@ __device__ __forceinline__ float3 brdf_cos(const DevMaterial& m, const Surface& 
   if (kind_of(m) != kLambertian) return f3(0.f, 0.f, 0.f);
   const float c = dot3(s.n, wi);
   if (c <= 0.f || dot3(s.gn, wi) <= 0.f) return f3(0.f, 0.f, 0.f);
-  return albedo_at(m, s.p) * (c * kInvPiF);
+  return albedo_at(m, s.p) * __fmul_rn(c, kInvPiF);
 }
 
 // brdf_cos for a Lambertian surface of albedo `albedo` (the only non-specular
@@ -156,7 +156,7 @@ __device__ __forceinline__ float3 brdf_cos(const DevMaterial& m, const Surface& 
 __device__ __forceinline__ float3 lambert_cos(float3 albedo, const Surface& s, float3 wi) {
   const float c = dot3(s.n, wi);
   if (c <= 0.f || dot3(s.gn, wi) <= 0.f) return f3(0.f, 0.f, 0.f);
-  return albedo * (c * kInvPiF);
+  return albedo * __fmul_rn(c, kInvPiF);
 }
 
 struct LightSample {
@@ -179,11 +179,11 @@ struct ShadowRay {
 __device__ __forceinline__ ShadowRay shadow_ray(const Surface& s, const LightSample& ls) {
   ShadowRay r;
   r.o = spawn_towards(s.p, s.gn, ls.wi);
-  const float3 target = s.p + ls.dist * ls.wi;
+  const float3 target = mad3(ls.dist, ls.wi, s.p);
   const float3 span = target - r.o;
   const float len = sqrtf(dot3(span, span));
   r.d = len > 0.f ? span * (1.f / len) : ls.wi;
-  r.tmax = fmaxf(len - shadow_margin(target), 0.f);
+  r.tmax = fmaxf(fmaf(-kShadowMargin, shadow_scale(target), len), 0.f);
   return r;
 }
 
@@ -218,28 +218,28 @@ __device__ __forceinline__ LightSample sample_light(const DevLight* __restrict__
       // Inside the sphere: area-sample its surface (only two-sided emitters light their inside).
       if (!two_sided) return out;
       const float3 nl = unit_vector(rng);
-      const float3 dv = c + r * nl - p;
-      const float dd2 = dot3(dv, dv);
+      const float3 dv = mad3(r, nl, c) - p;
+      const float dd2 = dot3p(dv, dv);
       if (dd2 < 1e-16f) return out;
       out.dist = sqrtf(dd2);
       out.wi = dv * (1.f / out.dist);
       const float cos_l = fabsf(dot3(nl, out.wi));
       if (cos_l < 1e-9f) return out;
-      out.li_over_pdf = emit * (cos_l * area / dd2);
-      out.pdf = dd2 / (cos_l * area);
+      out.li_over_pdf = emit * (__fmul_rn(cos_l, area) / dd2);
+      out.pdf = dd2 / __fmul_rn(cos_l, area);
       out.valid = true;
       return out;
     }
     // Cone of directions subtended by the sphere; 1 - cos written without cancellation.
     const float x = r2 / d2;
-    const float one_minus_cos = x / (1.f + sqrtf(1.f - x));
+    const float one_minus_cos = x / __fadd_rn(1.f, sqrtf(__fsub_rn(1.f, x)));
     const float3 axis = oc * rsqrtf(d2);
     out.wi = Frame(axis).to_world(uniform_cone(rng, one_minus_cos));
     float t;
     if (!sphere_test(p, out.wi, c, f3(0.f, 0.f, 0.f), r, 0.f, __int_as_float(0x7f800000), t)) return out;  // grazing miss
     out.dist = t;
-    out.li_over_pdf = emit * (2.f * kPiF * one_minus_cos);
-    out.pdf = 1.f / (2.f * kPiF * one_minus_cos);
+    out.li_over_pdf = emit * __fmul_rn(2.f * kPiF, one_minus_cos);
+    out.pdf = 1.f / __fmul_rn(2.f * kPiF, one_minus_cos);
     out.valid = true;
     return out;
   }
@@ -249,7 +249,7 @@ __device__ __forceinline__ LightSample sample_light(const DevLight* __restrict__
   const float area = q1.w;
   const bool two_sided = q2.w != 0.f;
   const float2 b = uniform_triangle(rng);
-  const float3 q = (1.f - b.x - b.y) * v0 + b.x * v1 + b.y * v2;
+  const float3 q = mad3(b.y, v2, mad3(b.x, v1, __fsub_rn(__fsub_rn(1.f, b.x), b.y) * v0));
   const float3 dv = q - p;
   const float d2 = dot3(dv, dv);
   if (d2 < 1e-16f) return out;
@@ -259,8 +259,8 @@ __device__ __forceinline__ LightSample sample_light(const DevLight* __restrict__
   if (cos_signed <= 0.f && !two_sided) return out;
   const float cos_l = fabsf(cos_signed);
   if (cos_l < 1e-9f) return out;
-  out.li_over_pdf = f3(__ldg(&Lp->q4)) * (cos_l * area / d2);
-  out.pdf = d2 / (cos_l * area);
+  out.li_over_pdf = f3(__ldg(&Lp->q4)) * (__fmul_rn(cos_l, area) / d2);
+  out.pdf = d2 / __fmul_rn(cos_l, area);
   out.valid = true;
   return out;
 }
@@ -279,20 +279,21 @@ __device__ __forceinline__ float light_pdf_of_hit(const RtgSceneDev& sc, float3 
     const float r2 = p1.y;  // radius squared (p1.x holds the radius)
     const float3 oc = f3(p0) - o;
     const float d2 = dot3(oc, oc);
-    if (d2 <= r2) return cos_l > 0.f ? h.t * h.t / (cos_l * 4.f * kPiF * r2) : 0.f;
+    if (d2 <= r2)
+      return cos_l > 0.f ? __fmul_rn(h.t, h.t) / __fmul_rn(__fmul_rn(__fmul_rn(cos_l, 4.f), kPiF), r2) : 0.f;
     const float x = r2 / d2;
-    return 1.f / (2.f * kPiF * (x / (1.f + sqrtf(1.f - x))));
+    return 1.f / __fmul_rn(2.f * kPiF, x / __fadd_rn(1.f, sqrtf(__fsub_rn(1.f, x))));
   }
   const float4 p2 = __ldg(&sc.prims[3 * slot + 2]);
   const float3 c = cross3(f3(p1), f3(p2));
-  const float area = 0.5f * sqrtf(dot3(c, c));
-  return cos_l > 0.f && area > 0.f ? h.t * h.t / (cos_l * area) : 0.f;
+  const float area = __fmul_rn(0.5f, sqrtf(dot3(c, c)));
+  return cos_l > 0.f && area > 0.f ? __fmul_rn(h.t, h.t) / __fmul_rn(cos_l, area) : 0.f;
 }
 
 // Power heuristic (Veach, beta = 2) of the strategy with pdf a against one with pdf b.
 __device__ __forceinline__ float power_heuristic(float a, float b) {
-  const float a2 = a * a, b2 = b * b;
-  return a2 + b2 > 0.f ? a2 / (a2 + b2) : 0.f;
+  const float a2 = __fmul_rn(a, a), sum = fmaf(b, b, a2);
+  return sum > 0.f ? a2 / sum : 0.f;
 }
 
 }  // namespace rtg
