@@ -899,40 +899,72 @@ __device__ __forceinline__ std::uint8_t srgb8(double v) {
   return static_cast<std::uint8_t>(llround(s * 255.0));
 }
 
-__global__ void k_resolve(const double* __restrict__ fb_sum, const std::uint32_t* __restrict__ fb_count,
-                          std::uint64_t pixels, int op, double exposure, std::uint8_t* rgb8, double* mean_out) {
-  const std::uint64_t p = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (p >= pixels) return;
-  const std::uint32_t n = fb_count[p];
-  double c[3] = {0, 0, 0};
-  if (n) {
-    const double inv = 1.0 / static_cast<double>(n);
-    for (int k = 0; k < 3; ++k) c[k] = fb_sum[4 * p + k] * inv;
+// Means (mean_out) and/or their tone-mapped bytes (rgb8) of `pixels` pixels. A block's
+// output is collected in shared memory and leaves in 16-byte (means) or 4-byte (image)
+// pieces in order: the destination may be pinned host memory, where a pixel's own 8-
+// and 1-byte stores would each cross the bus alone.
+constexpr int kResolveBlock = 256;
+__global__ void __launch_bounds__(kResolveBlock)
+k_resolve(const double* __restrict__ fb_sum, const std::uint32_t* __restrict__ fb_count, std::uint64_t pixels, int op,
+          double exposure, std::uint8_t* rgb8, double* mean_out) {
+  __shared__ __align__(16) double s_mean[3 * kResolveBlock];
+  __shared__ __align__(16) std::uint8_t s_rgb[3 * kResolveBlock];
+  const std::uint64_t first = static_cast<std::uint64_t>(blockIdx.x) * kResolveBlock;
+  const std::uint64_t p = first + threadIdx.x;
+  const int here = static_cast<int>(pixels - first < kResolveBlock ? pixels - first : kResolveBlock);
+  if (p < pixels) {
+    const std::uint32_t n = fb_count[p];
+    double c[3] = {0, 0, 0};
+    if (n) {
+      const double inv = 1.0 / static_cast<double>(n);
+      for (int k = 0; k < 3; ++k) c[k] = fb_sum[4 * p + k] * inv;
+    }
+    if (mean_out)
+      for (int k = 0; k < 3; ++k) s_mean[3 * threadIdx.x + k] = c[k];
+    if (rgb8) {
+      double t[3];
+      bool finite = true;
+      for (int k = 0; k < 3; ++k) {
+        t[k] = c[k] * exposure;
+        finite = finite && isfinite(t[k]);
+      }
+      for (int k = 0; k < 3; ++k) {
+        double v = finite ? t[k] : 0.0;
+        if (op == 0) v = v < 0 ? 0 : (v > 1 ? 1 : v);
+        else if (op == 1) v = v / (1 + v);
+        else v = aces_curve(v);
+        s_rgb[3 * threadIdx.x + k] = srgb8(v);
+      }
+    }
   }
-  if (mean_out)
-    for (int k = 0; k < 3; ++k) mean_out[3 * p + k] = c[k];
-  if (!rgb8) return;
-  double t[3];
-  bool finite = true;
-  for (int k = 0; k < 3; ++k) {
-    t[k] = c[k] * exposure;
-    finite = finite && isfinite(t[k]);
+  __syncthreads();
+  // Both outputs start 16-byte aligned and every block's part is a multiple of 16 bytes,
+  // but for the last block's.
+  if (mean_out) {
+    double* const to = mean_out + 3 * first;
+    const int n2 = 3 * here / 2;
+    for (int k = threadIdx.x; k < n2; k += kResolveBlock)
+      reinterpret_cast<double2*>(to)[k] = reinterpret_cast<const double2*>(s_mean)[k];
+    if ((3 * here & 1) && threadIdx.x == 0) to[3 * here - 1] = s_mean[3 * here - 1];
   }
-  for (int k = 0; k < 3; ++k) {
-    double v = finite ? t[k] : 0.0;
-    if (op == 0) v = v < 0 ? 0 : (v > 1 ? 1 : v);
-    else if (op == 1) v = v / (1 + v);
-    else v = aces_curve(v);
-    rgb8[3 * p + k] = srgb8(v);
+  if (rgb8) {
+    std::uint8_t* const to = rgb8 + 3 * first;
+    const int n4 = 3 * here / 4;
+    for (int k = threadIdx.x; k < n4; k += kResolveBlock)
+      reinterpret_cast<std::uint32_t*>(to)[k] = reinterpret_cast<const std::uint32_t*>(s_rgb)[k];
+    for (int k = 4 * n4 + threadIdx.x; k < 3 * here; k += kResolveBlock) to[k] = s_rgb[k];
   }
 }
 
 // ---------------------------------------------------------------------------
 // `tree` picks the walk: 8 the eight-wide tree; otherwise the binary tree
 // (closest hit) or the four-wide tree (any hit).
+// Results leave in the form the caller gets (t 0 and id -1 on a miss; the plane's
+// index where `plane` is 1). Rays and results may be pinned host memory: each is read
+// or written once, in order.
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock) k_ray_closest(const RtgSceneDev* __restrict__ job, const float4* __restrict__ rays,
-                                                        std::uint32_t n, float4* out, int brute, int tree) {
+                                                        std::uint32_t n, RayResults out, int brute, int tree) {
   __shared__ uint2 stack[kStackSmem * kBlock];
   const std::uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -943,12 +975,18 @@ __global__ void __launch_bounds__(kBlock) k_ray_closest(const RtgSceneDev* __res
   else if (tree == 8) h = closest_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack + threadIdx.x, tc);
   else h = closest_hit<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack) + threadIdx.x, tc);
   refine_hit(*job, f3(a), f3(b), h);
-  out[i] = make_float4(h.t, __uint_as_float(h.word), h.b1, h.b2);
+  const bool miss = h.word == kHitMiss, plane = !miss && (h.word & kHitPlaneBit);
+  out.t[i] = miss ? 0.f : h.t;
+  out.prim[i] = miss ? -1
+                     : static_cast<std::int32_t>(plane ? h.word & ~kHitPlaneBit
+                                                       : __float_as_uint(job->prims[3 * h.word].w) & kIdMask);
+  out.plane[i] = plane ? 1 : 0;
+  out.bary[i] = make_float2(h.b1, h.b2);
 }
 
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock) k_ray_any(const RtgSceneDev* __restrict__ job, const float4* __restrict__ rays,
-                                                    std::uint32_t n, std::uint32_t* out, int brute, int tree) {
+                                                    std::uint32_t n, std::uint8_t* out, int brute, int tree) {
   __shared__ uint2 stack[kStackSmem * kBlock];
   const std::uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -958,7 +996,7 @@ __global__ void __launch_bounds__(kBlock) k_ray_any(const RtgSceneDev* __restric
   if (brute) hit = any_brute(*job, f3(a), f3(b), a.w, b.w);
   else if (tree == 8) hit = any_hit8<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, stack + threadIdx.x, tc);
   else hit = any_hit4<kStackSmem, kBlock, false>(*job, f3(a), f3(b), a.w, b.w, reinterpret_cast<int*>(stack) + threadIdx.x, tc);
-  out[i] = hit ? 1u : 0u;
+  out[i] = hit ? 1 : 0;
 }
 
 // Launch with programmatic stream serialization (when enabled) so the kernel's
@@ -1076,19 +1114,19 @@ cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, flo
 cudaError_t launch_resolve(const double* fb_sum, const std::uint32_t* fb_count, std::uint64_t pixels, int tone_map,
                            double exposure, std::uint8_t* rgb8, double* mean_out, cudaStream_t stream) {
   if (pixels == 0) return cudaSuccess;
-  const unsigned blocks = static_cast<unsigned>((pixels + 255) / 256);
-  k_resolve<<<blocks, 256, 0, stream>>>(fb_sum, fb_count, pixels, tone_map, exposure, rgb8, mean_out);
+  const unsigned blocks = static_cast<unsigned>((pixels + kResolveBlock - 1) / kResolveBlock);
+  k_resolve<<<blocks, kResolveBlock, 0, stream>>>(fb_sum, fb_count, pixels, tone_map, exposure, rgb8, mean_out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ray_closest(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, float4* out, int brute,
-                               int tree, cudaStream_t stream) {
+cudaError_t launch_ray_closest(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, const RayResults& out,
+                               int brute, int tree, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   k_ray_closest<128><<<(n + 127) / 128, 128, 0, stream>>>(job_dev, rays, n, out, brute, tree);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ray_any(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, std::uint32_t* out, int brute,
+cudaError_t launch_ray_any(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, std::uint8_t* out, int brute,
                            int tree, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   k_ray_any<128><<<(n + 127) / 128, 128, 0, stream>>>(job_dev, rays, n, out, brute, tree);

@@ -67,17 +67,24 @@ cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, flo
                           float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream);
 
 // Framebuffer means (mean_out, 3 doubles per pixel) and/or their tone-mapped
-// sRGB encoding (rgb8, 3 bytes per pixel); either output may be null.
+// sRGB encoding (rgb8, 3 bytes per pixel), each 16-byte aligned, in device or pinned
+// host memory; either output may be null.
 cudaError_t launch_resolve(const double* fb_sum, const std::uint32_t* fb_count, std::uint64_t pixels, int tone_map,
                            double exposure, std::uint8_t* rgb8, double* mean_out, cudaStream_t stream);
 
 // Ray queries for parity tests and the ray API. rays: 2 float4 per ray
-// (origin, tmin), (direction, tmax). closest -> float4 (t, word, b1, b2) per ray.
+// (origin, tmin), (direction, tmax). Rays and results may be in pinned host memory.
 // tree: 8 walks the eight-wide tree; otherwise the binary tree (closest hit) or
 // the four-wide tree (any hit).
-cudaError_t launch_ray_closest(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, float4* out,
+struct RayResults {
+  float* t;
+  std::int32_t* prim;
+  std::int32_t* plane;
+  float2* bary;
+};
+cudaError_t launch_ray_closest(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, const RayResults& out,
                                int brute, int tree, cudaStream_t stream);
-cudaError_t launch_ray_any(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, std::uint32_t* out,
+cudaError_t launch_ray_any(const RtgSceneDev* job_dev, const float4* rays, std::uint32_t n, std::uint8_t* out,
                            int brute, int tree, cudaStream_t stream);
 
 }  // namespace rtg

@@ -186,7 +186,10 @@ Engine::~Engine() {
     cudaEventDestroy(upload_ev_[b]);
     if (upload_host_[b]) cudaFreeHost(upload_host_[b]);
   }
-  if (readback_host_) cudaFreeHost(readback_host_);
+  for (Slot& sl : slots_) {
+    if (sl.done) cudaEventDestroy(sl.done);
+    if (sl.mem) cudaFreeHost(sl.mem);
+  }
   cudaStreamSynchronize(build_stream_);
   cudaStreamDestroy(build_stream_);
   cudaStreamDestroy(stream_);
@@ -209,6 +212,7 @@ void Engine::reset_wave() {
     wave_.reset();
   }
   segs_.clear();
+  counters_final_ = false;
 }
 
 int Engine::add_scene(std::shared_ptr<const CompiledScene> scene) {
@@ -712,21 +716,22 @@ GpuFrame Engine::make_frame(int w, int h) {
   f.width = w;
   f.height = h;
   const std::size_t px = std::size_t(w) * std::size_t(h);
-  f.sum = dev_alloc_async<double>(px * 4, pool_, stream_);
-  f.sumsq = dev_alloc_async<double>(px * 4, pool_, stream_);
-  f.count = dev_alloc_async<std::uint32_t>(px, pool_, stream_);
-  f.stats = dev_alloc_async<std::uint64_t>(4, pool_, stream_);
-  CK(cudaMemsetAsync(f.sum, 0, px * 4 * sizeof(double), stream_));
-  CK(cudaMemsetAsync(f.sumsq, 0, px * 4 * sizeof(double), stream_));
-  CK(cudaMemsetAsync(f.count, 0, px * sizeof(std::uint32_t), stream_));
-  CK(cudaMemsetAsync(f.stats, 0, 4 * sizeof(std::uint64_t), stream_));
+  // sum, sumsq (4 doubles a pixel each), count, stats: one allocation, one memset.
+  const std::size_t plane = px * 4 * sizeof(double);
+  const std::size_t count = (px * sizeof(std::uint32_t) + 15) & ~std::size_t(15);
+  const std::size_t bytes = 2 * plane + count + 4 * sizeof(std::uint64_t);
+  unsigned char* m = dev_alloc_async<unsigned char>(bytes, pool_, stream_);
+  f.block = m;
+  f.sum = reinterpret_cast<double*>(m);
+  f.sumsq = reinterpret_cast<double*>(m + plane);
+  f.count = reinterpret_cast<std::uint32_t*>(m + 2 * plane);
+  f.stats = reinterpret_cast<std::uint64_t*>(m + 2 * plane + count);
+  CK(cudaMemsetAsync(m, 0, bytes, stream_));
   return f;
 }
 
 void Engine::free_frame(GpuFrame& f) {
-  for (void* p : {static_cast<void*>(f.sum), static_cast<void*>(f.sumsq), static_cast<void*>(f.count),
-                  static_cast<void*>(f.stats)})
-    if (p) cudaFreeAsync(p, stream_);
+  if (f.block) cudaFreeAsync(f.block, stream_);
   f = GpuFrame{};
 }
 
@@ -912,6 +917,7 @@ bool Engine::issue_pass(Job& j) {
 
 bool Engine::run_direct_pass(Job& j) {
   Wave& W = *wave_;
+  counters_final_ = false;
   const std::uint32_t k = next_pass_size(j);
   const std::uint64_t count = j.pixels * k;
   int pending_depth = 0;
@@ -1099,6 +1105,7 @@ void Engine::process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events
 
 void Engine::launch_one_iteration() {
   Wave& W = *wave_;
+  counters_final_ = false;
   if (gen_dirty_) write_gen_table();
   const int par = static_cast<int>(W.it & 1);
   const int r = static_cast<int>(W.it % kRing);
@@ -1175,15 +1182,18 @@ void Engine::abort_all() {
 void Engine::begin_stats() {
   stats_ = RenderStats{};
   CK(cudaStreamSynchronize(stream_));
-  CK(cudaMemcpy(&base_counters_, wave_->wb.cnt, sizeof(base_counters_), cudaMemcpyDeviceToHost));
-  last_counters_ = base_counters_;
+  if (!counters_final_) CK(cudaMemcpy(&last_counters_, wave_->wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+  base_counters_ = last_counters_;
   CK(cudaEventRecord(ev_begin_, stream_));
 }
 
-void Engine::end_stats() {
+void Engine::end_stats(bool cancelled) {
   finish_timing();
-  WaveCounters end{};
-  CK(cudaMemcpy(&end, wave_->wb.cnt, sizeof(end), cudaMemcpyDeviceToHost));
+  // Every path had ended when the last snapshot was taken, so its counters are final;
+  // only a cancelled render leaves paths behind it.
+  if (cancelled) CK(cudaMemcpy(&last_counters_, wave_->wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+  counters_final_ = true;
+  const WaveCounters& end = last_counters_;
   if (end.error) throw CudaFailure("device error flag " + std::to_string(end.error));
   const WaveCounters& b = base_counters_;
   stats_.rays = end.rays - b.rays;
@@ -1252,6 +1262,10 @@ std::vector<RenderProgress> Engine::render_batch(const std::vector<BatchJob>& ba
       if (j.on_pass) j.on_pass(j.prog);
     }
   rendering_.clear();
+  // The frames' invalid-sample counts cross while the last passes are folded.
+  std::uint64_t* const inv = reinterpret_cast<std::uint64_t*>(slot(0).mem);
+  for (std::size_t k = 0; k < handles.size(); ++k)
+    CK(cudaMemcpyAsync(inv + k, jobs_.at(handles[k]).frame.stats, sizeof(*inv), cudaMemcpyDeviceToHost, stream_));
   for (int h : handles) {
     Job& j = jobs_.at(h);
     out.push_back(j.prog);
@@ -1261,12 +1275,8 @@ std::vector<RenderProgress> Engine::render_batch(const std::vector<BatchJob>& ba
     close_job(j);
     jobs_.erase(h);
   }
-  end_stats();
-  for (const GpuFrame& f : frames_) {
-    std::uint64_t inv = 0;
-    CK(cudaMemcpy(&inv, f.stats, sizeof(inv), cudaMemcpyDeviceToHost));
-    invalid += inv;
-  }
+  end_stats(cancelled);
+  for (std::size_t k = 0; k < handles.size(); ++k) invalid += inv[k];
   stats_.camera_samples = samples;
   stats_.invalid_samples = invalid;
   stats_.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1367,80 +1377,151 @@ const GpuFrame& Engine::frame(int job) const {
   return frames_[j];
 }
 
-void Engine::read_mean(int job, double* rgb) const { read_mean_frame(frame(job), rgb); }
-
-void Engine::read_moments(int job, double* sum, double* sumsq, std::uint32_t* count) const {
-  const GpuFrame& f = frame(job);
-  const std::uint64_t px = std::uint64_t(f.width) * f.height;
-  if (sum) CK(cudaMemcpyAsync(sum, f.sum, px * 4 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  if (sumsq) CK(cudaMemcpyAsync(sumsq, f.sumsq, px * 4 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  if (count) CK(cudaMemcpyAsync(count, f.count, px * sizeof(std::uint32_t), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaStreamSynchronize(stream_));
+Engine::Slot& Engine::slot(std::size_t piece) {
+  Slot& sl = slots_[piece % kSlots];
+  if (!sl.mem) {
+    count_allocation();
+    CK(cudaMallocHost(reinterpret_cast<void**>(&sl.mem), kSlotBytes));
+    CK(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
+  }
+  return sl;
 }
 
-void Engine::read_image(int job, ToneMap op, double exposure, std::uint8_t* rgb) const {
+void Engine::pieces(std::size_t n, const std::function<void(std::size_t, unsigned char*)>& launch,
+                    const std::function<void(std::size_t, const unsigned char*)>& finish) {
+  std::size_t finished = 0;
+  auto finish_one = [&] {
+    Slot& sl = slot(finished);
+    CK(cudaEventSynchronize(sl.done));
+    finish(finished++, sl.mem);
+  };
+  try {
+    for (std::size_t k = 0; k < n; ++k) {
+      // Up to three pieces are with the GPU; the host empties the oldest.
+      if (k >= kSlots - 1) finish_one();
+      Slot& sl = slot(k);
+      launch(k, sl.mem);
+      CK(cudaEventRecord(sl.done, stream_));
+    }
+    while (finished < n) finish_one();
+  } catch (...) {
+    cudaStreamSynchronize(stream_);  // nothing may write a slot after this call
+    throw;
+  }
+}
+
+void Engine::read_mean(int job, double* rgb) { read_mean_frame(frame(job), rgb); }
+
+void Engine::read_moments(int job, double* sum, double* sumsq, std::uint32_t* count) {
+  CK(cudaSetDevice(device_));
+  const GpuFrame& f = frame(job);
+  const std::size_t px = std::size_t(f.width) * f.height;
+  struct Part {
+    unsigned char* to;
+    const unsigned char* from;
+    std::size_t bytes;
+  };
+  std::vector<Part> parts;
+  auto add = [&](void* to, const void* from, std::size_t bytes) {
+    for (std::size_t at = 0; to && at < bytes; at += kSlotBytes)
+      parts.push_back({static_cast<unsigned char*>(to) + at, static_cast<const unsigned char*>(from) + at,
+                       std::min(kSlotBytes, bytes - at)});
+  };
+  add(sum, f.sum, px * 4 * sizeof(double));
+  add(sumsq, f.sumsq, px * 4 * sizeof(double));
+  add(count, f.count, px * sizeof(std::uint32_t));
+  pieces(parts.size(),
+         [&](std::size_t k, unsigned char* mem) {
+           CK(cudaMemcpyAsync(mem, parts[k].from, parts[k].bytes, cudaMemcpyDeviceToHost, stream_));
+         },
+         [&](std::size_t k, const unsigned char* mem) { host_pool_.copy(parts[k].to, mem, parts[k].bytes); });
+}
+
+void Engine::read_image(int job, ToneMap op, double exposure, std::uint8_t* rgb) {
   read_image_frame(frame(job), op, exposure, rgb);
 }
 
-void Engine::read_mean_frame(const GpuFrame& f, double* rgb) const {
-  const std::uint64_t px = std::uint64_t(f.width) * f.height;
-  double* tmp = dev_alloc_async<double>(px * 3, pool_, stream_);
-  CK(launch_resolve(f.sum, f.count, px, 0, 1.0, nullptr, tmp, stream_));
-  CK(cudaMemcpyAsync(rgb, tmp, px * 3 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaFreeAsync(tmp, stream_));
-  CK(cudaStreamSynchronize(stream_));
+void Engine::read_mean_frame(const GpuFrame& f, double* rgb) {
+  CK(cudaSetDevice(device_));
+  const std::size_t px = std::size_t(f.width) * f.height;
+  constexpr std::size_t kPixels = std::size_t(1) << 17;  // 3 MiB of means
+  static_assert(kPixels * 3 * sizeof(double) <= kSlotBytes, "a piece fits its slot");
+  auto size = [&](std::size_t k) { return std::min(kPixels, px - k * kPixels); };
+  pieces((px + kPixels - 1) / kPixels,
+         [&](std::size_t k, unsigned char* mem) {
+           const std::size_t at = k * kPixels;
+           CK(launch_resolve(f.sum + 4 * at, f.count + at, size(k), 0, 1.0, nullptr, reinterpret_cast<double*>(mem),
+                             stream_));
+         },
+         [&](std::size_t k, const unsigned char* mem) {
+           host_pool_.copy(rgb + 3 * k * kPixels, mem, size(k) * 3 * sizeof(double));
+         });
 }
 
-void Engine::read_image_frame(const GpuFrame& f, ToneMap op, double exposure, std::uint8_t* rgb) const {
-  const std::uint64_t px = std::uint64_t(f.width) * f.height;
-  std::uint8_t* tmp = dev_alloc_async<std::uint8_t>(px * 3, pool_, stream_);
-  CK(launch_resolve(f.sum, f.count, px, static_cast<int>(op), exposure, tmp, nullptr, stream_));
-  CK(cudaMemcpyAsync(rgb, tmp, px * 3, cudaMemcpyDeviceToHost, stream_));
-  CK(cudaFreeAsync(tmp, stream_));
-  CK(cudaStreamSynchronize(stream_));
+void Engine::read_image_list(const std::vector<ImageRead>& list) {
+  CK(cudaSetDevice(device_));
+  // A slot takes parts of several small images, or a part of a large one.
+  struct Part {
+    const ImageRead* image;
+    std::size_t first, pixels, at;  // pixel range, and its place in the slot
+  };
+  std::vector<std::vector<Part>> loads;
+  std::size_t used = kSlotBytes;
+  for (const ImageRead& r : list) {
+    const std::size_t px = std::size_t(r.frame->width) * r.frame->height;
+    for (std::size_t first = 0; first < px;) {
+      if (kSlotBytes - used < 4096 || loads.empty()) {
+        loads.emplace_back();
+        used = 0;
+      }
+      const std::size_t n = std::min(px - first, (kSlotBytes - used) / 3 & ~std::size_t(255));
+      loads.back().push_back({&r, first, n, used});
+      used += (3 * n + 255) & ~std::size_t(255);
+      first += n;
+    }
+  }
+  pieces(loads.size(),
+         [&](std::size_t k, unsigned char* mem) {
+           for (const Part& p : loads[k])
+             CK(launch_resolve(p.image->frame->sum + 4 * p.first, p.image->frame->count + p.first, p.pixels,
+                               static_cast<int>(p.image->op), p.image->exposure, mem + p.at, nullptr, stream_));
+         },
+         [&](std::size_t k, const unsigned char* mem) {
+           if (loads[k].size() == 1) {
+             const Part& p = loads[k][0];
+             host_pool_.copy(p.image->rgb + 3 * p.first, mem + p.at, 3 * p.pixels);
+             return;
+           }
+           host_pool_.run(loads[k].size(), [&](std::size_t q) {
+             const Part& p = loads[k][q];
+             std::memcpy(p.image->rgb + 3 * p.first, mem + p.at, 3 * p.pixels);
+           });
+         });
+}
+
+void Engine::read_image_frame(const GpuFrame& f, ToneMap op, double exposure, std::uint8_t* rgb) {
+  read_image_list({{&f, op, exposure, rgb}});
 }
 
 void Engine::read_images(int n, const int* jobs, const ToneMap* ops, const double* exposures, std::uint8_t* const* rgb) {
-  CK(cudaSetDevice(device_));
-  if (n <= 0) return;
-  std::vector<const GpuFrame*> fr(static_cast<std::size_t>(n));
-  std::vector<std::size_t> at(static_cast<std::size_t>(n) + 1, 0), bytes(static_cast<std::size_t>(n));
-  for (int k = 0; k < n; ++k) {
-    fr[k] = &frame(jobs[k]);
-    bytes[k] = std::uint64_t(fr[k]->width) * fr[k]->height * 3;
-    at[k + 1] = at[k] + ((bytes[k] + 255) & ~std::size_t(255));
-  }
-  const std::size_t total = at[n];
-  if (total == 0) return;
-  std::uint8_t* dev = dev_alloc_async<std::uint8_t>(total, pool_, stream_);
-  for (int k = 0; k < n; ++k)
-    CK(launch_resolve(fr[k]->sum, fr[k]->count, std::uint64_t(fr[k]->width) * fr[k]->height, static_cast<int>(ops[k]),
-                      exposures[k], dev + at[k], nullptr, stream_));
-  if (readback_cap_ < total) {
-    CK(cudaStreamSynchronize(stream_));
-    if (readback_host_) CK(cudaFreeHost(readback_host_));
-    readback_host_ = nullptr;
-    readback_cap_ = 0;
-    count_allocation();
-    CK(cudaMallocHost(reinterpret_cast<void**>(&readback_host_), total));
-    readback_cap_ = total;
-  }
-  CK(cudaMemcpyAsync(readback_host_, dev, total, cudaMemcpyDeviceToHost, stream_));
-  CK(cudaFreeAsync(dev, stream_));
-  CK(cudaStreamSynchronize(stream_));
-  // Out of pinned memory into the caller's buffers, one image per task.
-  std::atomic<int> next{0};
-  auto copy = [&] {
-    for (int k; (k = next.fetch_add(1)) < n;) std::memcpy(rgb[k], readback_host_ + at[k], bytes[k]);
-  };
-  const int workers = std::min(n, static_cast<int>(std::min(16u, std::max(1u, std::thread::hardware_concurrency()))));
-  std::vector<std::thread> pool;
-  for (int w = 1; w < workers; ++w) pool.emplace_back(copy);
-  copy();
-  for (auto& t : pool) t.join();
+  std::vector<ImageRead> list;
+  for (int k = 0; k < n; ++k) list.push_back({&frame(jobs[k]), ops[k], exposures[k], rgb[k]});
+  read_image_list(list);
 }
 
 // ---------------------------------------------------------------------------
+namespace {
+// Rays of one piece of a query: 2 MiB of rays and 1.25 MiB of results in a slot.
+constexpr std::size_t kQueryRays = std::size_t(1) << 16;
+}  // namespace
+
+RtgSceneDev* Engine::upload_descriptor(const RtgSceneDev& d) {
+  static_assert(kQueryRays * (8 * sizeof(float) + 20) <= kSlotBytes, "a piece fits its slot");
+  RtgSceneDev* p = dev_alloc_async<RtgSceneDev>(1, pool_, stream_);
+  CK(cudaMemcpyAsync(p, &d, sizeof(d), cudaMemcpyHostToDevice, stream_));
+  return p;
+}
+
 void Engine::trace_closest(int scene_id, const float* rays, std::uint64_t n, bool brute, float* t, std::int32_t* prim,
                            std::int32_t* is_plane, float* bary) {
   CK(cudaSetDevice(device_));
@@ -1474,31 +1555,29 @@ void Engine::trace_closest(int scene_id, const float* rays, std::uint64_t n, boo
   s.use_bvh = !brute;
   RtgSceneDev d = job_descriptor(sc, s, GpuFrame{});
   if (!cfg_.refine_hits) d.prims64 = d.planes64 = nullptr;
-  RtgSceneDev* dd = dev_alloc<RtgSceneDev>(1);
-  float4* in = dev_alloc<float4>(2 * n);
-  float4* out = dev_alloc<float4>(n);
-  CK(cudaMemcpyAsync(dd, &d, sizeof(d), cudaMemcpyHostToDevice, stream_));
-  CK(cudaMemcpyAsync(in, rays, n * 8 * sizeof(float), cudaMemcpyHostToDevice, stream_));
-  CK(launch_ray_closest(dd, in, static_cast<std::uint32_t>(n), out, brute ? 1 : 0, cfg_.shape.closest_tree, stream_));
-  std::vector<float4> host(n);
-  CK(cudaMemcpyAsync(host.data(), out, n * sizeof(float4), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaStreamSynchronize(stream_));
-  dev_free(dd);
-  dev_free(in);
-  dev_free(out);
-  for (std::uint64_t i = 0; i < n; ++i) {
-    std::uint32_t w;
-    std::memcpy(&w, &host[i].y, 4);
-    const bool miss = w == kHitMiss;
-    const bool plane = !miss && (w & kHitPlaneBit);
-    if (t) t[i] = miss ? 0.f : host[i].x;
-    if (prim) prim[i] = miss ? -1 : (plane ? static_cast<std::int32_t>(w & ~kHitPlaneBit) : static_cast<std::int32_t>(sc.slot_prim[w]));
-    if (is_plane) is_plane[i] = plane ? 1 : 0;
-    if (bary) {
-      bary[2 * i] = host[i].z;
-      bary[2 * i + 1] = host[i].w;
-    }
-  }
+  RtgSceneDev* dd = upload_descriptor(d);
+  const std::size_t ns = static_cast<std::size_t>(n);
+  auto size = [&](std::size_t k) { return std::min(kQueryRays, ns - k * kQueryRays); };
+  auto results = [](unsigned char* mem) {
+    unsigned char* const r = mem + kQueryRays * 8 * sizeof(float);
+    return RayResults{reinterpret_cast<float*>(r), reinterpret_cast<std::int32_t*>(r + kQueryRays * 4),
+                      reinterpret_cast<std::int32_t*>(r + kQueryRays * 8), reinterpret_cast<float2*>(r + kQueryRays * 12)};
+  };
+  pieces((ns + kQueryRays - 1) / kQueryRays,
+         [&](std::size_t k, unsigned char* mem) {
+           host_pool_.copy(mem, rays + 8 * k * kQueryRays, size(k) * 8 * sizeof(float));
+           CK(launch_ray_closest(dd, reinterpret_cast<const float4*>(mem), static_cast<std::uint32_t>(size(k)),
+                                 results(mem), brute ? 1 : 0, cfg_.shape.closest_tree, stream_));
+         },
+         [&](std::size_t k, const unsigned char* mem) {
+           const RayResults r = results(const_cast<unsigned char*>(mem));
+           const std::size_t at = k * kQueryRays;
+           if (t) host_pool_.copy(t + at, r.t, size(k) * sizeof(float));
+           if (prim) host_pool_.copy(prim + at, r.prim, size(k) * sizeof(std::int32_t));
+           if (is_plane) host_pool_.copy(is_plane + at, r.plane, size(k) * sizeof(std::int32_t));
+           if (bary) host_pool_.copy(bary + 2 * at, r.bary, size(k) * 2 * sizeof(float));
+         });
+  CK(cudaFreeAsync(dd, stream_));
 }
 
 void Engine::trace_any(int scene_id, const float* rays, std::uint64_t n, bool brute, std::uint8_t* occluded) {
@@ -1509,19 +1588,19 @@ void Engine::trace_any(int scene_id, const float* rays, std::uint64_t n, bool br
   RenderSettings s = sc.host->settings;
   s.use_bvh = !brute;
   const RtgSceneDev d = job_descriptor(sc, s, GpuFrame{});
-  RtgSceneDev* dd = dev_alloc<RtgSceneDev>(1);
-  float4* in = dev_alloc<float4>(2 * n);
-  std::uint32_t* out = dev_alloc<std::uint32_t>(n);
-  CK(cudaMemcpyAsync(dd, &d, sizeof(d), cudaMemcpyHostToDevice, stream_));
-  CK(cudaMemcpyAsync(in, rays, n * 8 * sizeof(float), cudaMemcpyHostToDevice, stream_));
-  CK(launch_ray_any(dd, in, static_cast<std::uint32_t>(n), out, brute ? 1 : 0, cfg_.shape.shadow_tree, stream_));
-  std::vector<std::uint32_t> host(n);
-  CK(cudaMemcpyAsync(host.data(), out, n * sizeof(std::uint32_t), cudaMemcpyDeviceToHost, stream_));
-  CK(cudaStreamSynchronize(stream_));
-  dev_free(dd);
-  dev_free(in);
-  dev_free(out);
-  for (std::uint64_t i = 0; i < n; ++i) occluded[i] = host[i] ? 1 : 0;
+  RtgSceneDev* dd = upload_descriptor(d);
+  const std::size_t ns = static_cast<std::size_t>(n);
+  auto size = [&](std::size_t k) { return std::min(kQueryRays, ns - k * kQueryRays); };
+  pieces((ns + kQueryRays - 1) / kQueryRays,
+         [&](std::size_t k, unsigned char* mem) {
+           host_pool_.copy(mem, rays + 8 * k * kQueryRays, size(k) * 8 * sizeof(float));
+           CK(launch_ray_any(dd, reinterpret_cast<const float4*>(mem), static_cast<std::uint32_t>(size(k)),
+                             mem + kQueryRays * 8 * sizeof(float), brute ? 1 : 0, cfg_.shape.shadow_tree, stream_));
+         },
+         [&](std::size_t k, const unsigned char* mem) {
+           host_pool_.copy(occluded + k * kQueryRays, mem + kQueryRays * 8 * sizeof(float), size(k));
+         });
+  CK(cudaFreeAsync(dd, stream_));
 }
 
 }  // namespace rtg

@@ -31,6 +31,7 @@
 #include "device/wave.h"
 #include "host/compiled_scene.hpp"
 #include "host/flatten.hpp"
+#include "host/host_pool.hpp"
 
 namespace rtg {
 
@@ -96,6 +97,7 @@ struct GpuScene {
 // Per-job device framebuffer.
 struct GpuFrame {
   int width = 0, height = 0;
+  void* block = nullptr;  // one allocation holding the arrays below
   double* sum = nullptr;
   double* sumsq = nullptr;
   std::uint32_t* count = nullptr;
@@ -170,14 +172,13 @@ class Engine {
 
   // Results of the last render (plain) or of job `j` of the last batch.
   const GpuFrame& frame(int job = -1) const;
-  void read_mean(int job, double* rgb) const;
-  void read_moments(int job, double* sum, double* sumsq, std::uint32_t* count) const;
-  void read_image(int job, ToneMap op, double exposure, std::uint8_t* rgb) const;
-  // Several jobs' images: every resolve, then one device-to-host copy into pinned
-  // memory and one synchronisation, then copies out to rgb[k] on the host cores.
+  void read_mean(int job, double* rgb);
+  void read_moments(int job, double* sum, double* sumsq, std::uint32_t* count);
+  void read_image(int job, ToneMap op, double exposure, std::uint8_t* rgb);
+  // Several jobs' images, piece by piece through the pinned slots.
   void read_images(int n, const int* jobs, const ToneMap* ops, const double* exposures, std::uint8_t* const* rgb);
-  void read_mean_frame(const GpuFrame& f, double* rgb) const;
-  void read_image_frame(const GpuFrame& f, ToneMap op, double exposure, std::uint8_t* rgb) const;
+  void read_mean_frame(const GpuFrame& f, double* rgb);
+  void read_image_frame(const GpuFrame& f, ToneMap op, double exposure, std::uint8_t* rgb);
   const RenderStats& stats() const { return stats_; }
 
   // ---- serving: requests live in the wavefront across calls ----
@@ -299,7 +300,8 @@ class Engine {
   void stage(void* dst, const void* src, std::size_t n);
   void write_gen_table();
   void begin_stats();
-  void end_stats();
+  RtgSceneDev* upload_descriptor(const RtgSceneDev& d);
+  void end_stats(bool cancelled);
   void finish_timing();  // records the end event and fills stats_.device_ms
 
   int device_;
@@ -313,9 +315,30 @@ class Engine {
   std::size_t upload_cap_[2] = {0, 0};
   cudaEvent_t upload_ev_[2] = {nullptr, nullptr};
   bool upload_pending_[2] = {false, false};
-  // Pinned read-back buffer of read_images (grown on demand).
-  unsigned char* readback_host_ = nullptr;
-  std::size_t readback_cap_ = 0;
+  // Pinned slots that results (and rays) cross the bus through, and the threads that
+  // copy between them and the caller's memory. A read or a query is cut into pieces
+  // of at most a slot; while the GPU works on one, the host fills or empties others.
+  // Pageable copies cross at some 8 GB/s. Slots are allocated as they are first used.
+  static constexpr int kSlots = 4;
+  static constexpr std::size_t kSlotBytes = std::size_t(4) << 20;
+  struct Slot {
+    unsigned char* mem = nullptr;
+    cudaEvent_t done = nullptr;
+  };
+  Slot slots_[kSlots];
+  Slot& slot(std::size_t piece);
+  // launch(k, mem) fills or takes the slot and queues work for piece k on the stream,
+  // finish(k, mem) runs once that work is done; pieces finish in order.
+  void pieces(std::size_t n, const std::function<void(std::size_t, unsigned char*)>& launch,
+              const std::function<void(std::size_t, const unsigned char*)>& finish);
+  struct ImageRead {
+    const GpuFrame* frame;
+    ToneMap op;
+    double exposure;
+    std::uint8_t* rgb;
+  };
+  void read_image_list(const std::vector<ImageRead>& list);
+  HostPool host_pool_;
   int upload_next_ = 0;
   std::size_t pool_reserved_ = 0;
   bool bvh_preloaded_ = false;
@@ -338,6 +361,7 @@ class Engine {
   bool gen_dirty_ = false;
   WaveCounters last_counters_{};   // from the latest snapshot
   WaveCounters base_counters_{};   // at the start of the current render
+  bool counters_final_ = false;    // last_counters_ are the device's: nothing has run since
 };
 
 }  // namespace rtg

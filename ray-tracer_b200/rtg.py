@@ -511,21 +511,21 @@ class Context:
         return width, height
 
     def framebuffer_mean(self, job: int, width: int, height: int) -> np.ndarray:
-        out = np.zeros((height, width, 3), dtype=np.float64)
+        out = np.empty((height, width, 3), dtype=np.float64)
         self._check(lib().rtg_framebuffer_mean(self._h, job, _ptr(out, C.c_double)))
         return out
 
     def framebuffer_moments(self, job: int, width: int, height: int):
-        s = np.zeros((height, width, 4), dtype=np.float64)
-        q = np.zeros((height, width, 4), dtype=np.float64)
-        n = np.zeros((height, width), dtype=np.uint32)
+        s = np.empty((height, width, 4), dtype=np.float64)
+        q = np.empty((height, width, 4), dtype=np.float64)
+        n = np.empty((height, width), dtype=np.uint32)
         self._check(lib().rtg_framebuffer_moments(self._h, job, _ptr(s, C.c_double), _ptr(q, C.c_double),
                                                   _ptr(n, C.c_uint32)))
         return s[..., :3], q[..., :3], n
 
     def image(self, job: int, width: int, height: int, tone_map: Optional[str] = None,
               exposure: float = 1.0) -> np.ndarray:
-        out = np.zeros((height, width, 3), dtype=np.uint8)
+        out = np.empty((height, width, 3), dtype=np.uint8)
         op = -1 if tone_map is None else TONE_MAPS[tone_map]
         self._check(lib().rtg_image_rgb8(self._h, job, op, exposure, _ptr(out, C.c_uint8)))
         return out
@@ -558,10 +558,10 @@ class Context:
     def trace_closest(self, scene_id: int, rays: np.ndarray, brute: bool = False):
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
         n = rays.shape[0]
-        t = np.zeros(n, np.float32)
-        prim = np.zeros(n, np.int32)
-        plane = np.zeros(n, np.int32)
-        bary = np.zeros((n, 2), np.float32)
+        t = np.empty(n, np.float32)
+        prim = np.empty(n, np.int32)
+        plane = np.empty(n, np.int32)
+        bary = np.empty((n, 2), np.float32)
         self._check(lib().rtg_trace_closest(self._h, scene_id, _ptr(rays, C.c_float), n, int(brute),
                                             _ptr(t, C.c_float), _ptr(prim, C.c_int32), _ptr(plane, C.c_int32),
                                             _ptr(bary, C.c_float)))
@@ -580,10 +580,10 @@ class Context:
         (at most NOALLOC_MAX_RAYS rays per call)."""
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
         n = rays.shape[0]
-        t = np.zeros(n, np.float32)
-        prim = np.zeros(n, np.int32)
-        plane = np.zeros(n, np.int32)
-        bary = np.zeros((n, 2), np.float32)
+        t = np.empty(n, np.float32)
+        prim = np.empty(n, np.int32)
+        plane = np.empty(n, np.int32)
+        bary = np.empty((n, 2), np.float32)
         self._check(lib().rtg_trace_closest_noalloc(self._h, scene_id, _ptr(rays, C.c_float), n, int(brute),
                                                     _ptr(t, C.c_float), _ptr(prim, C.c_int32),
                                                     _ptr(plane, C.c_int32), _ptr(bary, C.c_float)))
@@ -592,7 +592,7 @@ class Context:
     def trace_any(self, scene_id: int, rays: np.ndarray, brute: bool = False) -> np.ndarray:
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
         n = rays.shape[0]
-        occ = np.zeros(n, np.uint8)
+        occ = np.empty(n, np.uint8)
         self._check(lib().rtg_trace_any(self._h, scene_id, _ptr(rays, C.c_float), n, int(brute), _ptr(occ, C.c_uint8)))
         return occ
 
@@ -643,13 +643,13 @@ class Context:
         return RenderProgress.from_c(p)
 
     def request_mean(self, rid: int, width: int, height: int) -> np.ndarray:
-        out = np.zeros((height, width, 3), dtype=np.float64)
+        out = np.empty((height, width, 3), dtype=np.float64)
         self._check(lib().rtg_request_mean(self._h, rid, _ptr(out, C.c_double)))
         return out
 
     def request_image(self, rid: int, width: int, height: int, tone_map: Optional[str] = None,
                       exposure: float = 1.0) -> np.ndarray:
-        out = np.zeros((height, width, 3), dtype=np.uint8)
+        out = np.empty((height, width, 3), dtype=np.uint8)
         op = -1 if tone_map is None else TONE_MAPS[tone_map]
         self._check(lib().rtg_request_image_rgb8(self._h, rid, op, exposure, _ptr(out, C.c_uint8)))
         return out
