@@ -601,23 +601,37 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
 }
 
 // ---------------------------------------------------------------------------
+// Sample i of a list of passes.
+__device__ __forceinline__ CameraSample listed_sample(const RtgSceneDev& J, const PassList& passes, std::uint64_t i) {
+  int k = 0;
+  while (k + 1 < passes.n && i >= passes.seg[k].count) i -= passes.seg[k++].count;
+  return camera_sample(J, passes.seg[k], i);
+}
+
 // Whitted-style direct integrator (src/rendering/integrator.cpp:141-174): every
 // light at diffuse hits, recursion through metal, and a deterministic Fresnel
 // split at dielectrics. The recursion becomes a depth-first walk of each sample's
 // tree with a stack of pending refraction branches, which keeps the reference's RNG
 // draw order.
 //
-// Scheduled like the path kernel: each warp holds kDirectPaths samples in shared
-// memory; `ready` ones have a ray to trace, `lit` ones the next light of a diffuse
-// hit to sample and test. The surface of a lit sample is made again from its hit for
-// each light, which costs less than keeping it. Pending branches are in device
-// memory: at most one per level, so min(max depth, kDirectStack) records a sample.
-// Bound by the serial walk of the largest trees: of the 7.3 ms that the mesh takes
-// at 640x360x16, depth 8, some 4.3 ms are the longest sample's chain (that is also
-// what one sample a pixel takes), 2.5 ms the throughput. One thread per whole sample,
-// where lanes wait for the longest tree of their warp, measured 8.4 ms with the same
-// walk. First in, first out queues, which advance the long samples sooner, measured
-// 7.6 ms: they lose more coherence than tail.
+// Two kernels. From kDirectWarpSamples samples a launch up, k_direct schedules them like
+// the path kernel: each warp holds kDirectPaths samples in shared memory; `ready` ones
+// have a ray to trace, `lit` ones the next light of a diffuse hit to sample and test
+// (its surface is made again from the hit for each light, which costs less than
+// keeping it). Pending branches are in device memory: at most one per level, so
+// min(max depth, kDirectStack) records a sample. Smaller launches take a thread a
+// sample, k_direct_sample.
+//
+// What bounds both: the divergence between trees (k_direct's lanes are full, a warp of
+// k_direct_sample waits for its longest tree), and the serial chain of the largest
+// tree: on the mesh at depth 8 one sample a pixel takes 4.3 of the 7.2 ms that 640x360x16
+// take. A vertex of that chain takes k_direct longer (its state goes through shared
+// memory), so what wins is the number of samples. k_direct_sample's time over k_direct's
+// on the mesh / the sphere field at depth 8: 16 ki samples 0.91 / 0.79, 256 ki 0.93 / 0.78,
+// 1 Mi 1.11 to 1.28 / 0.95 to 0.98, 4 Mi 1.18 / 1.05, 12 Mi 1.26 / 1.04 (Cornell: 0.70 at 16
+// ki, 1.0 at 1 Mi, 1.05 at 4 Mi). First in, first out queues, which advance the long
+// samples sooner, cost 4%: they lose more coherence than tail.
+constexpr std::uint64_t kDirectWarpSamples = std::uint64_t(1) << 20;
 constexpr int kDirectStack = 48;
 constexpr int kDirectPaths = 48;
 constexpr int kPendingRows = 3;  // float4 rows of a pending branch: (o, d.x), (d.yz, w.xy), (w.z, depth)
@@ -641,8 +655,8 @@ constexpr std::size_t kDirectWarpSmem = sizeof(DirectPaths) + sizeof(typename Wa
 
 template <int kBlock, bool kGeneral>
 __global__ void __launch_bounds__(kBlock, kPathThreads / kBlock)
-k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, WaveCounters* C, float4* stack_rows,
-         int stack_depth, int tree) {
+k_direct(const RtgSceneDev* __restrict__ job, const __grid_constant__ PassList passes, float4* radiance, WaveCounters* C,
+         float4* stack_rows, int stack_depth, int tree) {
   extern __shared__ __align__(16) unsigned char smem[];
   using Entry = typename Walk<kGeneral>::Entry;
   const int lane = threadIdx.x & 31;
@@ -656,7 +670,7 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
   for (int k = lane; k < kDirectPaths; k += 32) S.idle[k] = static_cast<std::uint8_t>(k);
   __syncwarp();
   const RtgSceneDev& J = *job;
-  const std::uint32_t count = static_cast<std::uint32_t>(seg.count);  // under 2^32 (the radiance slots are)
+  const std::uint32_t count = static_cast<std::uint32_t>(passes.samples());  // under 2^32 (the radiance slots are)
   const unsigned below = (1u << lane) - 1u;
   Walk<kGeneral> walk;
   TraceCount tc;
@@ -665,23 +679,29 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
   int n_idle = kDirectPaths, n_ready = 0, n_lit = 0;
   while (true) {
     const int n_new = more ? n_idle : 0;
-    enum { kLight, kTrace, kNew } step;
-    if (n_lit >= 32) step = kLight;
-    else if (n_ready >= 32) step = kTrace;
-    else if (n_new >= 32) step = kNew;
-    else {
-      if ((n_lit | n_ready | n_new) == 0) break;
-      step = n_lit >= n_ready && n_lit >= n_new ? kLight : (n_ready >= n_new ? kTrace : kNew);
+    // Full batches of one kind while there are any; else lights and rays together, so
+    // that what is left of the long samples does not wait for each other's kind.
+    int n_light = 0, n_trace = 0;
+    if (n_lit >= 32) {
+      n_light = 32;
+    } else if (n_ready >= 32) {
+      n_trace = 32;
+    } else if (n_new < 32) {
+      n_light = n_lit;
+      n_trace = min(n_ready, 32 - n_lit);
     }
     bool on = false, ray = false;  // the lane has a sample; the sample has a ray to trace in this step
+    bool light = false;            // that ray is a shadow ray
     int p = 0;
     float3 o = f3(0.f, 0.f, 0.f), d = o;
     float tmax = FLT_MAX;
-    if (step == kLight) {
-      const int take = min(n_lit, 32);
-      n_lit -= take;
-      on = lane < take;
-      if (on) {
+    if (n_light + n_trace > 0) {
+      n_lit -= n_light;
+      n_ready -= n_trace;
+      rays += n_trace;
+      light = lane < n_light;
+      on = lane < n_light + n_trace;
+      if (light) {
         p = S.lit[n_lit + lane];
         const Surface s = make_surface(J, get3(S.o, p), get3(S.d, p),
                                        RayHit{S.hit[0][p], __float_as_uint(S.hit[1][p]), S.hit[2][p], S.hit[3][p]});
@@ -701,18 +721,15 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
             ray = true;
           }
         }
-      }
-      shadow_rays += __popc(__ballot_sync(kFull, ray));
-    } else if (step == kTrace) {
-      const int take = min(n_ready, 32);
-      n_ready -= take;
-      on = ray = lane < take;
-      rays += take;
-      if (on) {
-        p = S.ready[n_ready + lane];
+      } else if (on) {
+        p = S.ready[n_ready + lane - n_light];
         o = get3(S.o, p);
         d = get3(S.d, p);
+        ray = true;
       }
+      shadow_rays += __popc(__ballot_sync(kFull, light && ray));
+    } else if (n_new == 0) {
+      break;
     } else {
       int take = min(n_idle, 32);
       std::uint32_t base = 0;
@@ -731,7 +748,7 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
       rays += take;
       if (on) {
         p = S.idle[n_idle + lane];
-        const CameraSample cs = camera_sample(J, seg, base + lane);
+        const CameraSample cs = listed_sample(J, passes, base + lane);
         o = cs.o;
         d = cs.d;
         set3(S.o, p, o);
@@ -749,11 +766,11 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
     }
     __syncwarp();
     RayHit h{tmax, kHitMiss, 0.f, 0.f};
-    if (ray) h = walk(J, o, d, tmax, step == kLight, stack, tree, tc);
+    if (ray) h = walk(J, o, d, tmax, light, stack, tree, tc);
     // What the sample does next: trace S.o, S.d; sample a light; or neither, and then
     // a pending branch is next, or the sample is done.
     bool go = false, lit = false;
-    if (on && step == kLight) {
+    if (light) {
       if (ray && h.word == kHitMiss) mad_to(S.sum, p, get3(S.f, p), get3(S.li, p));
       const int next = S.light_index[p] + 1;
       S.light_index[p] = next;
@@ -856,31 +873,141 @@ k_direct(const RtgSceneDev* __restrict__ job, DevSegment seg, float4* radiance, 
   }
 }
 
+struct Pending {
+  float3 o, d, w;
+  int depth;
+};
+
+// One sample a thread: the whole tree, with the pending branches in local memory.
+template <int kBlock, bool kGeneral>
+__global__ void __launch_bounds__(kBlock) k_direct_sample(const RtgSceneDev* __restrict__ job,
+                                                          const __grid_constant__ PassList passes, float4* radiance,
+                                                          WaveCounters* C, int tree) {
+  __shared__ uint2 stack[kStackSmem * kBlock];
+  int* const column = reinterpret_cast<int*>(stack) + threadIdx.x;
+  TraceCount tc;
+  std::uint64_t rays = 0, shadow_rays = 0;
+  const RtgSceneDev& J = *job;
+  const std::uint64_t count = passes.samples();
+  auto closest = [&](float3 o, float3 d) {
+    if (kGeneral) {
+      if (!J.use_bvh) return closest_brute<false>(J, o, d, kRayTMin, FLT_MAX, tc);
+      if (tree == 8) return closest_hit8<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, stack + threadIdx.x, tc);
+    }
+    return closest_hit<kStackSmem, kBlock, false>(J, o, d, kRayTMin, FLT_MAX, column, tc);
+  };
+  auto blocked = [&](const ShadowRay& r) {
+    if (kGeneral) {
+      if (!J.use_bvh) return any_brute(J, r.o, r.d, kRayTMin, r.tmax);
+      if (tree == 8) return any_hit8<kStackSmem, kBlock, false>(J, r.o, r.d, kRayTMin, r.tmax, stack + threadIdx.x, tc);
+    }
+    return any_hit4<kStackSmem, kBlock, false>(J, r.o, r.d, kRayTMin, r.tmax, column, tc);
+  };
+  const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * kBlock;
+  for (std::uint64_t w = static_cast<std::uint64_t>(blockIdx.x) * kBlock + threadIdx.x; w < count; w += stride) {
+    CameraSample cs = listed_sample(J, passes, w);
+    Pending todo[kDirectStack];
+    int sp = 0;
+    Pending cur{cs.o, cs.d, f3(1.f, 1.f, 1.f), 0};
+    float3 L = f3(0.f, 0.f, 0.f);
+    bool overflow = false;
+    while (true) {
+      ++rays;
+      const RayHit h = closest(cur.o, cur.d);
+      bool next = false;
+      if (h.word == kHitMiss) {
+        L = mad3(cur.w, background(J, cur.d), L);
+      } else {
+        const Surface s = make_surface(J, cur.o, cur.d, h);
+        const DevMaterial m = J.materials[s.material];
+        L = mad3(cur.w, emitted(m, s.front), L);
+        if (cur.depth < J.max_depth) {
+          const std::uint32_t kind = kind_of(m);
+          if (kind == kLambertian) {
+            // Every light, in order.
+            float3 sum = f3(0.f, 0.f, 0.f);
+            for (int li = 0; li < J.n_lights; ++li) {
+              const LightSample ls = sample_light(J.lights + li, s, cs.rng);
+              if (!ls.valid) continue;
+              const float3 f = brdf_cos(m, s, ls.wi);
+              if (is_zero3(f) || is_zero3(ls.li_over_pdf)) continue;
+              ++shadow_rays;
+              if (!blocked(shadow_ray(s, ls))) sum = mad3(f, ls.li_over_pdf, sum);
+            }
+            L = mad3(cur.w, sum, L);
+          } else if (kind == kMetal) {
+            Scatter sr;
+            if (scatter(m, cur.d, s, cs.rng, sr)) {
+              cur = Pending{spawn_towards(s.p, s.gn, sr.dir), sr.dir, cur.w * f3(m.colour_a), cur.depth + 1};
+              next = true;
+            }
+          } else if (kind == kDielectric) {
+            const float ior = m.head.z;
+            const float3 in = unit_or(cur.d, f3(0.f, 0.f, 0.f));
+            const float eta = s.front ? 1.f / ior : ior;
+            const float cos_i = fminf(-dot3(in, s.n), 1.f);
+            float3 refr;
+            const bool can = refract3(in, s.n, eta, refr);
+            const float F = can ? schlick(cos_i, eta) : 1.f;
+            const float3 tint = f3(m.colour_a);
+            if (can) {
+              if (sp < kDirectStack) {
+                const float3 td = unit_or(refr, f3(0.f, 0.f, 0.f));
+                todo[sp++] = Pending{spawn_towards(s.p, s.gn, td), td, cur.w * tint * __fsub_rn(1.f, F), cur.depth + 1};
+              } else {
+                overflow = true;
+              }
+            }
+            const float3 rd = reflect3(in, s.n);
+            cur = Pending{spawn_towards(s.p, s.gn, rd), rd, cur.w * tint * F, cur.depth + 1};
+            next = true;
+          }
+        }
+      }
+      if (next) continue;
+      if (sp == 0) break;
+      cur = todo[--sp];
+    }
+    if (overflow) atomicExch(&C->error, 2u);
+    radiance[cs.sample] = make_float4(L.x, L.y, L.z, 0.f);
+  }
+  warp_add_u64(rays, &C->rays);
+  warp_add_u64(shadow_rays, &C->shadow_rays);
+}
+
 // ---------------------------------------------------------------------------
-__global__ void k_accumulate(const RtgSceneDev* __restrict__ job, DevSegment seg, const float4* __restrict__ radiance) {
+// Folds finished passes of one job, in their order: each pixel's framebuffer entry is
+// read and written once for all of them (136 bytes a pixel, as much as 8 samples).
+__global__ void __launch_bounds__(256) k_accumulate(const RtgSceneDev* __restrict__ job,
+                                                    const __grid_constant__ PassList passes,
+                                                    const float4* __restrict__ radiance) {
   const RtgSceneDev& J = *job;
   const std::uint64_t pixels = static_cast<std::uint64_t>(J.width) * static_cast<std::uint64_t>(J.height);
   const std::uint64_t p = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   std::uint64_t bad = 0;
   if (p < pixels) {
-    const std::uint32_t k = seg.pass_spp;
-    const float4* src = radiance + seg.sample_base + p * k;
     double s0 = J.fb_sum[4 * p], s1 = J.fb_sum[4 * p + 1], s2 = J.fb_sum[4 * p + 2];
     double q0 = J.fb_sumsq[4 * p], q1 = J.fb_sumsq[4 * p + 1], q2 = J.fb_sumsq[4 * p + 2];
-    for (std::uint32_t j = 0; j < k; ++j) {
-      const float4 v = src[j];
-      double r = v.x, g = v.y, b = v.z;
-      // A non-finite or negative sample would poison the pixel: record it as black.
-      if (!isfinite(r) || !isfinite(g) || !isfinite(b) || r < 0 || g < 0 || b < 0) {
-        r = g = b = 0;
-        ++bad;
+    std::uint32_t n = 0;
+    for (int i = 0; i < passes.n; ++i) {
+      const std::uint32_t k = passes.seg[i].pass_spp;
+      const float4* src = radiance + passes.seg[i].sample_base + p * k;
+      n += k;
+      for (std::uint32_t j = 0; j < k; ++j) {
+        const float4 v = src[j];
+        double r = v.x, g = v.y, b = v.z;
+        // A non-finite or negative sample would poison the pixel: record it as black.
+        if (!isfinite(r) || !isfinite(g) || !isfinite(b) || r < 0 || g < 0 || b < 0) {
+          r = g = b = 0;
+          ++bad;
+        }
+        s0 = __dadd_rn(s0, r); s1 = __dadd_rn(s1, g); s2 = __dadd_rn(s2, b);
+        q0 = fma(r, r, q0); q1 = fma(g, g, q1); q2 = fma(b, b, q2);
       }
-      s0 += r; s1 += g; s2 += b;
-      q0 += r * r; q1 += g * g; q2 += b * b;
     }
     J.fb_sum[4 * p] = s0; J.fb_sum[4 * p + 1] = s1; J.fb_sum[4 * p + 2] = s2;
     J.fb_sumsq[4 * p] = q0; J.fb_sumsq[4 * p + 1] = q1; J.fb_sumsq[4 * p + 2] = q2;
-    J.fb_count[p] += k;
+    J.fb_count[p] += n;
   }
   warp_add_u64(bad, J.stats);
 }
@@ -1070,10 +1197,10 @@ cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& s
   }
 }
 
-cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const DevSegment& seg,
+cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const PassList& passes,
                               const float4* radiance, cudaStream_t stream) {
   const unsigned blocks = static_cast<unsigned>((pixels + 255) / 256);
-  k_accumulate<<<blocks, 256, 0, stream>>>(job_dev, seg, radiance);
+  k_accumulate<<<blocks, 256, 0, stream>>>(job_dev, passes, radiance);
   return cudaGetLastError();
 }
 
@@ -1087,28 +1214,38 @@ const Grid& direct_grid() {
 }
 
 template <bool kGeneral>
-cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance,
+cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance,
                                    WaveCounters* cnt, float4* pending, int pending_depth, int tree, cudaStream_t stream) {
+  if (passes.samples() < kDirectWarpSamples) {
+    constexpr int kMaxPerSm = 2048 / kDirectBlock;
+    static const Grid grid = resident_grid(k_direct_sample<kDirectBlock, kGeneral>, kDirectBlock, 0, kMaxPerSm);
+    if (grid.err != cudaSuccess) return grid.err;
+    k_direct_sample<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, 0, stream>>>(job_dev, passes,
+                                                                                               radiance, cnt, tree);
+    return cudaGetLastError();
+  }
   const Grid& grid = direct_grid<kGeneral>();
   if (grid.err != cudaSuccess) return grid.err;
   const cudaError_t e = cudaMemsetAsync(&cnt->direct_fetch, 0, sizeof(cnt->direct_fetch), stream);
   if (e != cudaSuccess) return e;
   k_direct<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, kDirectBlock / 32 * kDirectWarpSmem<kGeneral>,
-                                     stream>>>(job_dev, seg, radiance, cnt, pending, pending_depth, tree);
+                                     stream>>>(job_dev, passes, radiance, cnt, pending, pending_depth, tree);
   return cudaGetLastError();
 }
 }  // namespace
 
-int direct_pending_depth(int max_depth) { return max_depth < kDirectStack ? max_depth : kDirectStack; }
+int direct_pending_depth(int max_depth, std::uint64_t samples) {
+  return samples < kDirectWarpSamples ? 0 : (max_depth < kDirectStack ? max_depth : kDirectStack);
+}
 
 std::size_t direct_pending_bytes(int sms, int pending_depth) {
   return static_cast<std::size_t>(sms) * (kPathThreads / 32) * kDirectPaths * pending_depth * kPendingRows * sizeof(float4);
 }
 
-cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance, WaveCounters* cnt,
+cudaError_t launch_direct(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance, WaveCounters* cnt,
                           float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream) {
-  return general ? launch_direct_instance<true>(job_dev, seg, radiance, cnt, pending, pending_depth, tree, stream)
-                 : launch_direct_instance<false>(job_dev, seg, radiance, cnt, pending, pending_depth, tree, stream);
+  return general ? launch_direct_instance<true>(job_dev, passes, radiance, cnt, pending, pending_depth, tree, stream)
+                 : launch_direct_instance<false>(job_dev, passes, radiance, cnt, pending, pending_depth, tree, stream);
 }
 
 cudaError_t launch_resolve(const double* fb_sum, const std::uint32_t* fb_count, std::uint64_t pixels, int tone_map,

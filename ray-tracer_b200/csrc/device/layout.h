@@ -178,6 +178,22 @@ struct alignas(16) DevSegment {
                               // is at sample_base + p * pass_spp + (s - pass_s0)
 };
 
+// Passes of one job, in order: what the direct integrator traces and what is folded
+// into the framebuffer in one launch.
+constexpr int kMaxPassList = 8;
+struct PassList {
+  int n = 0;
+  DevSegment seg[kMaxPassList];
+#if defined(__CUDACC__)
+  __host__ __device__
+#endif
+  std::uint64_t samples() const {
+    std::uint64_t c = 0;
+    for (int k = 0; k < n; ++k) c += seg[k].count;
+    return c;
+  }
+};
+
 // Device-side progress of one segment slot (zeroed when the slot is assigned).
 struct alignas(16) SegmentProgress {
   std::uint64_t generated;    // camera samples handed to the wavefront

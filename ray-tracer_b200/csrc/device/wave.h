@@ -52,18 +52,17 @@ struct LaunchShape {
 cudaError_t launch_plan(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream);
 cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& shape, cudaStream_t stream);
 
-// Per-pixel reduction of a finished segment into its job's framebuffer.
-cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const DevSegment& seg,
+// Per-pixel reduction of finished passes into their job's framebuffer.
+cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const PassList& passes,
                               const float4* radiance, cudaStream_t stream);
 
-// Direct (Whitted) integrator over one whole segment. Writes each sample's radiance
-// slot. `pending` holds direct_pending_bytes(SMs, pending_depth) bytes for the
+// Direct (Whitted) integrator over whole passes. Writes each sample's radiance slot. `pending` holds direct_pending_bytes(SMs, pending_depth) bytes for the
 // samples' pending refraction branches, pending_depth of them a sample
-// (direct_pending_depth of the job's maximum depth; 0 for a scene without dielectrics,
-// whose samples have none). `general`: an eight-wide walk (tree 8) or brute force.
-int direct_pending_depth(int max_depth);
+// (direct_pending_depth of the job's maximum depth and the passes' samples; 0 for a
+// scene without dielectrics, whose samples have none). `general`: an eight-wide walk (tree 8) or brute force.
+int direct_pending_depth(int max_depth, std::uint64_t samples);
 std::size_t direct_pending_bytes(int sms, int pending_depth);
-cudaError_t launch_direct(const RtgSceneDev* job_dev, const DevSegment& seg, float4* radiance, WaveCounters* cnt,
+cudaError_t launch_direct(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance, WaveCounters* cnt,
                           float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream);
 
 // Framebuffer means (mean_out, 3 doubles per pixel) and/or their tone-mapped

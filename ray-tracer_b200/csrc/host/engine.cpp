@@ -79,6 +79,7 @@ constexpr int kJobSlots = 4096;  // job descriptors resident at once
 // ends with a wait for its slowest warps (0.03 ms on the sphere field, 0.1 ms on the
 // mix, 0.2 ms on the mesh); requests take one, so a preview waits less for its turn.
 constexpr std::uint32_t kRenderItems = 4;
+constexpr std::uint64_t kDirectSamples = std::uint64_t(1) << 22;  // of the passes the direct integrator traces together
 
 }  // namespace
 
@@ -915,14 +916,35 @@ bool Engine::issue_pass(Job& j) {
   return true;
 }
 
-bool Engine::run_direct_pass(Job& j) {
+bool Engine::run_direct_passes(Job& j) {
   Wave& W = *wave_;
   counters_final_ = false;
-  const std::uint32_t k = next_pass_size(j);
-  const std::uint64_t count = j.pixels * k;
+  // Passes of one launch: a progressive render's small ones go together, since the
+  // serial chain of a launch's largest tree costs the same for one sample a pixel as
+  // for many (mesh 256x256x16, depth 8, progressive: 22 ms pass by pass, 6 ms together).
+  PassList passes;
+  const std::uint32_t issued = j.issued;
+  while (j.issued < j.target && passes.n < kMaxPassList) {
+    const std::uint32_t k = next_pass_size(j);
+    const std::uint64_t count = j.pixels * k;
+    if (passes.n && passes.samples() + count > kDirectSamples) break;
+    std::uint64_t at = 0;
+    if (!W.rad_alloc(count, at)) break;
+    DevSegment& d = passes.seg[passes.n++];
+    d = DevSegment{};
+    d.job = static_cast<std::uint32_t>(j.desc_slot);
+    d.pass_s0 = j.issued;
+    d.pass_spp = k;
+    d.count = count;
+    d.sample_base = at;
+    j.issued += k;
+  }
+  j.issued = issued;  // counted pass by pass below
+  if (!passes.n) return false;  // retried once radiance space frees up
   int pending_depth = 0;
   for (const Material& m : scene(j.scene_id).host->materials)
-    if (std::holds_alternative<Dielectric>(m)) pending_depth = direct_pending_depth(j.settings.max_depth);
+    if (std::holds_alternative<Dielectric>(m))
+      pending_depth = direct_pending_depth(j.settings.max_depth, passes.samples());
   const std::size_t pending_bytes = direct_pending_bytes(W.sms, pending_depth);
   if (W.direct_pending_bytes < pending_bytes) {
     CK(cudaStreamSynchronize(stream_));
@@ -932,43 +954,47 @@ bool Engine::run_direct_pass(Job& j) {
     W.direct_pending = dev_alloc<float4>(pending_bytes / sizeof(float4));
     W.direct_pending_bytes = pending_bytes;
   }
-  std::uint64_t at = 0;
-  if (!W.rad_alloc(count, at)) return false;  // retried once radiance space frees up
-  DevSegment d{};
-  d.job = static_cast<std::uint32_t>(j.desc_slot);
-  d.pass_s0 = j.issued;
-  d.pass_spp = k;
-  d.count = count;
-  d.sample_base = at;
   const bool timed = cfg_.time_kernels;
   if (timed) CK(cudaEventRecord(W.tev[8], stream_));
-  CK(launch_direct(W.jobs_dev + j.desc_slot, d, W.wb.radiance, W.wb.cnt, W.direct_pending, pending_depth,
+  CK(launch_direct(W.jobs_dev + j.desc_slot, passes, W.wb.radiance, W.wb.cnt, W.direct_pending, pending_depth,
                    !j.settings.use_bvh || cfg_.shape.closest_tree == 8, cfg_.shape.closest_tree, stream_));
   if (timed) CK(cudaEventRecord(W.tev[9], stream_));
-  CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, d, W.wb.radiance, stream_));
-  stats_.kernel_launches += 2;
-  // Reported once it has run, so progress times are device-complete.
-  CK(cudaStreamSynchronize(stream_));
-  if (timed) {
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
-    stats_.direct_ms += ms;
+  stats_.kernel_launches++;
+  for (int k = 0; k < passes.n; ++k) W.rad_release(passes.seg[k].sample_base, passes.seg[k].count);
+  for (int p = 0; p < passes.n;) {
+    if (p > 0 && cancel_ && *cancel_) break;  // as between launches: the rest is dropped
+    // As in retire_segments: one by one where a callback may look.
+    PassList fold;
+    for (; fold.n < (j.on_pass ? 1 : passes.n); ++fold.n) fold.seg[fold.n] = passes.seg[p++];
+    CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, fold, W.wb.radiance, stream_));
+    stats_.kernel_launches++;
+    // Reported once it has run, so progress times are device-complete.
+    CK(cudaStreamSynchronize(stream_));
+    if (j.done == issued) {
+      if (timed) {
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
+        stats_.direct_ms += ms;
+      }
+      CK(cudaMemcpy(&last_counters_, W.wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+      if (last_counters_.error)
+        throw CudaFailure("device error flag " + std::to_string(last_counters_.error) +
+                          (last_counters_.error == 2 ? " (direct integrator branch stack overflow)" : ""));
+    }
+    const WaveCounters& c = last_counters_;
+    for (int k = 0; k < fold.n; ++k) {
+      j.issued += fold.seg[k].pass_spp;
+      j.passes_issued++;
+      j.done += fold.seg[k].pass_spp;
+      j.prog.pass++;
+      j.prog.spp_done = j.done;
+      j.prog.finished = j.done >= j.target;
+      j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
+      j.prog.rays = (c.rays - base_counters_.rays) + (c.shadow_rays - base_counters_.shadow_rays);
+      stats_.passes++;
+      if (j.on_pass) j.on_pass(j.prog);
+    }
   }
-  W.rad_release(at, count);
-  WaveCounters c{};
-  CK(cudaMemcpy(&c, W.wb.cnt, sizeof(c), cudaMemcpyDeviceToHost));
-  if (c.error) throw CudaFailure("device error flag " + std::to_string(c.error) +
-                                 (c.error == 2 ? " (direct integrator branch stack overflow)" : ""));
-  last_counters_ = c;
-  j.issued += k;
-  j.passes_issued++;
-  j.done += k;
-  j.prog.pass++;
-  j.prog.spp_done = j.done;
-  j.prog.finished = j.done >= j.target;
-  j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
-  j.prog.rays = (c.rays - base_counters_.rays) + (c.shadow_rays - base_counters_.shadow_rays);
-  stats_.passes++;
   return true;
 }
 
@@ -994,8 +1020,7 @@ void Engine::refill() {
     }
     if (!best) return;
     if (best->direct) {
-      // One whole pass per call, so cancellation is checked between passes.
-      if (run_direct_pass(*best) && best->on_pass) best->on_pass(best->prog);
+      run_direct_passes(*best);
       return;
     }
     // Enough samples are open ahead of this job: wait. A priority-0 job (a plain
@@ -1033,11 +1058,17 @@ void Engine::retire_segments(Job& j, std::vector<PassEvent>* events) {
     return;
   }
   while (!j.segs.empty() && segs_[j.segs.front()].complete) {
-    const int slot = j.segs.front();
-    const Seg& s = segs_[slot];
+    // A pass callback may read the framebuffer, which then holds the passes reported so
+    // far and no other; without one, the finished passes are folded together.
+    PassList passes;
+    const int most = j.on_pass ? 1 : kMaxPassList;
+    for (int slot : j.segs) {
+      if (passes.n == most || !segs_[slot].complete) break;
+      passes.seg[passes.n++] = segs_[slot].d;
+    }
     const bool timed = cfg_.time_kernels;
     if (timed) CK(cudaEventRecord(W.tev[8], stream_));
-    CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, s.d, W.wb.radiance, stream_));
+    CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, passes, W.wb.radiance, stream_));
     stats_.kernel_launches++;
     if (timed) {
       CK(cudaEventRecord(W.tev[9], stream_));
@@ -1046,17 +1077,19 @@ void Engine::retire_segments(Job& j, std::vector<PassEvent>* events) {
       CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
       stats_.accumulate_ms += ms;
     }
-    j.done += s.d.pass_spp;
-    free_seg(slot);
-    j.segs.pop_front();
-    stats_.passes++;
-    j.prog.pass++;
-    j.prog.spp_done = j.done;
-    j.prog.finished = j.done >= j.target;
-    j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
-    j.prog.rays = (last_counters_.rays - base_counters_.rays) + (last_counters_.shadow_rays - base_counters_.shadow_rays);
-    if (events) events->push_back(PassEvent{j.handle, j.prog});
-    if (j.on_pass) j.on_pass(j.prog);
+    for (int k = 0; k < passes.n; ++k) {
+      j.done += passes.seg[k].pass_spp;
+      free_seg(j.segs.front());
+      j.segs.pop_front();
+      stats_.passes++;
+      j.prog.pass++;
+      j.prog.spp_done = j.done;
+      j.prog.finished = j.done >= j.target;
+      j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
+      j.prog.rays = (last_counters_.rays - base_counters_.rays) + (last_counters_.shadow_rays - base_counters_.shadow_rays);
+      if (events) events->push_back(PassEvent{j.handle, j.prog});
+      if (j.on_pass) j.on_pass(j.prog);
+    }
   }
 }
 
@@ -1140,6 +1173,7 @@ void Engine::launch_one_iteration() {
 void Engine::drain(const volatile std::int32_t* cancel, std::vector<PassEvent>* events, double budget_ms,
                    bool return_on_event) {
   Wave& W = *wave_;
+  cancel_ = cancel;
   const auto t0 = std::chrono::steady_clock::now();
   const std::size_t events0 = events ? events->size() : 0;
   while (true) {

@@ -290,7 +290,7 @@ class Engine {
   std::uint32_t next_pass_size(const Job& j) const;
   bool issue_pass(Job& j);          // false if no radiance space or slot is free now
   void refill();
-  bool run_direct_pass(Job& j);     // false if no radiance space is free now
+  bool run_direct_passes(Job& j);   // false if no radiance space is free now
   void process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events);
   void retire_segments(Job& j, std::vector<PassEvent>* events);
   void launch_one_iteration();
@@ -361,6 +361,7 @@ class Engine {
   bool gen_dirty_ = false;
   WaveCounters last_counters_{};   // from the latest snapshot
   WaveCounters base_counters_{};   // at the start of the current render
+  const volatile std::int32_t* cancel_ = nullptr;  // of the render in progress
   bool counters_final_ = false;    // last_counters_ are the device's: nothing has run since
 };
 

@@ -116,3 +116,57 @@ def test_direct_trees_match_the_oracle(ctx, depth):
     err = np.abs(got - want).max(-1) / np.maximum(1.0, np.abs(want).max(-1))
     print(depth, "largest error", err.max(), "agree", (err <= 1e-3).mean())
     assert (err <= 1e-3).mean() >= 0.97
+
+
+@pytest.mark.parametrize("scene", ["mesh", "glass", "cornell"])
+def test_direct_kernels_agree(ctx, scene):
+    """A direct pass of 2^20 samples takes the per-warp kernel, smaller launches a thread a sample: the same render as
+    one pass of 512x512x4 and with its passes in callbacks' sight has to give the same bits. The callbacks see every
+    pass, in order, each with just its samples; a cancel in one drops the passes traced with it."""
+    make = SCENES.get(scene, workloads.mesh_stress)()
+    sid = ctx.load_json(json.dumps(make))
+    try:
+        s = ctx.scene_settings(sid)
+        s.width = s.height = 512
+        s.spp, s.max_depth, s.integrator, s.rr_min_depth = 4, 4, "direct", 3
+        ctx.render(sid, s, rtg.RenderOptions(progressive=False))
+        one = [x.tobytes() for x in ctx.framebuffer_moments(-1, 512, 512)]
+        s.width, s.height = 500, 520  # 260,000 pixels: passes of 1, 1 and 2 samples together are just under 2^20
+        seen = []
+
+        def on_pass(p):
+            n = ctx.framebuffer_moments(-1, 500, 520)[2]
+            assert (n == p.spp_done).all()
+            seen.append((p.pass_, p.spp_done))
+
+        ctx.render(sid, s, rtg.RenderOptions(progressive=True), on_pass)
+        assert seen == [(1, 1), (2, 2), (3, 4)]
+        small = [x.tobytes() for x in ctx.framebuffer_moments(-1, 500, 520)]
+        s.spp = 5  # with a fourth pass, over 2^20 samples
+        ctx.render(sid, s, rtg.RenderOptions(progressive=True))
+        assert (ctx.framebuffer_moments(-1, 500, 520)[2] == 5).all()
+        s.spp = 4
+        ctx.render(sid, s, rtg.RenderOptions(progressive=True))
+        assert [x.tobytes() for x in ctx.framebuffer_moments(-1, 500, 520)] == small
+        # 512x512 in passes of one sample: 2^18 samples each, four in a launch of 2^20 or alone.
+        s.width = s.height = 512
+        ctx.render(sid, s, rtg.RenderOptions(progressive=True, max_pass_spp=1))
+        assert [x.tobytes() for x in ctx.framebuffer_moments(-1, 512, 512)] == one
+        before = ctx.tuning()
+        ctx.set_tuning(max_pass_samples=512 * 512)  # room for one such pass
+        try:
+            ctx.render(sid, s, rtg.RenderOptions(progressive=True, max_pass_spp=1))
+        finally:
+            ctx.set_tuning(max_pass_samples=before["max_pass_samples"])
+        assert [x.tobytes() for x in ctx.framebuffer_moments(-1, 512, 512)] == one
+        import ctypes
+        cancel = ctypes.c_int32(0)
+
+        def stop(p):
+            cancel.value = 1
+
+        prog = ctx.render(sid, s, rtg.RenderOptions(progressive=True, max_pass_spp=1), stop, cancel)
+        assert prog.cancelled and prog.spp_done == 1
+        assert (ctx.framebuffer_moments(-1, 512, 512)[2] == 1).all()
+    finally:
+        ctx.release(sid)
