@@ -119,12 +119,14 @@ int rtg_compile(const char* scene_json, const char* base_dir, rtg_host_scene** o
 /* rtg_compile with flags. RTG_COMPILE_DEFER_BVH leaves the BVH out of the host
  * compile (Bvh::build, src/geometry/bvh.cpp:133-163, is skipped; the view below
  * then has no nodes): rtg_scene_upload builds the same tree at upload, on the GPU
- * for scenes of 32,768 primitives or more and on the host below that, where the
+ * for scenes of 1,024 primitives or more and on the host below that, where the
  * host is faster. */
 #define RTG_COMPILE_DEFER_BVH 1u
-/* RTG_COMPILE_AUTO_BVH: the compile builds the tree itself for scenes under 32,768
+/* RTG_COMPILE_AUTO_BVH: the compile builds the tree itself for scenes under 1,024
  * primitives and defers it to the GPU build for larger ones, so the host work stays
- * on the compiling thread (not on the thread that uploads). */
+ * on the compiling thread (not on the thread that uploads). The view and the host
+ * layout of a deferred scene under 32,768 primitives still have the tree: it is
+ * built on the host when one of them is first asked for. */
 #define RTG_COMPILE_AUTO_BVH 2u
 int rtg_compile_flags(const char* scene_json, const char* base_dir, uint32_t flags, rtg_host_scene** out, char* err,
                       size_t err_cap);
@@ -174,7 +176,7 @@ int rtg_device_count(void);
  *      src/io/scene_io.cpp:480-502) ---- */
 
 /* Parse, validate, compile and upload. The BVH is built on the host for scenes under
- * 32,768 primitives and on the GPU for larger ones (RTG_COMPILE_AUTO_BVH): the same
+ * 1,024 primitives and on the GPU for larger ones (RTG_COMPILE_AUTO_BVH): the same
  * tree either way. base_dir resolves relative OBJ paths (may be NULL). */
 int rtg_scene_load_json(rtg_context* ctx, const char* scene_json, const char* base_dir, rtg_scene_id* out);
 int rtg_scene_load_file(rtg_context* ctx, const char* path, rtg_scene_id* out);

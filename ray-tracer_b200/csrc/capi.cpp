@@ -213,7 +213,8 @@ void build_view_arrays(const rtg_host_scene& hs) {
     const double r[8] = {pl.point.x, pl.point.y, pl.point.z, pl.normal.x, pl.normal.y, pl.normal.z, double(pl.material), 0};
     hs.planes.insert(hs.planes.end(), r, r + 8);
   }
-  for (const rtg::BinaryNode& n : s.bvh.nodes) {
+  const rtg::BinaryBvh* tree = rtg::host_tree(s);
+  for (const rtg::BinaryNode& n : tree ? tree->nodes : s.bvh.nodes) {
     const double r[10] = {n.box.lo.x, n.box.lo.y, n.box.lo.z, n.box.hi.x, n.box.hi.y, n.box.hi.z,
                           double(n.first), double(n.count), double(n.axis), 0};
     hs.nodes.insert(hs.nodes.end(), r, r + 10);
@@ -292,8 +293,15 @@ void rtg_host_scene_free(rtg_host_scene* scene) { delete scene; }
 int64_t rtg_host_scene_layout(const rtg_host_scene* hs, int32_t part, void* out, uint64_t cap) {
   if (!hs) return RTG_ERR_INVALID;
   try {
-    if (!hs->scene->bvh_built) return RTG_ERR_INVALID;
-    const rtg::FlatScene f = rtg::flatten(*hs->scene, true);
+    const rtg::BinaryBvh* tree = rtg::host_tree(*hs->scene);
+    if (!tree) return RTG_ERR_INVALID;
+    rtg::CompiledScene with_tree;
+    if (!hs->scene->bvh_built) {
+      with_tree = *hs->scene;
+      with_tree.bvh = *tree;
+      with_tree.bvh_built = true;
+    }
+    const rtg::FlatScene f = rtg::flatten(hs->scene->bvh_built ? *hs->scene : with_tree, true);
     const std::int32_t roots[5] = {f.root, f.root4, static_cast<std::int32_t>(f.slot_prim.size()), 0, f.root8};
     const void* src = nullptr;
     std::size_t bytes = 0;
@@ -325,15 +333,17 @@ int rtg_host_scene_view(const rtg_host_scene* hs, rtg_scene_view* out) {
   *out = rtg_scene_view{};
   out->n_prims = s.prims.size();
   out->n_planes = s.planes.size();
-  out->n_nodes = s.bvh.nodes.size();
-  out->n_order = s.bvh.order.size();
+  const rtg::BinaryBvh* late = rtg::host_tree(s);
+  const rtg::BinaryBvh& tree = late ? *late : s.bvh;
+  out->n_nodes = tree.nodes.size();
+  out->n_order = tree.order.size();
   out->n_lights = s.lights.size();
   out->n_point_lights = s.point_lights.size();
   out->n_materials = s.materials.size();
   out->prims = hs->prims.data();
   out->planes = hs->planes.data();
   out->nodes = hs->nodes.data();
-  out->order = s.bvh.order.data();
+  out->order = tree.order.data();
   out->lights = hs->lights.data();
   out->point_lights = hs->point_lights.data();
   out->materials = hs->materials.data();
@@ -351,10 +361,11 @@ int rtg_host_scene_view(const rtg_host_scene* hs, rtg_scene_view* out) {
   std::memcpy(out->background, bg, sizeof bg);
   out->settings = to_c(s.settings);
   out->degenerate_skipped = s.info.degenerate_skipped;
-  out->bvh_max_depth = s.info.bvh.max_depth;
-  out->bvh_leaves = s.info.bvh.leaves;
-  out->bvh_max_leaf = s.info.bvh.max_leaf;
-  out->bvh_sah_cost = s.info.bvh.sah_cost;
+  const rtg::BvhStats& stats = s.bvh_built ? s.info.bvh : tree.stats;
+  out->bvh_max_depth = stats.max_depth;
+  out->bvh_leaves = stats.leaves;
+  out->bvh_max_leaf = stats.max_leaf;
+  out->bvh_sah_cost = stats.sah_cost;
   return RTG_OK;
 }
 
@@ -514,6 +525,8 @@ int rtg_scene_get_info(rtg_context* ctx, rtg_scene_id scene, rtg_scene_info* out
     out->device_bytes = g.device_bytes;
     out->bvh_build_ms = b.build_ms;
     out->bvh_sah_cost = b.sah_cost;
+    if (g.host_stats)  // the GPU build does not add the cost up; it has the host tree's
+      if (const rtg::BinaryBvh* tree = rtg::host_tree(*g.host, true)) out->bvh_sah_cost = tree->stats.sah_cost;
     return RTG_OK;
   });
 }

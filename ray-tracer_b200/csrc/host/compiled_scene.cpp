@@ -82,6 +82,15 @@ void parallel_for(std::size_t n, F&& body, std::size_t grain = 1024) {
 
 }  // namespace
 
+namespace {
+void build_tree(const CompiledScene& s, BinaryBvh& bvh) {
+  std::vector<Box> boxes;
+  boxes.reserve(s.prims.size());
+  for (const Prim& p : s.prims) boxes.push_back(p.bounds());
+  bvh.build(boxes, 4);
+}
+}  // namespace
+
 CompiledScene compile_scene(const SceneDesc& desc, BvhBuild where) {
   CompiledScene s;
   s.settings = desc.render;
@@ -223,14 +232,22 @@ CompiledScene compile_scene(const SceneDesc& desc, BvhBuild where) {
 
   if (where == BvhBuild::Defer || (where == BvhBuild::Auto && s.prims.size() >= kGpuBuildMinPrims)) {
     s.bvh_built = false;
+    if (s.prims.size() < kHostTreePrims) {
+      s.late = std::make_shared<CompiledScene::LateTree>();
+      s.late->automatic = where == BvhBuild::Auto;
+    }
     return s;
   }
-  std::vector<Box> boxes;
-  boxes.reserve(s.prims.size());
-  for (const Prim& p : s.prims) boxes.push_back(p.bounds());
-  s.bvh.build(boxes, 4);
+  build_tree(s, s.bvh);
   s.info.bvh = s.bvh.stats;
   return s;
+}
+
+const BinaryBvh* host_tree(const CompiledScene& s, bool deferred) {
+  if (s.bvh_built) return &s.bvh;
+  if (!s.late || !(s.late->automatic || deferred)) return nullptr;
+  std::call_once(s.late->once, [&s] { build_tree(s, s.late->bvh); });
+  return &s.late->bvh;
 }
 
 }  // namespace rtg

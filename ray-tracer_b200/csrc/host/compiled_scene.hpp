@@ -9,6 +9,8 @@
 // reference's hit ids. The device copy is produced from this by flatten.hpp.
 #include <cstdint>
 #include <string>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "host/bvh_build.hpp"
@@ -65,17 +67,33 @@ struct CompiledScene {
   std::vector<LightEntry> lights;
   BinaryBvh bvh;
   bool bvh_built = true;  // false: compiled without the BVH (built on the GPU at upload)
+  struct LateTree {
+    std::once_flag once;
+    BinaryBvh bvh;
+    bool automatic = false;  // left to the GPU by Auto (else by Defer)
+  };
+  std::shared_ptr<LateTree> late;  // of scenes without `bvh` under kHostTreePrims primitives
   BuildInfo info;
 };
 
-// Scenes from this many primitives up build their BVH faster on the GPU than on
-// the host (latency of the GPU build's level passes against the host build's work).
-constexpr std::size_t kGpuBuildMinPrims = 32768;
+// Scenes from this many primitives up build their BVH faster on the GPU: its level
+// passes cost some 1.1 ms however few primitives they have (2.7 ms for 25k, 6.4 ms for
+// 174k, upload included), the host 1.2 to 1.6 us a primitive below 34k (2.5 ms for 2,053,
+// 38 ms for 25k), where it runs on one thread.
+constexpr std::size_t kGpuBuildMinPrims = 1024;
+// Scenes of fewer primitives than this that the rule above sends to the GPU still have
+// their tree where a caller asks for it on the host (host_tree).
+constexpr std::size_t kHostTreePrims = 32768;
 
 // Where the BVH is built: in the compile (Host); at upload, on the GPU from
 // kGpuBuildMinPrims primitives up and on the host below (Defer: `bvh` stays empty
 // here); or chosen by size here (Auto: small scenes built now, large ones deferred).
 enum class BvhBuild { Host, Defer, Auto };
 CompiledScene compile_scene(const SceneDesc& desc, BvhBuild where = BvhBuild::Host);
+
+// The scene's host tree: the compile's, or for a scene of under kHostTreePrims
+// primitives whose compile left it to the GPU, one built on the first call. Null for
+// larger deferred scenes, and for scenes compiled with Defer unless `deferred`.
+const BinaryBvh* host_tree(const CompiledScene& s, bool deferred = false);
 
 }  // namespace rtg

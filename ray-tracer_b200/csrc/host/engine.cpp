@@ -218,14 +218,15 @@ void Engine::reset_wave() {
 
 int Engine::add_scene(std::shared_ptr<const CompiledScene> scene) {
   if (!scene->bvh_built) {
-    if (scene->prims.size() >= kGpuBuildMinPrims) return add_scene_gpu_bvh(std::move(scene));
+    if (scene->prims.size() >= kGpuBuildMinPrims) {
+      const int id = add_scene_gpu_bvh(std::move(scene));
+      scenes_.at(id)->host_stats = true;
+      return id;
+    }
     // Small scene: the host builds the same tree faster than the GPU build's
     // level-by-level passes can start and finish.
     auto built = std::make_shared<CompiledScene>(*scene);
-    std::vector<Box> boxes;
-    boxes.reserve(built->prims.size());
-    for (const Prim& p : built->prims) boxes.push_back(p.bounds());
-    built->bvh.build(boxes, 4);
+    if (const BinaryBvh* tree = host_tree(*scene, true)) built->bvh = *tree;
     built->info.bvh = built->bvh.stats;
     built->bvh_built = true;
     FlatScene flat = flatten(*built, wants_wide8());

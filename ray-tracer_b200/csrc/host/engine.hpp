@@ -92,6 +92,7 @@ struct GpuScene {
   int jobs_open = 0;           // jobs in the wavefront that use this scene
   BvhStats bvh;                // of the tree on the device (host or device build)
   bool device_built = false;   // the BVH was built on the GPU
+  bool host_stats = false;     // ... because the scene is large enough, not by request
 };
 
 // Per-job device framebuffer.

@@ -355,7 +355,7 @@ def parse_scene(scene_json: str, base_dir: Optional[str] = None, defer_bvh=False
     """Parse + validate + compile a scene (raises SceneError with the field path).
 
     defer_bvh=True skips the host BVH build: uploading the scene builds it (on the
-    GPU from 32,768 primitives up). defer_bvh="auto" builds small scenes' trees here
+    GPU from 1,024 primitives up). defer_bvh="auto" builds small scenes' trees here
     and defers only large ones."""
     h = C.c_void_p()
     err = C.create_string_buffer(1024)

@@ -11,7 +11,7 @@ Cold previews (optional) are previews of scenes that are not resident: the scene
 JSON arrives with the request, a worker thread compiles it, the serving thread
 uploads it (with the BVH built on the GPU, or flattened from a host-built tree)
 and submits it; the scene is released when its request finishes. Their TTFP
-includes the compile and the upload. With the GPU build, scenes under 32,768
+includes the compile and the upload. With the GPU build, scenes under 1,024
 primitives still get their tree on the worker (the host is faster there).
 """
 import collections
