@@ -304,8 +304,8 @@ int rtg_probe_read_bandwidth(rtg_context* ctx, uint64_t bytes, int32_t reps, int
 
 /* ---- engine tuning (no reference counterpart) ---- */
 typedef struct rtg_tuning {
-  uint32_t pool_paths;       /* paths of one wavefront iteration while requests are open; a render's
-                              * iterations take four times as many (default 1 << 20) */
+  uint32_t pool_paths;       /* a render's wavefront iterations trace up to four times as many paths, with
+                              * requests open half as many, or the whole pool up to 2^20 (default 1 << 20) */
   uint32_t block;            /* threads per block of the path kernel: 64, 128, 256 */
   uint64_t max_pass_samples; /* radiance slots shared by all passes in flight (default 1 << 27) */
   int32_t extend_blocks; /* grid of the path kernel; 0 = every resident block */

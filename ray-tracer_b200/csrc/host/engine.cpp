@@ -75,10 +75,16 @@ constexpr int kLag = 2;    // iterations queued ahead of the snapshot being read
 constexpr std::size_t kStageBytes = std::size_t(1) << 20;  // host->device staging per iteration
 constexpr std::size_t kStagePiece = std::size_t(1) << 20;  // batch upload: bytes per host copy task
 constexpr int kJobSlots = 4096;  // job descriptors resident at once
-// Paths of one iteration, in pools: renders take several, since every iteration
+// Paths of one iteration. A render's iterations take four pools, since every iteration
 // ends with a wait for its slowest warps (0.03 ms on the sphere field, 0.1 ms on the
-// mix, 0.2 ms on the mesh); requests take one, so a preview waits less for its turn.
-constexpr std::uint32_t kRenderItems = 4;
+// mix, 0.2 ms on the mesh). While requests are open they take half a pool (or a pool of
+// up to 2^20, whose iterations are short), so that a preview waits less for its turn: with 8,388,608 paths, half a pool serves 3573
+// Msamples/s with previews at 7.7 ms (median) and 15 ms (p99), a whole one 3687 at 13 and
+// 22.5 ms, a third 3446 at 6.2 and 13 ms.
+constexpr std::uint32_t kRenderPools = 4;
+std::uint32_t iteration_paths(std::uint32_t pool, bool serving) {
+  return serving ? std::min(pool, std::max(1u << 20, pool / 2)) : pool * kRenderPools;
+}
 constexpr std::uint64_t kDirectSamples = std::uint64_t(1) << 22;  // of the passes the direct integrator traces together
 
 }  // namespace
@@ -103,6 +109,11 @@ struct Engine::Wave {
   std::map<std::uint64_t, std::uint64_t> rad_free;  // free radiance ranges: begin -> length
   std::vector<int> free_jobs;          // descriptor slots, popped from the back
   std::vector<int> free_segs;
+  // Upper bounds, after the iterations launched so far: samples of issued passes not
+  // yet generated, and paths left over. Both zero: the launched iterations finish
+  // everything, and another one would find nothing to do.
+  std::uint64_t ungenerated = 0, left = 0;
+  bool all_listed = true;              // the generation table holds every open segment
   std::uint32_t snapshot_slots = 0;
   std::uint32_t hi_slot = 0;           // segment slots ever used are below this
   int sms = 0;
@@ -668,9 +679,9 @@ void Engine::ensure_wave() {
   Wave& W = *wave_;
   WaveBuffers& b = W.wb;
   const std::uint32_t P = cfg_.pool_paths;
-  b.capacity = P * kRenderItems;
+  b.capacity = P * kRenderPools;
   CK(cudaDeviceGetAttribute(&W.sms, cudaDevAttrMultiProcessorCount, device_));
-  const std::uint32_t left = std::min<std::uint32_t>(P * kRenderItems, static_cast<std::uint32_t>(W.sms) * kMaxPathsPerSm);
+  const std::uint32_t left = std::min<std::uint32_t>(P * kRenderPools, static_cast<std::uint32_t>(W.sms) * kMaxPathsPerSm);
   for (int i = 0; i < 2; ++i) {
     b.st_a[i] = dev_alloc<float4>(left);
     b.st_b[i] = dev_alloc<float4>(left);
@@ -822,6 +833,7 @@ void Engine::write_gen_table() {
   }
   g.snapshot_slots = hi;
   W.snapshot_slots = hi;
+  W.all_listed = open.size() <= static_cast<std::size_t>(kMaxGen);
   stage(W.gen_dev, &g, offsetof(GenTable, slot) + sizeof(std::uint32_t) * std::max<std::uint32_t>(g.n, 1));
   gen_dirty_ = false;
 }
@@ -910,6 +922,7 @@ bool Engine::issue_pass(Job& j) {
   const SegmentProgress zero{};
   stage(W.segs_dev + slot, &s.d, sizeof(s.d));
   stage(W.prog_dev + slot, &zero, sizeof(zero));
+  W.ungenerated += count;
   j.issued += k;
   j.passes_issued++;
   j.segs.push_back(slot);
@@ -1008,7 +1021,7 @@ void Engine::refill() {
     if (!s.used || s.complete || s.abandoned) continue;
     backlog[jobs_.at(s.job).priority] += s.d.count - std::min<std::uint64_t>(s.done, s.d.count);
   }
-  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderItems);
+  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderPools);
   while (true) {
     Job* best = nullptr;
     for (auto& kv : jobs_) {
@@ -1137,26 +1150,36 @@ void Engine::process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events
   for (auto& kv : jobs_) retire_segments(kv.second, events);
 }
 
-void Engine::launch_one_iteration() {
+void Engine::launch_one_iteration(bool look) {
   Wave& W = *wave_;
   counters_final_ = false;
   if (gen_dirty_) write_gen_table();
   const int par = static_cast<int>(W.it & 1);
   const int r = static_cast<int>(W.it % kRing);
   const bool timed = cfg_.time_kernels;
-  W.wb.capacity = cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderItems);
+  W.wb.capacity = iteration_paths(cfg_.pool_paths, serve_open_ > 0);
   LaunchShape shape = cfg_.shape;
   shape.mis = mis_jobs_ > 0;
   shape.general = cfg_.count_traversal || brute_jobs_ > 0 || shape.closest_tree == 8 || shape.shadow_tree == 8;
   if (timed) CK(cudaEventRecord(W.tev[0], stream_));
   CK(launch_plan(W.wb, par, shape, stream_));
   if (timed) CK(cudaEventRecord(W.tev[1], stream_));
+  // The plan's snapshot and this slot's staged copies are complete once the event
+  // fires. It comes after the whole iteration, so that none sits between chained
+  // kernels, unless the iteration is launched for its snapshot.
+  if (look) CK(cudaEventRecord(W.plan_ev[r], stream_));
   CK(launch_paths(W.wb, par, shape, stream_));
-  // After the whole iteration, so no event sits between chained kernels; the
-  // plan's snapshot and this slot's staged copies are complete once it fires.
   if (timed) CK(cudaEventRecord(W.tev[2], stream_));
-  CK(cudaEventRecord(W.plan_ev[r], stream_));
+  if (!look) CK(cudaEventRecord(W.plan_ev[r], stream_));
   W.plan_recorded[r] = true;
+  if (W.all_listed) {
+    // The plan gives every free place away while samples are open; with some to spare
+    // it runs the paths to their end.
+    const std::uint64_t room = W.wb.capacity > W.left ? W.wb.capacity - W.left : 0;
+    const bool finishes = W.ungenerated < room;
+    W.ungenerated -= std::min(W.ungenerated, room);
+    W.left = finishes ? 0 : std::min<std::uint64_t>(W.wb.capacity, std::uint64_t(W.sms) * kMaxPathsPerSm);
+  }
   if (timed) {
     CK(cudaEventSynchronize(W.tev[2]));
     float plan_ms = 0, path_ms = 0;
@@ -1180,9 +1203,16 @@ void Engine::drain(const volatile std::int32_t* cancel, std::vector<PassEvent>* 
   while (true) {
     if (cancel && *cancel) return;
     refill();
-    if (all_jobs_drained()) return;
-    launch_one_iteration();
-    while (W.seen + kLag < W.it) process_snapshot(W.seen++, events);
+    if (all_jobs_drained()) {
+      W.ungenerated = W.left = 0;
+      return;
+    }
+    launch_one_iteration(false);
+    // Nothing to run ahead of: look at once instead of two empty iterations later.
+    const bool idle_next = W.ungenerated == 0 && W.left == 0;
+    if (idle_next) launch_one_iteration(true);
+    const std::uint64_t lag = idle_next ? 0 : kLag;
+    while (W.seen + lag < W.it) process_snapshot(W.seen++, events);
     if (return_on_event && events && events->size() > events0) return;
     if (budget_ms < std::numeric_limits<double>::infinity() &&
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count() >= budget_ms)
@@ -1210,6 +1240,7 @@ void Engine::abort_all() {
   W.seen = W.it;
   W.stall = 0;
   W.last_done_sum = 0;
+  W.ungenerated = W.left = 0;
   gen_dirty_ = true;
   write_gen_table();
 }
