@@ -215,6 +215,10 @@ __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
 //   four-wide walk for shadow rays), warps in different steps evict each other's
 //   loops: 2.1 of 9.5 cycles per instruction went to fetching, now 0.4.
 constexpr int kWarpPaths = 56;
+// Least paths a warp takes at once where there are too few for full batches: 4 and 8
+// measure alike, 16 loses half of the gain (mesh 64x64x1: 465 us with full batches only,
+// 408 with 16, 313 with 8, 331 with 4; 32x32x1: 465, 355, 319, 260).
+constexpr std::uint32_t kMinBatch = 4;
 
 constexpr std::uint32_t kPathSpecular = 1u << 12;   // last bounce was specular (or the path is new)
 constexpr std::uint32_t kPathContinues = 1u << 13;  // goes on after its shadow ray
@@ -319,6 +323,10 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
   WaveCounters* const C = wb.cnt;
   const std::uint32_t live = C->live[par], n = C->n_items;
   const bool finish = C->finish != 0;
+  // New items come 32 at a time, or fewer when that gives every warp some: with few
+  // paths the time is a warp's chain of steps, and a step is as long as its longest ray.
+  const std::uint32_t warps = gridDim.x * (blockDim.x / 32);
+  const int batch = static_cast<int>(min(32u, max(kMinBatch, (n + warps - 1) / warps)));
   const unsigned below = (1u << lane) - 1u;
   Walk<kGeneral> walk;
   TraceCount tc, sh_tc;
@@ -373,7 +381,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
         job = S.job[p];
       }
     } else {
-      int take = min(n_idle, 32);
+      int take = min(n_idle, batch);
       std::uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&C->fetch, static_cast<std::uint32_t>(take));
       base = __shfl_sync(kFull, base, 0);
