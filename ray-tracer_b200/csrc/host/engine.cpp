@@ -1526,21 +1526,25 @@ void Engine::read_mean_frame(const GpuFrame& f, double* rgb) {
 
 void Engine::read_image_list(const std::vector<ImageRead>& list) {
   CK(cudaSetDevice(device_));
-  // A slot takes parts of several small images, or a part of a large one.
+  // A slot takes parts of several small images, or a part of a large one: at most
+  // kPixels pixels, so that the copies of a single image overlap its resolves
+  // (1024x1024: 157 us, against 369 us in one piece).
+  constexpr std::size_t kPixels = std::size_t(1) << 18;
   struct Part {
     const ImageRead* image;
     std::size_t first, pixels, at;  // pixel range, and its place in the slot
   };
   std::vector<std::vector<Part>> loads;
-  std::size_t used = kSlotBytes;
+  static_assert(2 * kPixels * 3 + 256 <= kSlotBytes, "a piece fits its slot");
+  std::size_t used = 0;
   for (const ImageRead& r : list) {
     const std::size_t px = std::size_t(r.frame->width) * r.frame->height;
     for (std::size_t first = 0; first < px;) {
-      if (kSlotBytes - used < 4096 || loads.empty()) {
+      if (loads.empty() || used >= 3 * kPixels) {
         loads.emplace_back();
         used = 0;
       }
-      const std::size_t n = std::min(px - first, (kSlotBytes - used) / 3 & ~std::size_t(255));
+      const std::size_t n = std::min(px - first, kPixels);
       loads.back().push_back({&r, first, n, used});
       used += (3 * n + 255) & ~std::size_t(255);
       first += n;

@@ -52,8 +52,8 @@ class HostPool {
 
   // memcpy, split over the threads when it is worth waking them.
   void copy(void* dst, const void* src, std::size_t bytes) {
-    constexpr std::size_t kPiece = std::size_t(1) << 18;
-    if (bytes < 4 * kPiece) {
+    constexpr std::size_t kPiece = std::size_t(1) << 17;
+    if (bytes < 2 * kPiece) {
       std::memcpy(dst, src, bytes);
       return;
     }
