@@ -21,7 +21,7 @@ bench.py starts torchrun itself.
 Cornell box (256^2 x 64 spp, depth 8), the sphere field (512^2 x 128, depth 16)
 and the 174k-triangle mesh (1024^2 x 64, depth 12): GPU Msamples/s on device
 time and end to end, Mrays/s (closest-hit + shadow rays), the roofline of the
-closest-hit kernel, and the reference's own CPU renderer on the same scene file:
+path kernel, and the reference's own CPU renderer on the same scene file:
 its stock command-line renderer (`rt --threads 0 --single-pass`) for the two
 scenes its JSON schema expresses, its Renderer::render through oracle/_ref's
 harness for the mesh (whose 256x180 torus needs a schema extension).
@@ -415,10 +415,71 @@ def ncu_profile(kernel: str, pool_paths: int, tree: int = 2):
     return None
 
 
+def path_profile():
+    """Per-ray counters of the path kernel from the committed ncu capture of the mix, or None."""
+    path = os.path.join(ROOT, "profiles", "k_path_mix_counters.json")
+    if not os.path.exists(path):
+        return None
+    return dict(json.load(open(path)), file=os.path.basename(path))
+
+
+def path_roofline(ctx, step, peaks, profile=True):
+    """Roofline figures of the path kernel (k_path), which does all of a path's work,
+    for one step of a workload: one run with per-kernel CUDA events, one with
+    traversal counters. Its time cannot be lower than any of
+      HBM:   16 B of radiance written per camera path / HBM peak (path state stays
+             on the SM);
+      L1:    the walks' fetches (64 B per node visit, 48 B per primitive test,
+             closest-hit and shadow rays) / aggregate L1 read peak;
+      L2:    the L2 bytes per ray of the committed capture / L2 peak;
+      issue: the warp instructions per ray of that capture / the SM's peak issue
+             rate (4 schedulers per SM, one instruction per clock each, at the SM
+             clock sampled during the timed steps).
+    The last two need `profile`: the capture is of the mix, so they hold for it
+    alone. The level with the largest frac (its bound on the time / the measured
+    time) is the `bound`."""
+    ctx.set_tuning(time_kernels=1, count_traversal=0)
+    t_st = step()
+    ctx.set_tuning(time_kernels=0, count_traversal=1)
+    c_st = step()
+    ctx.set_tuning(time_kernels=0, count_traversal=0)
+    launches = max(1, t_st["extend_launches"])
+    secs = t_st["extend_ms"] / 1e3
+    rays = c_st["rays"] + c_st["shadow_rays"]
+    nodes = c_st["node_visits"] + c_st["shadow_node_visits"]
+    prims = c_st["prim_tests"] + c_st["shadow_prim_tests"]
+    amounts = {"hbm": (c_st["camera_samples"] * 16, peaks["hbm"], "GB/s"),
+               "l1": (nodes * NODE_BYTES[2] + prims * PRIM_BYTES, peaks["l1"], "GB/s")}
+    prof = path_profile() if profile else None
+    if prof:
+        amounts["l2"] = (prof["l2_bytes_per_ray"] * rays, peaks["l2"], "GB/s")
+        if peaks.get("sms") and peaks.get("sm_mhz"):
+            amounts["issue"] = (prof["warp_inst_per_ray"] * rays, 4 * peaks["sms"] * peaks["sm_mhz"] / 1e3,
+                                "G warp instructions/s")
+    levels = {k: {"achieved": n / secs / 1e9, "peak": peak, "unit": unit, "frac": n / secs / 1e9 / peak}
+              for k, (n, peak, unit) in amounts.items()}
+    bound = max(levels, key=lambda k: levels[k]["frac"])
+    traffic = prof["dram_bytes_per_ray"] * rays / launches if prof else None
+    kernel_ms = {k: t_st[k] for k in ("extend_ms", "accumulate_ms", "plan_ms")}
+    out = {"kernel": "k_path (camera paths, closest-hit and shadow rays, shading)", "bound": bound, **levels[bound],
+           "traffic": traffic, "levels": levels,
+           "dram_frac": traffic * launches / secs / 1e9 / peaks["hbm"] if traffic else None,
+           "avg_launch_ms": secs / launches * 1e3, "launches": launches, "rays_per_launch": rays / launches,
+           "share_of_kernel_time": t_st["extend_ms"] / sum(kernel_ms.values()),
+           "per_ray": {"nodes": nodes / max(1, rays), "prim_tests": prims / max(1, rays), "node_bytes": NODE_BYTES[2]}}
+    if prof:
+        out["ncu"] = {k: prof[k] for k in ("lanes_active", "issue_active", "l1_hit_rate", "l2_hit_rate",
+                                           "warp_inst_per_ray", "thread_inst_per_ray", "file")}
+        # Useful share of the issue slots: lanes doing work in each issued instruction.
+        out["lane_efficiency"] = prof["thread_inst_per_ray"] / (32 * prof["warp_inst_per_ray"])
+    return out, kernel_ms, c_st
+
+
 def rooflines(ctx, step, peaks, profile=True):
-    """Roofline figures of the closest-hit kernel (k_extend) and the shade kernel
-    (k_shade) for one step of a workload: one run with per-kernel CUDA events,
-    one with traversal counters.
+    """Roofline figures of a wavefront that has a kernel for each stage (k_extend,
+    k_shade), from its statistics: one run with per-kernel CUDA events, one with
+    traversal counters. The library traced paths that way before the path kernel;
+    path_roofline() is for the path kernel.
 
     k_extend is bounded at three levels; its time cannot be lower than any of
       HBM: the queue traffic that cannot stay on chip (32 B ray read per
@@ -532,7 +593,7 @@ def render_config(ctx, name, a, peaks):
     steps = max(3, a.steps)
     t = timed_steps(_NoDist, None, step, steps)
     value = t["samples"] / (t["t_max_ms"] / 1e3) / 1e6
-    ext, shade, kernel_ms, c_st = rooflines(ctx, step, peaks, profile=False)
+    roof, kernel_ms, c_st = path_roofline(ctx, step, peaks, profile=False)
     h2d = ctx.scene_info(sid)["device_bytes"]
     ctx.release(sid)
     # End to end: upload, render, tone-mapped image read-back, release.
@@ -551,7 +612,7 @@ def render_config(ctx, name, a, peaks):
             "ms_per_render": t["t_max_ms"] / steps, "mrays_per_s": t["rays"] / (t["t_max_ms"] / 1e3) / 1e6,
             "e2e": {"value": e2e, "unit": "Msamples/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": st.width * st.height * 3},
-            "roofline": ext, "shade_roofline": shade, "kernel_ms": kernel_ms,
+            "roofline": roof, "kernel_ms": kernel_ms,
             "invalid_samples": c_st["invalid_samples"]}
 
 
@@ -684,7 +745,7 @@ def run_rtg(a, dist, scenes, desc):
 
     peaks["sm_mhz"] = t["clocks"].get("sm_mhz") or t["clocks"].get("sm_max_mhz")
     peaks["sms"] = sm_count(dev)
-    ext, shade, kernel_ms, c_st = rooflines(ctx, step, peaks)
+    roof, kernel_ms, c_st = path_roofline(ctx, step, peaks)
 
     # Serving: Poisson arrivals of previews and finals over 32 resident scenes.
     serve = None
@@ -767,19 +828,18 @@ def run_rtg(a, dist, scenes, desc):
                            "target_2x_plain": "not met" if plain and plain["batched_over_plain"] < 2 else None,
                            "preview_p99_ms": serve["preview"]["ttfp_ms_p99"] if serve else None,
                            "cpu": cpu["value"] if cpu else None},
-                   "k_extend": {"bound": ext["bound"], "frac": ext["frac"], "dram_frac": ext["dram_frac"],
-                                "levels": {k: v["frac"] for k, v in ext["levels"].items()},
-                                **({"lanes_active": ext["ncu"].get("lanes_active"),
-                                    "issue_active": ext["ncu"].get("issue_active"),
-                                    "lane_efficiency": ext.get("lane_efficiency")} if "ncu" in ext else {})},
-                   "k_shade_hbm_frac": shade["frac"]}
+                   "k_path": {"bound": roof["bound"], "frac": roof["frac"], "dram_frac": roof["dram_frac"],
+                              "levels": {k: v["frac"] for k, v in roof["levels"].items()},
+                              **({"lanes_active": roof["ncu"]["lanes_active"],
+                                  "issue_active": roof["ncu"]["issue_active"],
+                                  "lane_efficiency": roof["lane_efficiency"]} if "ncu" in roof else {})}}
         if per_config:
             for tag, e in per_config.items():
                 summary[tag] = {"value": e["value"], "e2e": e["e2e"]["value"], "mrays_per_s": e["mrays_per_s"],
                                 "cpu": e.get("cpu_baseline", {}).get("value"),
                                 "cpu_cores": e.get("cpu_baseline", {}).get("cores"),
-                                "over_cpu": e.get("over_cpu"), "extend_bound": e["roofline"]["bound"],
-                                "extend_frac": e["roofline"]["frac"]}
+                                "over_cpu": e.get("over_cpu"), "path_bound": e["roofline"]["bound"],
+                                "path_frac": e["roofline"]["frac"]}
         tun = ctx.tuning()
         line = {
             "metric": METRIC, "value": value, "unit": "Msamples/s", "n_gpus": dist.world, "steps": a.steps,
@@ -801,8 +861,7 @@ def run_rtg(a, dist, scenes, desc):
                     "d2h_bytes_per_step": d2h, "phases_per_step": phase},
             "gpu_launches": t["launches"],
             "clocks": t["clocks"],
-            "roofline": ext,
-            "shade_roofline": shade,
+            "roofline": roof,
             "kernel_ms": kernel_ms,
             "peaks": peaks,
             "cpu_baseline": cpu,

@@ -19,6 +19,8 @@
 // pixel's samples into the double framebuffer in sample order (Framebuffer::add,
 // include/raytracer/rendering/framebuffer.hpp:31), passes of one render in order.
 #include <cfloat>
+#include <map>
+#include <mutex>
 
 #include "device/shade.cuh"
 #include "device/wave.h"
@@ -1158,24 +1160,41 @@ struct Grid {
   cudaError_t err = cudaSuccess;
   int sms = 0, per_sm = 0;
 };
-template <class K>
-Grid resident_grid(K kernel, int block, std::size_t smem, int cap) {
-  Grid g;
-  int dev = 0;
-  g.err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (g.err == cudaSuccess) g.err = cudaGetDevice(&dev);
-  if (g.err == cudaSuccess) g.err = cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, dev);
-  if (g.err == cudaSuccess) g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g.per_sm, kernel, block, smem);
-  g.per_sm = g.per_sm < 1 ? 1 : (g.per_sm > cap ? cap : g.per_sm);
-  return g;
-}
+
+// A kernel's grids by device: the shared-memory limit is set on each device that the
+// kernel runs on, and contexts of several devices launch from several threads. What
+// fails is asked again at the next launch.
+class GridTable {
+ public:
+  template <class K>
+  Grid get(K kernel, int block, std::size_t smem, int cap) {
+    Grid g;
+    int dev = 0;
+    g.err = cudaGetDevice(&dev);
+    if (g.err != cudaSuccess) return g;
+    std::lock_guard<std::mutex> hold(lock_);
+    const auto known = by_device_.find(dev);
+    if (known != by_device_.end()) return known->second;
+    g.err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (g.err == cudaSuccess) g.err = cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (g.err == cudaSuccess) g.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g.per_sm, kernel, block, smem);
+    if (g.err != cudaSuccess) return g;
+    g.per_sm = g.per_sm < 1 ? 1 : (g.per_sm > cap ? cap : g.per_sm);
+    return by_device_.emplace(dev, g).first->second;
+  }
+
+ private:
+  std::mutex lock_;
+  std::map<int, Grid> by_device_;
+};
 
 // At most kMaxPathsPerSm path slots per SM, whatever extend_blocks asks for.
 template <int kBlock, bool kMis, bool kGeneral>
 cudaError_t launch_path(const WaveBuffers& wb, int par, const LaunchShape& shape, cudaStream_t stream) {
   constexpr std::size_t smem = kBlock / 32 * kWarpSmem<kMis, kGeneral>;
   constexpr int kMaxBlocksPerSm = kMaxPathsPerSm / kWarpPaths / (kBlock / 32);
-  static const Grid grid = resident_grid(k_path<kBlock, kMis, kGeneral>, kBlock, smem, kMaxBlocksPerSm);
+  static GridTable grids;
+  const Grid grid = grids.get(k_path<kBlock, kMis, kGeneral>, kBlock, smem, kMaxBlocksPerSm);
   if (grid.err != cudaSuccess) return grid.err;
   int blocks = shape.extend_blocks > 0 ? shape.extend_blocks : grid.sms * grid.per_sm;
   blocks = blocks < grid.sms * kMaxBlocksPerSm ? blocks : grid.sms * kMaxBlocksPerSm;
@@ -1215,29 +1234,25 @@ cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, 
 namespace {
 constexpr int kDirectBlock = 128;
 template <bool kGeneral>
-const Grid& direct_grid() {
-  static const Grid grid = resident_grid(k_direct<kDirectBlock, kGeneral>, kDirectBlock,
-                                         kDirectBlock / 32 * kDirectWarpSmem<kGeneral>, kPathThreads / kDirectBlock);
-  return grid;
-}
-
-template <bool kGeneral>
 cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance,
                                    WaveCounters* cnt, float4* pending, int pending_depth, int tree, cudaStream_t stream) {
   if (passes.samples() < kDirectWarpSamples) {
     constexpr int kMaxPerSm = 2048 / kDirectBlock;
-    static const Grid grid = resident_grid(k_direct_sample<kDirectBlock, kGeneral>, kDirectBlock, 0, kMaxPerSm);
+    static GridTable grids;
+    const Grid grid = grids.get(k_direct_sample<kDirectBlock, kGeneral>, kDirectBlock, 0, kMaxPerSm);
     if (grid.err != cudaSuccess) return grid.err;
     k_direct_sample<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, 0, stream>>>(job_dev, passes,
                                                                                                radiance, cnt, tree);
     return cudaGetLastError();
   }
-  const Grid& grid = direct_grid<kGeneral>();
+  constexpr std::size_t smem = kDirectBlock / 32 * kDirectWarpSmem<kGeneral>;
+  static GridTable grids;
+  const Grid grid = grids.get(k_direct<kDirectBlock, kGeneral>, kDirectBlock, smem, kPathThreads / kDirectBlock);
   if (grid.err != cudaSuccess) return grid.err;
   const cudaError_t e = cudaMemsetAsync(&cnt->direct_fetch, 0, sizeof(cnt->direct_fetch), stream);
   if (e != cudaSuccess) return e;
-  k_direct<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, kDirectBlock / 32 * kDirectWarpSmem<kGeneral>,
-                                     stream>>>(job_dev, passes, radiance, cnt, pending, pending_depth, tree);
+  k_direct<kDirectBlock, kGeneral><<<grid.sms * grid.per_sm, kDirectBlock, smem, stream>>>(
+      job_dev, passes, radiance, cnt, pending, pending_depth, tree);
   return cudaGetLastError();
 }
 }  // namespace
