@@ -22,6 +22,8 @@ namespace {
 constexpr int kBins = 16;
 constexpr int kDepthCap = 60;
 constexpr int kSmallItems = 32;          // a warp builds a node this small, and its subtree, whole
+constexpr int kMidItems = 1024;          // a block builds a node this small down to the small ones
+constexpr int kMidWarps = 8;
 constexpr int kChunk = 256;              // primitives per warp in the level passes (8 per lane)
 constexpr int kBinWords = 3 * kBins * 7; // per large node: 3 axes x 16 bins x (6 box keys + count)
 constexpr int kMaxLevels = 64;
@@ -38,15 +40,17 @@ constexpr int kWarpsPerBlock = 4;
 struct LevelCount {
   int tasks;   // large nodes of a level
   int chunks;  // their 256-primitive chunks
+  int base;    // the first of them in the task list
 };
 struct Counters {
   int nodes;          // node ids handed out
+  int mid_roots;      // nodes built by one block
   int small_roots;    // nodes built whole by one warp
   int error;          // 1: a leaf of more than 65535 primitives; 2: partition counts disagree
   int leaves, max_leaf, max_depth;
   int interior;       // interior nodes (root's interior subtree size)
   int wide_total;
-  LevelCount lvl[2];  // by level parity: the level being created
+  LevelCount lvl[kMaxLevels + 1];
   int wide_cnt[kMaxLevels + 2];
   int wide_off[kMaxLevels + 2];
 };
@@ -86,14 +90,20 @@ __device__ __forceinline__ void load_box(const double* boxes, unsigned id, doubl
   hi[0] = m.y; hi[1] = z.x; hi[2] = z.y;
 }
 
+// Smallest and largest double of a warp (no NaN), by the order of its key's words: four
+// reductions in hardware in place of 30 shuffles and compares.
 __device__ __forceinline__ double warp_min(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
+  const long long k = key_of(v);
+  const int hi = static_cast<int>(k >> 32);
+  const unsigned lo = static_cast<unsigned>(k);
+  const int best = __reduce_min_sync(0xFFFFFFFFu, hi);
+  const unsigned low = __reduce_min_sync(0xFFFFFFFFu, hi == best ? lo : 0xFFFFFFFFu);
+  return value_of((static_cast<long long>(best) << 32) | low);
 }
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
-}
+__device__ __forceinline__ double warp_max(double v) { return -warp_min(-v); }
+// Of two doubles, no NaN (fmin and fmax spend most of their instructions on those).
+__device__ __forceinline__ double less_of(double a, double b) { return b < a ? b : a; }
+__device__ __forceinline__ double more_of(double a, double b) { return b > a ? b : a; }
 
 // One float step toward -inf / +inf by bits (std::nextafterf for finite f).
 __device__ __forceinline__ float step_down(float f) {
@@ -147,6 +157,9 @@ struct GpuBvhBuilder::State {
   int* local = nullptr;               // preorder index inside the small subtree
   int* ilocal = nullptr;              // interior preorder index inside the small subtree
   int* tasks = nullptr;               // large nodes, level after level
+  int* mid_roots = nullptr;
+  int* mid_nodes = nullptr;           // nodes a block builds, level after level, from its root's first primitive on
+  int* mid_ends = nullptr;            // ends of those levels, kMaxLevels per root
   int* small_roots = nullptr;
   // per level of large nodes, by parity
   long long* bins[2] = {};
@@ -165,6 +178,7 @@ struct GpuBvhBuilder::State {
   int* cnt_rt[2] = {};
   int* base_lf[2] = {};
   int* base_rt[2] = {};
+  unsigned* moves = nullptr;
   // four-wide collapse
   int* wide_list = nullptr;
   int* wide_kids = nullptr;           // 4 per binary node
@@ -172,15 +186,14 @@ struct GpuBvhBuilder::State {
   std::uint32_t* wscan = nullptr;
   std::uint32_t* scan_sums = nullptr;
   std::uint8_t* last = nullptr;       // last slot of a leaf
-  std::vector<std::pair<int, int>> levels;  // (first task, tasks) of each level
 };
 
 namespace {
 
 __device__ __forceinline__ double pos_inf() { return __longlong_as_double(0x7FF0000000000000LL); }
 
-// Pointers and sizes the level kernels share. `parity` is the level's parity;
-// the *_next arrays belong to the level the kernels create.
+// Pointers the level kernels share; the *_next arrays belong to the level they create.
+// Sizes come from the counters, so the host launches levels without waiting for them.
 struct LevelArgs {
   const double* boxes;
   std::uint32_t* items;
@@ -194,11 +207,11 @@ struct LevelArgs {
   int* depth;
   int* axis;
   int* sub;
-  const int* tasks_cur;  // this level's large nodes
-  int* tasks_next;       // the next level's
+  int* tasks;  // large nodes, level after level
+  int* mid_roots;
   int* small_roots;
   Counters* counters;
-  int n_tasks, n_chunks, parity;
+  int level;
   long long* bins;
   int* need_part;
   int* part_t;
@@ -215,11 +228,15 @@ struct LevelArgs {
   int* cnt_rt;
   int* base_lf;
   int* base_rt;
+  unsigned* moves;  // 8 words a chunk
   long long* bins_next;
   int* task_chunk0_next;
   int* task_nchunks_next;
   int* chunk_task_next;
   std::uint32_t* chunk_start_next;
+  __device__ int n_tasks() const { return counters->lvl[level].tasks; }
+  __device__ int n_chunks() const { return counters->lvl[level].chunks; }
+  __device__ int task(int i) const { return tasks[counters->lvl[level].base + i]; }
 };
 
 // One bin of one axis as a lane holds it.
@@ -245,9 +262,10 @@ __device__ __forceinline__ void note_leaf(Counters* c, std::uint32_t n, int d) {
 }
 
 // Registers node c (primitives [first, first + n) of the working order, at
-// `depth`) as a large node of the next level, with its chunks, or as the root
-// of a subtree that one warp builds whole. Called by all 32 lanes of a warp.
-__device__ void enqueue_node(const LevelArgs& a, int c, std::uint32_t first, std::uint32_t n, int depth) {
+// `depth`) as a large node of level `next`, with its chunks, or as the root of a
+// subtree that one block or one warp builds. Called by all 32 lanes of a warp.
+__device__ void enqueue_node(const LevelArgs& a, int next, int next_base, int c, std::uint32_t first, std::uint32_t n,
+                             int depth) {
   const int lane = threadIdx.x & 31;
   if (lane == 0) {
     a.first[c] = first;
@@ -257,13 +275,15 @@ __device__ void enqueue_node(const LevelArgs& a, int c, std::uint32_t first, std
     a.left[c] = -1;
     a.right[c] = -1;
   }
-  if (n > static_cast<std::uint32_t>(kSmallItems)) {
+  if (n > static_cast<std::uint32_t>(kMidItems)) {
     const int nch = static_cast<int>((n + kChunk - 1) / kChunk);
     int slot = 0, c0 = 0;
     if (lane == 0) {
-      slot = atomicAdd(&a.counters->lvl[a.parity ^ 1].tasks, 1);
-      c0 = atomicAdd(&a.counters->lvl[a.parity ^ 1].chunks, nch);
-      a.tasks_next[slot] = c;
+      LevelCount& l = a.counters->lvl[next];
+      slot = atomicAdd(&l.tasks, 1);
+      c0 = atomicAdd(&l.chunks, nch);
+      l.base = next_base;
+      a.tasks[next_base + slot] = c;
       a.task_chunk0_next[slot] = c0;
       a.task_nchunks_next[slot] = nch;
     }
@@ -281,12 +301,13 @@ __device__ void enqueue_node(const LevelArgs& a, int c, std::uint32_t first, std
       a.chunk_start_next[c0 + j] = first + static_cast<std::uint32_t>(j) * kChunk;
     }
   } else if (lane == 0) {
-    a.small_roots[atomicAdd(&a.counters->small_roots, 1)] = c;
+    if (n > static_cast<std::uint32_t>(kSmallItems)) a.mid_roots[atomicAdd(&a.counters->mid_roots, 1)] = c;
+    else a.small_roots[atomicAdd(&a.counters->small_roots, 1)] = c;
   }
 }
 
-// The root: node 0 over every primitive. Launched with one warp; `a.parity` is 1
-// so that the root lands in level 0's arrays.
+// The root: node 0 over every primitive. Launched with one warp, with level 0's
+// arrays as the next.
 __global__ void k_init(LevelArgs a, std::uint32_t n, int* dfs, int* idfs) {
   if (blockIdx.x != 0) return;
   if (threadIdx.x == 0) {
@@ -294,30 +315,36 @@ __global__ void k_init(LevelArgs a, std::uint32_t n, int* dfs, int* idfs) {
     dfs[0] = 0;
     idfs[0] = 0;
   }
-  enqueue_node(a, 0, 0, n, 0);
+  enqueue_node(a, 0, 0, 0, 0, n, 0);
 }
 
 // Box and centroid bounds of each large node: one warp per 256-primitive chunk.
 __global__ void __launch_bounds__(128) k_bounds(LevelArgs a) {
   const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= a.n_chunks) return;
-  const int t = a.tasks_cur[a.chunk_task[w]];
+  if (w >= a.n_chunks()) return;
+  const int t = a.task(a.chunk_task[w]);
   const std::uint32_t start = a.chunk_start[w];
   const std::uint32_t end = min(start + static_cast<std::uint32_t>(kChunk), a.first[t] + a.count[t]);
   const double inf = pos_inf();
   double lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
   double clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+  std::uint32_t id[kChunk / 32];
+#pragma unroll
   for (int j = 0; j < kChunk / 32; ++j) {
+    // Past the end, the chunk's first primitive once more: a union may take it twice.
     const std::uint32_t pos = start + static_cast<std::uint32_t>(j * 32 + lane);
-    if (pos >= end) break;
+    id[j] = a.items[pos < end ? pos : start];
+  }
+#pragma unroll 4
+  for (int j = 0; j < kChunk / 32; ++j) {
     double bl[3], bh[3];
-    load_box(a.boxes, a.items[pos], bl, bh);
+    load_box(a.boxes, id[j], bl, bh);
     for (int k = 0; k < 3; ++k) {
-      lo[k] = fmin(lo[k], bl[k]);
-      hi[k] = fmax(hi[k], bh[k]);
+      lo[k] = less_of(lo[k], bl[k]);
+      hi[k] = more_of(hi[k], bh[k]);
       const double c = 0.5 * (bl[k] + bh[k]);
-      clo[k] = fmin(clo[k], c);
-      chi[k] = fmax(chi[k], c);
+      clo[k] = less_of(clo[k], c);
+      chi[k] = more_of(chi[k], c);
     }
   }
   for (int k = 0; k < 3; ++k) {
@@ -343,9 +370,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_bins(LevelArgs a) {
   __shared__ long long s_bins[kWarpsPerBlock][kBinWords];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = blockIdx.x * kWarpsPerBlock + wib;
-  if (w >= a.n_chunks) return;
+  if (w >= a.n_chunks()) return;
   const int lt = a.chunk_task[w];
-  const int t = a.tasks_cur[lt];
+  const int t = a.task(lt);
   if (a.depth[t] >= kDepthCap) return;  // becomes a leaf
   const long long* key = a.key + 12ll * t;
   double clo[3], inv[3];
@@ -394,8 +421,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_bins(LevelArgs a) {
         bin_clear(run[k]);
       }
       for (int m = 0; m < 3; ++m) {
-        run[k].lo[m] = fmin(run[k].lo[m], bl[m]);
-        run[k].hi[m] = fmax(run[k].hi[m], bh[m]);
+        run[k].lo[m] = less_of(run[k].lo[m], bl[m]);
+        run[k].hi[m] = more_of(run[k].hi[m], bh[m]);
       }
       ++run[k].n;
     }
@@ -416,57 +443,49 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_bins(LevelArgs a) {
   }
 }
 
-// The reference's SAH sweep over one axis's 16 bins (src/geometry/bvh.cpp:62-88),
-// with lane b of each 16-lane half holding bin b of that half's axis. The prefix
-// and suffix unions are scans (min / max and integer sums give the same values
-// in any order), every lane prices the plane after its bin, and the cheapest plane
-// wins with the lowest bin on ties, which is the first strictly cheaper plane of
-// the reference's loop. On return every lane of the half holds the axis's result
-// (cost +inf when no plane separates anything) and the primitives left of it.
-__device__ void half_sweep(const BinData& d, double area_floor, double& cost, int& bin, unsigned& left_n) {
-  const unsigned full = 0xFFFFFFFFu;
-  const int b = threadIdx.x & 15;
-  double pl[3], ph[3], sl[3], sh[3];
-  unsigned pn = d.n, sn = d.n;
+// A warp's bins during the sweep, 16 an axis: lower corners and negated upper ones, so
+// that every union is a minimum, and counts.
+struct Sweep {
+  double box[3 * kBins][6];
+  unsigned n[3 * kBins];
+};
+
+__device__ __forceinline__ void store_bins(Sweep& w, const BinData& r0, const BinData& r1) {
+  const int lane = threadIdx.x & 31;
   for (int k = 0; k < 3; ++k) {
-    pl[k] = sl[k] = d.lo[k];
-    ph[k] = sh[k] = d.hi[k];
+    w.box[lane][k] = r0.lo[k];
+    w.box[lane][3 + k] = -r0.hi[k];
   }
-  for (int o = 1; o < 16; o <<= 1) {
-    double ul[3], uh[3], dl[3], dh[3];
+  w.n[lane] = r0.n;
+  if (lane < kBins) {
     for (int k = 0; k < 3; ++k) {
-      ul[k] = __shfl_up_sync(full, pl[k], o, 16);
-      uh[k] = __shfl_up_sync(full, ph[k], o, 16);
-      dl[k] = __shfl_down_sync(full, sl[k], o, 16);
-      dh[k] = __shfl_down_sync(full, sh[k], o, 16);
+      w.box[2 * kBins + lane][k] = r1.lo[k];
+      w.box[2 * kBins + lane][3 + k] = -r1.hi[k];
     }
-    const unsigned un = __shfl_up_sync(full, pn, o, 16), dn = __shfl_down_sync(full, sn, o, 16);
-    if (b >= o) {
-      for (int k = 0; k < 3; ++k) {
-        pl[k] = fmin(pl[k], ul[k]);
-        ph[k] = fmax(ph[k], uh[k]);
-      }
-      pn += un;
-    }
-    if (b + o < 16) {
-      for (int k = 0; k < 3; ++k) {
-        sl[k] = fmin(sl[k], dl[k]);
-        sh[k] = fmax(sh[k], dh[k]);
-      }
-      sn += dn;
-    }
+    w.n[2 * kBins + lane] = r1.n;
   }
-  double rl[3], rh[3];
+}
+__device__ __forceinline__ void merge_bins(const Sweep& w, BinData& r0, BinData& r1) {
+  const int lane = threadIdx.x & 31;
   for (int k = 0; k < 3; ++k) {
-    rl[k] = __shfl_down_sync(full, sl[k], 1, 16);
-    rh[k] = __shfl_down_sync(full, sh[k], 1, 16);
+    r0.lo[k] = less_of(r0.lo[k], w.box[lane][k]);
+    r0.hi[k] = more_of(r0.hi[k], -w.box[lane][3 + k]);
   }
-  const unsigned rn = __shfl_down_sync(full, sn, 1, 16);
-  cost = pos_inf();
-  if (b < kBins - 1 && pn != 0 && rn != 0)
-    cost = 1.0 + (box_area(pl, ph) * double(pn) + box_area(rl, rh) * double(rn)) / area_floor;
-  bin = b;
-  left_n = pn;
+  r0.n += w.n[lane];
+  if (lane < kBins) {
+    for (int k = 0; k < 3; ++k) {
+      r1.lo[k] = less_of(r1.lo[k], w.box[2 * kBins + lane][k]);
+      r1.hi[k] = more_of(r1.hi[k], -w.box[2 * kBins + lane][3 + k]);
+    }
+    r1.n += w.n[2 * kBins + lane];
+  }
+}
+
+// The cheapest plane of each axis (src/geometry/bvh.cpp:62-88), as lane b of a
+// 16-lane half holds the plane after bin b of that half's axis: the lowest bin on ties,
+// which is the first strictly cheaper plane of the reference's loop.
+__device__ __forceinline__ void half_best(double& cost, int& bin, unsigned& left_n) {
+  const unsigned full = 0xFFFFFFFFu;
   for (int o = 8; o >= 1; o >>= 1) {
     const double oc = __shfl_xor_sync(full, cost, o, 16);
     const int ob = __shfl_xor_sync(full, bin, o, 16);
@@ -482,15 +501,68 @@ __device__ void half_sweep(const BinData& d, double area_floor, double& cost, in
 // The best split over the three axes, on every lane: r0 holds axis 0 (lanes
 // 0-15) and axis 1 (lanes 16-31), r1 axis 2 (lanes 0-15). Axes in order, the
 // first strictly cheaper wins; an axis whose centroids coincide is skipped.
-__device__ void warp_best_split(const BinData& r0, const BinData& r1, const bool use[3], double parent_area,
+//
+// The unions left and right of each plane are running minima in shared memory, a lane
+// for each axis and component: 2 x 16 short steps. Scans of 12 doubles by shuffles took
+// some 1,500 instructions a node, and their unrolled code missed the instruction cache.
+__device__ void warp_best_split(Sweep& w, const BinData& r0, const BinData& r1, const bool use[3], double parent_area,
                                 double& best_cost, int& best_axis, int& best_bin, unsigned& best_left) {
   const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31, b = lane & 15;
   const double area_floor = parent_area < 1e-30 ? 1e-30 : parent_area;
-  double c0, c1;
-  int b0, b1;
-  unsigned l0, l1;
-  half_sweep(r0, area_floor, c0, b0, l0);
-  half_sweep(r1, area_floor, c1, b1, l1);
+  // Of the planes after bin `lane` and bin 32 + lane: counts, and the left side's price.
+  double price[2];
+  unsigned ln[2], rn[2];
+  double c0 = pos_inf(), c1 = pos_inf();
+#pragma unroll 1
+  for (int right = 0; right < 2; ++right) {
+    store_bins(w, r0, r1);
+    __syncwarp();
+    if (lane < 18) {
+      const int ax = lane / 6, c = lane - 6 * ax, step = right ? -1 : 1;
+      int q = ax * kBins + (right ? kBins - 1 : 0);
+      double v = w.box[q][c];
+#pragma unroll 5
+      for (int k = 1; k < kBins; ++k) {
+        q += step;
+        v = less_of(v, w.box[q][c]);
+        w.box[q][c] = v;
+      }
+    } else if (lane < 21) {
+      const int step = right ? -1 : 1;
+      int q = (lane - 18) * kBins + (right ? kBins - 1 : 0);
+      unsigned v = w.n[q];
+#pragma unroll 5
+      for (int k = 1; k < kBins; ++k) {
+        q += step;
+        v += w.n[q];
+        w.n[q] = v;
+      }
+    }
+    __syncwarp();
+    auto side = [&](int q, unsigned& n) {
+      const double* e = w.box[q];
+      const double lo[3] = {e[0], e[1], e[2]}, hi[3] = {-e[3], -e[4], -e[5]};
+      n = w.n[q];
+      return box_area(lo, hi) * double(n);
+    };
+    // The right side of the plane after bin q starts at q + 1.
+    for (int r = 0; r < 2; ++r) {
+      if (r == 1 && lane >= kBins) break;
+      const int q = 2 * kBins * r + lane;
+      if (!right) {
+        price[r] = side(q, ln[r]);
+      } else if (b < kBins - 1) {
+        const double p = side(q + 1, rn[r]);
+        if (ln[r] != 0 && rn[r] != 0) (r ? c1 : c0) = 1.0 + (price[r] + p) / area_floor;
+      }
+    }
+    __syncwarp();
+  }
+  int b0 = b, b1 = b;
+  unsigned l0 = ln[0], l1 = lane < kBins ? ln[1] : 0u;
+  half_best(c0, b0, l0);
+  half_best(c1, b1, l1);
   const double cost[3] = {__shfl_sync(full, c0, 0), __shfl_sync(full, c0, 16), __shfl_sync(full, c1, 0)};
   const int bin[3] = {__shfl_sync(full, b0, 0), __shfl_sync(full, b0, 16), __shfl_sync(full, b1, 0)};
   const unsigned left[3] = {__shfl_sync(full, l0, 0), __shfl_sync(full, l0, 16), __shfl_sync(full, l1, 0)};
@@ -509,9 +581,10 @@ __device__ void warp_best_split(const BinData& r0, const BinData& r1, const bool
 
 // One warp per large node: box from the keys, SAH decision, children.
 __global__ void __launch_bounds__(128) k_decide(LevelArgs a) {
+  __shared__ Sweep s_sweep[4];
   const int i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (i >= a.n_tasks) return;
-  const int t = a.tasks_cur[i];
+  if (i >= a.n_tasks()) return;
+  const int t = a.task(i);
   const long long* key = a.key + 12ll * t;
   double lo[3], hi[3], clo[3], chi[3];
   for (int k = 0; k < 3; ++k) {
@@ -549,7 +622,7 @@ __global__ void __launch_bounds__(128) k_decide(LevelArgs a) {
     }
     double best_cost;
     unsigned left_n;
-    warp_best_split(r[0], r[1], use, box_area(lo, hi), best_cost, split_axis, best_bin, left_n);
+    warp_best_split(s_sweep[threadIdx.x >> 5], r[0], r[1], use, box_area(lo, hi), best_cost, split_axis, best_bin, left_n);
     if (split_axis < 0) {
       mid = n / 2;  // every centroid coincides
       split_axis = widest_axis(clo, chi);
@@ -588,48 +661,77 @@ __global__ void __launch_bounds__(128) k_decide(LevelArgs a) {
     a.right[t] = c + 1;
   }
   c = __shfl_sync(0xFFFFFFFFu, c, 0);
-  enqueue_node(a, c, f0, mid, d + 1);
-  enqueue_node(a, c + 1, f0 + mid, n - mid, d + 1);
+  const LevelCount& l = a.counters->lvl[a.level];
+  const int next_base = l.base + l.tasks;
+  enqueue_node(a, a.level + 1, next_base, c, f0, mid, d + 1);
+  enqueue_node(a, a.level + 1, next_base, c + 1, f0 + mid, n - mid, d + 1);
 }
 
-__device__ __forceinline__ bool goes_left(const LevelArgs& a, int lt, std::uint32_t id) {
-  const int ax = a.part_axis[lt];
-  const double* b = a.boxes + 6ull * id;
-  const double c = 0.5 * (__ldg(b + ax) + __ldg(b + 3 + ax));
-  return bin_of(c, a.part_lo[lt], a.part_inv[lt]) <= a.part_bin[lt];
-}
+// A warp's chunk in the partition passes.
+struct PartChunk {
+  int lt;                          // its node's task
+  std::uint32_t f0, start, split, end, last;  // node's first, chunk's first, first of the right side, chunk's and node's end
+  bool on;
+  __device__ PartChunk(const LevelArgs& a, int w) : on(false) {
+    if (w >= a.n_chunks()) return;
+    lt = a.chunk_task[w];
+    if (!a.need_part[lt]) return;
+    on = true;
+    const int t = a.task(lt);
+    f0 = a.first[t];
+    last = f0 + a.count[t];
+    start = a.chunk_start[w];
+    end = min(start + static_cast<std::uint32_t>(kChunk), last);
+    split = f0 + static_cast<std::uint32_t>(a.part_t[lt]);
+  }
+  // Bits of 32 places from `pos` on that lie on the right side.
+  __device__ unsigned right_side(std::uint32_t pos) const {
+    return pos >= split ? 0xFFFFFFFFu : (split - pos >= 32 ? 0u : 0xFFFFFFFFu << (split - pos));
+  }
+};
 
-// Partition, pass 1: per chunk, primitives on the left that belong on the right
-// ("left-false") and primitives on the right that belong on the left.
+// Partition, pass 1: per chunk, which primitives belong on the left (a word for 32
+// places, which the next passes read in place of the primitives), and how many on the
+// left belong on the right ("left-false") and the other way round.
 __global__ void __launch_bounds__(128) k_pcount(LevelArgs a) {
   const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= a.n_chunks) return;
-  const int lt = a.chunk_task[w];
-  if (!a.need_part[lt]) return;
-  const int t = a.tasks_cur[lt];
-  const std::uint32_t f0 = a.first[t], start = a.chunk_start[w];
-  const std::uint32_t end = min(start + static_cast<std::uint32_t>(kChunk), f0 + a.count[t]);
-  const std::uint32_t split = f0 + static_cast<std::uint32_t>(a.part_t[lt]);
-  unsigned lf = 0, rt = 0;
+  const PartChunk c(a, w);
+  if (!c.on) return;
+  const int ax = a.part_axis[c.lt], bin = a.part_bin[c.lt];
+  const double lo = a.part_lo[c.lt], inv = a.part_inv[c.lt];
+  std::uint32_t id[kChunk / 32];
+#pragma unroll
   for (int j = 0; j < kChunk / 32; ++j) {
-    const std::uint32_t pos = start + static_cast<std::uint32_t>(j * 32 + lane);
-    if (pos >= end) break;
-    const bool l = goes_left(a, lt, a.items[pos]);
-    if (pos < split) lf += !l;
-    else rt += l;
+    const std::uint32_t pos = c.start + static_cast<std::uint32_t>(j * 32 + lane);
+    id[j] = pos < c.end ? a.items[pos] : 0xFFFFFFFFu;
   }
-  lf = __reduce_add_sync(0xFFFFFFFFu, lf);
-  rt = __reduce_add_sync(0xFFFFFFFFu, rt);
+  int lf = 0, rt = 0;
+#pragma unroll
+  for (int j = 0; j < kChunk / 32; ++j) {
+    bool l = false;
+    if (id[j] != 0xFFFFFFFFu) {
+      const double* b = a.boxes + 6ull * id[j];
+      l = bin_of(0.5 * (__ldg(b + ax) + __ldg(b + 3 + ax)), lo, inv) <= bin;
+    }
+    const unsigned bits = __ballot_sync(0xFFFFFFFFu, l);
+    const std::uint32_t pos = c.start + static_cast<std::uint32_t>(j * 32);
+    const unsigned there = pos >= c.end ? 0u : (c.end - pos >= 32 ? 0xFFFFFFFFu : (1u << (c.end - pos)) - 1u);
+    const unsigned right = c.right_side(pos);
+    lf += __popc(~bits & there & ~right);
+    rt += __popc(bits & right);
+    // Left-false and right-true places, the only ones that move.
+    if (lane == 0) a.moves[w * (kChunk / 32) + j] = (~bits & there & ~right) | (bits & right);
+  }
   if (lane == 0) {
-    a.cnt_lf[w] = static_cast<int>(lf);
-    a.cnt_rt[w] = static_cast<int>(rt);
+    a.cnt_lf[w] = lf;
+    a.cnt_rt[w] = rt;
   }
 }
 
 // Partition, pass 2: one warp per node scans its chunks' counts.
 __global__ void __launch_bounds__(128) k_pscan(LevelArgs a) {
   const int i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (i >= a.n_tasks || !a.need_part[i]) return;
+  if (i >= a.n_tasks() || !a.need_part[i]) return;
   const int c0 = a.task_chunk0[i], nch = a.task_nchunks[i];
   int carry_lf = 0, carry_rt = 0;
   for (int b = 0; b < nch; b += 32) {
@@ -661,25 +763,19 @@ __global__ void __launch_bounds__(128) k_pscan(LevelArgs a) {
 // counted from the right end, records its position at scratch[first + k].
 __global__ void __launch_bounds__(128) k_pranks(LevelArgs a) {
   const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= a.n_chunks) return;
-  const int lt = a.chunk_task[w];
-  if (!a.need_part[lt]) return;
-  const int t = a.tasks_cur[lt];
-  const std::uint32_t f0 = a.first[t], start = a.chunk_start[w];
-  const std::uint32_t end = min(start + static_cast<std::uint32_t>(kChunk), f0 + a.count[t]);
-  const std::uint32_t split = f0 + static_cast<std::uint32_t>(a.part_t[lt]);
-  const int m = a.part_m[lt];
+  const PartChunk c(a, w);
+  if (!c.on) return;
+  const int m = a.part_m[c.lt];
   int run = a.base_rt[w];
+#pragma unroll
   for (int j = 0; j < kChunk / 32; ++j) {
-    const std::uint32_t pos = start + static_cast<std::uint32_t>(j * 32 + lane);
-    bool rt = false;
-    if (pos < end && pos >= split) rt = goes_left(a, lt, a.items[pos]);
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, rt);
-    if (rt) {
-      const int r = m - 1 - (run + __popc(bal & ((1u << lane) - 1u)));
-      if (r >= 0 && r < m) a.scratch[f0 + static_cast<std::uint32_t>(r)] = pos;
+    const std::uint32_t pos = c.start + static_cast<std::uint32_t>(j * 32);
+    const unsigned rt = a.moves[w * (kChunk / 32) + j] & c.right_side(pos);
+    if ((rt >> lane) & 1u) {
+      const int r = m - 1 - (run + __popc(rt & ((1u << lane) - 1u)));
+      if (r >= 0 && r < m) a.scratch[c.f0 + static_cast<std::uint32_t>(r)] = pos + lane;
     }
-    run += __popc(bal);
+    run += __popc(rt);
   }
 }
 
@@ -688,41 +784,310 @@ __global__ void __launch_bounds__(128) k_pranks(LevelArgs a) {
 // scheme, as std::partition runs it).
 __global__ void __launch_bounds__(128) k_pswap(LevelArgs a) {
   const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= a.n_chunks) return;
-  const int lt = a.chunk_task[w];
-  if (!a.need_part[lt]) return;
-  const int t = a.tasks_cur[lt];
-  const std::uint32_t f0 = a.first[t], start = a.chunk_start[w];
-  const std::uint32_t end = min(start + static_cast<std::uint32_t>(kChunk), f0 + a.count[t]);
-  const std::uint32_t split = f0 + static_cast<std::uint32_t>(a.part_t[lt]);
-  const int m = a.part_m[lt];
+  const PartChunk c(a, w);
+  if (!c.on) return;
+  const int m = a.part_m[c.lt];
   int run = a.base_lf[w];
+#pragma unroll
   for (int j = 0; j < kChunk / 32; ++j) {
-    const std::uint32_t pos = start + static_cast<std::uint32_t>(j * 32 + lane);
-    bool lf = false;
-    std::uint32_t mine = 0;
-    if (pos < end && pos < split) {
-      mine = a.items[pos];
-      lf = !goes_left(a, lt, mine);
-    }
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, lf);
-    if (lf) {
-      const int k = run + __popc(bal & ((1u << lane) - 1u));
+    const std::uint32_t first = c.start + static_cast<std::uint32_t>(j * 32), pos = first + lane;
+    const unsigned lf = a.moves[w * (kChunk / 32) + j] & ~c.right_side(first);
+    if ((lf >> lane) & 1u) {
+      const int k = run + __popc(lf & ((1u << lane) - 1u));
       if (k < m) {
-        const std::uint32_t q = a.scratch[f0 + static_cast<std::uint32_t>(k)];
-        if (q >= split && q < f0 + a.count[t]) {  // always true; keeps the swap in the node's range
+        const std::uint32_t q = a.scratch[c.f0 + static_cast<std::uint32_t>(k)];
+        if (q >= c.split && q < c.last) {  // always true; keeps the swap in the node's range
+          const std::uint32_t mine = a.items[pos];
           a.items[pos] = a.items[q];
           a.items[q] = mine;
         }
       }
     }
-    run += __popc(bal);
+    run += __popc(lf);
   }
 }
 
 }  // namespace
 
 namespace {
+
+// Adds 32 primitives to a node's bins: bin[k] is the bin of this lane's primitive on
+// axis k (-1: none), box(p) the box of lane p's. r[0] is axis 0 on lanes 0-15 and axis 1
+// on lanes 16-31, r[1] axis 2: primitives 0-15 on lanes 0-15, the others on lanes 16-31,
+// until fold_axis2 brings them together. Each lane then visits its own bin's primitives
+// only, two at a time. Before, every lane scanned all 32, in 64 divergent steps; with this,
+// the sweep and the reductions, k_small takes 240 us on 174k triangles (513). Neighbours
+// that share a bin make it slow: k_bins, with 256 neighbours a warp, merges runs instead
+// (35 us a level; 59 this way).
+template <class Box>
+__device__ __forceinline__ void bin_lanes(unsigned* mask, const int bin[3], BinData r[2], Box box) {
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  for (int q = lane; q < 3 * kBins; q += 32) mask[q] = 0;
+  __syncwarp();
+  for (int k = 0; k < 3; ++k) {
+    const unsigned same = __match_any_sync(full, bin[k]);
+    if (bin[k] >= 0 && lane == __ffs(same) - 1) mask[k * kBins + bin[k]] = same;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int round = 0; round < 2; ++round) {
+    BinData& e = r[round];
+    unsigned m = round == 0 ? mask[lane] : (mask[2 * kBins + (lane & 15)] & (lane < 16 ? 0xFFFFu : 0xFFFF0000u));
+    e.n += __popc(m);
+    while (m) {
+      const double* b = box(__ffs(m) - 1);
+      const unsigned rest = m & (m - 1);
+      const double* b2 = box(__ffs(rest ? rest : m) - 1);  // with none left, the same one again
+      m = rest & (rest - 1);
+      for (int k = 0; k < 3; ++k) {
+        e.lo[k] = less_of(e.lo[k], less_of(b[k], b2[k]));
+        e.hi[k] = more_of(e.hi[k], more_of(b[3 + k], b2[3 + k]));
+      }
+    }
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void fold_axis2(BinData& e) {
+  for (int k = 0; k < 3; ++k) {
+    e.lo[k] = less_of(e.lo[k], __shfl_xor_sync(0xFFFFFFFFu, e.lo[k], 16));
+    e.hi[k] = more_of(e.hi[k], __shfl_xor_sync(0xFFFFFFFFu, e.hi[k], 16));
+  }
+  e.n += __shfl_xor_sync(0xFFFFFFFFu, e.n, 16);
+}
+
+struct MidArgs {
+  const double* boxes;
+  std::uint32_t* items;
+  double* box;
+  int* left;
+  int* right;
+  std::uint32_t* first;
+  std::uint32_t* count;
+  int* depth;
+  int* axis;
+  int* sub;
+  const int* mid_roots;
+  int* mid_nodes;
+  int* mid_ends;
+  int* small_roots;
+  Counters* counters;
+};
+
+// A block's workspace: its root's primitives by the place they came in, and their order.
+struct MidBlock {
+  double box[kMidItems][6];
+  std::uint32_t id[kMidItems];
+  std::uint16_t order[kMidItems], partner[kMidItems];
+  unsigned mask[kMidWarps][3 * kBins];
+  Sweep sweep[kMidWarps];
+  double bounds[kMidWarps][12];
+  int listed;
+};
+
+// The last part of a node's split; one warp. Bounds, bins and the rest as split_mids has them.
+__device__ void split_mid(const MidArgs& a, MidBlock& s, int* list, std::uint32_t b0, int t, int lo, int n, int d,
+                          const double bl[3], const double bh[3], const double cl[3], const double ch[3],
+                          const bool use[3], const double inv[3], const BinData r[2]) {
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31, hi = lo + n;
+  const unsigned below = (1u << lane) - 1u;
+  if (lane == 0)
+    for (int k = 0; k < 3; ++k) {
+      a.box[6ll * t + k] = bl[k];
+      a.box[6ll * t + 3 + k] = bh[k];
+    }
+  if (d >= kDepthCap) {
+    if (lane == 0) {
+      a.left[t] = -1;
+      a.right[t] = -1;
+      a.axis[t] = 0;
+      note_leaf(a.counters, static_cast<std::uint32_t>(n), d);
+    }
+    return;
+  }
+  double best_cost;
+  int axis, best_bin;
+  unsigned left_n;
+  warp_best_split(s.sweep[threadIdx.x >> 5], r[0], r[1], use, box_area(bl, bh), best_cost, axis, best_bin, left_n);
+  int mid = n / 2;  // every centroid coincides, or rounding put everything on one side
+  if (axis < 0) {
+    axis = widest_axis(cl, ch);
+  } else if (left_n != 0 && left_n != static_cast<unsigned>(n)) {
+    mid = static_cast<int>(left_n);
+    const double c0 = cl[axis], scale = inv[axis];
+    auto goes_left = [&](int i) {
+      const double* b = s.box[s.order[i]];
+      return bin_of(0.5 * (b[axis] + b[3 + axis]), c0, scale) <= best_bin;
+    };
+    // The k-th primitive from the right end that belongs on the left ...
+    int n_right = 0, n_left = 0;
+    for (int i0 = hi - 1; i0 >= lo + mid; i0 -= 32) {
+      const int i = i0 - lane;
+      const bool moves = i >= lo + mid && goes_left(i);
+      const unsigned m = __ballot_sync(full, moves);
+      if (moves) s.partner[lo + n_right + __popc(m & below)] = static_cast<std::uint16_t>(i);
+      n_right += __popc(m);
+    }
+    __syncwarp();
+    // ... trades places with the k-th from the left that belongs on the right.
+    for (int i0 = lo; i0 < lo + mid; i0 += 32) {
+      const int i = i0 + lane;
+      const bool moves = i < lo + mid && !goes_left(i);
+      const unsigned m = __ballot_sync(full, moves);
+      const int k = n_left + __popc(m & below);
+      if (moves && k < n_right) {
+        const int q = s.partner[lo + k];
+        const std::uint16_t v = s.order[i];
+        s.order[i] = s.order[q];
+        s.order[q] = v;
+      }
+      n_left += __popc(m);
+    }
+    if (lane == 0 && n_left != n_right) atomicOr(&a.counters->error, 2);
+    __syncwarp();
+  }
+  if (lane == 0) {
+    const int c = atomicAdd(&a.counters->nodes, 2);
+    a.left[t] = c;
+    a.right[t] = c + 1;
+    a.axis[t] = axis;
+    for (int k = 0; k < 2; ++k) {
+      const int cn = k ? n - mid : mid;
+      a.first[c + k] = b0 + static_cast<std::uint32_t>(k ? lo + mid : lo);
+      a.count[c + k] = static_cast<std::uint32_t>(cn);
+      a.depth[c + k] = d + 1;
+      a.sub[c + k] = -1;
+      a.left[c + k] = -1;
+      a.right[c + k] = -1;
+      if (cn > kSmallItems) list[atomicAdd(&s.listed, 1)] = c + k;
+      else a.small_roots[atomicAdd(&a.counters->small_roots, 1)] = c + k;
+    }
+  }
+}
+
+// Splits the block's nodes list[begin .. end). The decisions are k_decide's, the
+// exchange the one of k_pcount to k_pswap. Where a level has fewer nodes than the block
+// has warps, a team of warps takes each: they share its bounds and its bins, and the
+// team's first warp does the rest.
+__device__ void split_mids(const MidArgs& a, MidBlock& s, int* list, std::uint32_t b0, int begin, int end) {
+  const int warp = static_cast<int>(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const double inf = pos_inf();
+  const int team_warps = max(1, kMidWarps / (end - begin)), teams = kMidWarps / team_warps;
+  const int team = warp / team_warps, member = warp % team_warps, leader = warp - member;
+  for (int at = begin; at < end; at += teams) {
+    const bool on = team < teams && at + team < end;
+    int t = 0, lo = 0, n = 0, hi = 0, d = kDepthCap;
+    if (on) {
+      t = list[at + team];
+      lo = static_cast<int>(a.first[t] - b0);
+      n = static_cast<int>(a.count[t]);
+      hi = lo + n;
+      d = a.depth[t];
+    }
+    // Box and centroid bounds, upper ends negated.
+    double v[12];
+    for (int k = 0; k < 12; ++k) v[k] = inf;
+    for (int i = lo + 32 * member + lane; i < hi; i += 32 * team_warps) {
+      const double* b = s.box[s.order[i]];
+      for (int k = 0; k < 3; ++k) {
+        v[k] = less_of(v[k], b[k]);
+        v[3 + k] = less_of(v[3 + k], -b[3 + k]);
+        const double c = 0.5 * (b[k] + b[3 + k]);
+        v[6 + k] = less_of(v[6 + k], c);
+        v[9 + k] = less_of(v[9 + k], -c);
+      }
+    }
+    for (int k = 0; k < 12; ++k) v[k] = warp_min(v[k]);
+    if (team_warps > 1) {
+      if (lane == 0)
+        for (int k = 0; k < 12; ++k) s.bounds[warp][k] = v[k];
+      __syncthreads();
+      for (int k = 0; k < 12; ++k)
+        for (int m = 0; on && m < team_warps; ++m) v[k] = less_of(v[k], s.bounds[leader + m][k]);
+    }
+    const double bl[3] = {v[0], v[1], v[2]}, bh[3] = {-v[3], -v[4], -v[5]};
+    const double cl[3] = {v[6], v[7], v[8]}, ch[3] = {-v[9], -v[10], -v[11]};
+    bool use[3];
+    double inv[3];
+    for (int k = 0; k < 3; ++k) {
+      use[k] = ch[k] > cl[k];
+      inv[k] = use[k] ? kBins / (ch[k] - cl[k]) : 0.0;
+    }
+    BinData r[2];
+    bin_clear(r[0]);
+    bin_clear(r[1]);
+    if (d < kDepthCap) {
+      for (int i0 = lo + 32 * member; i0 < hi; i0 += 32 * team_warps) {
+        int bin[3] = {-1, -1, -1};
+        if (i0 + lane < hi) {
+          const double* b = s.box[s.order[i0 + lane]];
+          for (int k = 0; k < 3; ++k)
+            if (use[k]) bin[k] = bin_of(0.5 * (b[k] + b[3 + k]), cl[k], inv[k]);
+        }
+        bin_lanes(s.mask[warp], bin, r, [&](int p) { return s.box[s.order[i0 + p]]; });
+      }
+      fold_axis2(r[1]);
+    }
+    if (team_warps > 1) {
+      if (member > 0) store_bins(s.sweep[warp], r[0], r[1]);
+      __syncthreads();
+      if (member == 0 && on)
+        for (int m = 1; m < team_warps; ++m) merge_bins(s.sweep[warp + m], r[0], r[1]);
+    }
+    if (member == 0 && on) split_mid(a, s, list, b0, t, lo, n, d, bl, bh, cl, ch, use, inv, r);
+    __syncthreads();
+  }
+}
+
+// Builds the subtree under each node of 33 to kMidItems primitives down to its small
+// nodes: one block per root, its boxes in shared memory, level by level. A level of the
+// level kernels is 7 launches and, before, a look at its size from the host: some 100 us,
+// however little it holds. On 174,085 triangles this kernel takes 195 us in place of 6 of
+// 15 levels; 2,048 primitives a block would save one level more and measure the same on
+// 2,000 primitives, but 0.1 ms worse on 174k. Latency bounds it: two roots take as long as
+// 250. With the shorter passes, the build takes 0.54 ms for 2,053 triangles (1.01 before),
+// 0.91 for 25,525 (1.57) and 1.40 for 174,085 (2.45).
+// Every node of the list holds more than 32 primitives, so a list never outgrows its
+// root's share of mid_nodes (one entry per primitive).
+__global__ void __launch_bounds__(kMidWarps * 32) k_mid(MidArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  MidBlock& s = *reinterpret_cast<MidBlock*>(smem);
+  if (static_cast<int>(blockIdx.x) >= a.counters->mid_roots) return;
+  const int root = a.mid_roots[blockIdx.x];
+  const std::uint32_t b0 = a.first[root];
+  const int n = static_cast<int>(a.count[root]);
+  for (int i = threadIdx.x; i < n; i += kMidWarps * 32) {
+    const std::uint32_t id = a.items[b0 + i];
+    double lo[3], hi[3];
+    load_box(a.boxes, id, lo, hi);
+    for (int k = 0; k < 3; ++k) {
+      s.box[i][k] = lo[k];
+      s.box[i][3 + k] = hi[k];
+    }
+    s.id[i] = id;
+    s.order[i] = static_cast<std::uint16_t>(i);
+  }
+  int* const list = a.mid_nodes + b0;
+  int* const ends = a.mid_ends + static_cast<long long>(blockIdx.x) * kMaxLevels;
+  if (threadIdx.x == 0) {
+    list[0] = root;
+    s.listed = 1;
+  }
+  __syncthreads();
+  int begin = 0, end = 1, level = 0;
+  // At most kDepthCap + 1 levels: deeper nodes are leaves.
+  while (begin < end) {
+    if (threadIdx.x == 0) ends[level] = end;
+    ++level;
+    split_mids(a, s, list, b0, begin, end);
+    begin = end;
+    end = s.listed;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && level < kMaxLevels) ends[level] = 0;
+  for (int i = threadIdx.x; i < n; i += kMidWarps * 32) a.items[b0 + i] = s.id[s.order[i]];
+}
 
 constexpr int kSmallNodes = 2 * kSmallItems - 1;
 
@@ -742,7 +1107,6 @@ struct SmallArgs {
   int* local;
   int* ilocal;
   const int* small_roots;
-  int n_small;
   Counters* counters;
 };
 
@@ -756,6 +1120,8 @@ struct SmallWarp {
   double nbox[kSmallNodes][6];
   int nl[kSmallNodes], nr[kSmallNodes], nfirst[kSmallNodes], ncount[kSmallNodes], naxis[kSmallNodes];
   int ndepth[kSmallNodes], nsize[kSmallNodes], nisize[kSmallNodes], nilocal[kSmallNodes];
+  unsigned mask[3 * kBins];
+  Sweep sweep;
   int stk_lo[kSmallItems], stk_hi[kSmallItems], stk_depth[kSmallItems], stk_parent[kSmallItems], stk_side[kSmallItems];
 };
 
@@ -769,13 +1135,8 @@ __device__ __forceinline__ int kth_highest(unsigned mask, int k) {
 // warp per node, exactly as the recursive build would: nodes are made in
 // preorder (left subtree before right), each with the same bounds, SAH decision
 // and partition as at the large levels.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_small(SmallArgs a) {
-  __shared__ SmallWarp s_all[kWarpsPerBlock];
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * kWarpsPerBlock + wib;
-  if (w >= a.n_small) return;
-  SmallWarp& s = s_all[wib];
-  const int r = a.small_roots[w];
+__device__ void build_small(const SmallArgs& a, SmallWarp& s, int r) {
+  const int lane = threadIdx.x & 31;
   const std::uint32_t b0 = a.first[r];
   const int n = static_cast<int>(a.count[r]);
   const double inf = pos_inf();
@@ -831,8 +1192,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_small(SmallArgs a) {
     int kind = 0;  // 0 leaf, 1 middle split, 2 SAH partition
     int sp_axis = 0, sp_bin = -1, mid = lo;
     if (!(cnt <= 4 || d >= kDepthCap)) {
-      // Lane (axis, bin) bins the node's primitives itself: round 0 covers axes
-      // 0 and 1 (lanes 0-15, 16-31), round 1 axis 2 (lanes 0-15).
       bool use[3];
       double inv[3];
       for (int k = 0; k < 3; ++k) {
@@ -840,24 +1199,16 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_small(SmallArgs a) {
         inv[k] = use[k] ? kBins / (ch[k] - cl[k]) : 0.0;
       }
       BinData r[2];
-      for (int round = 0; round < 2; ++round) {
-        BinData& e = r[round];
-        bin_clear(e);
-        const int ax = round == 0 ? (lane >> 4) : 2, b = lane & 15;
-        if ((round == 1 && lane >= 16) || !use[ax]) continue;
-        for (int p = lo; p < hi; ++p) {
-          if (bin_of(s.cen[p][ax], cl[ax], inv[ax]) != b) continue;
-          for (int k = 0; k < 3; ++k) {
-            e.lo[k] = fmin(e.lo[k], s.box[p][k]);
-            e.hi[k] = fmax(e.hi[k], s.box[p][3 + k]);
-          }
-          ++e.n;
-        }
-      }
+      bin_clear(r[0]);
+      bin_clear(r[1]);
+      int bin[3];
+      for (int k = 0; k < 3; ++k) bin[k] = act && use[k] ? bin_of(s.cen[lane][k], cl[k], inv[k]) : -1;
+      bin_lanes(s.mask, bin, r, [&](int p) { return s.box[p]; });
+      fold_axis2(r[1]);
       double best_cost;
       int best_axis, best_bin;
       unsigned left_n;
-      warp_best_split(r[0], r[1], use, box_area(bl, bh), best_cost, best_axis, best_bin, left_n);
+      warp_best_split(s.sweep, r[0], r[1], use, box_area(bl, bh), best_cost, best_axis, best_bin, left_n);
       if (best_axis < 0) {
         kind = 1;
         sp_axis = widest_axis(cl, ch);
@@ -971,6 +1322,16 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_small(SmallArgs a) {
   if (lane < n) a.items[b0 + lane] = s.id[lane];
 }
 
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_small(SmallArgs a) {
+  __shared__ SmallWarp s_all[kWarpsPerBlock];
+  const int wib = threadIdx.x >> 5;
+  const int n_small = a.counters->small_roots;
+  for (int w = blockIdx.x * kWarpsPerBlock + wib; w < n_small; w += gridDim.x * kWarpsPerBlock) {
+    build_small(a, s_all[wib], a.small_roots[w]);
+    __syncwarp();
+  }
+}
+
 }  // namespace
 
 namespace {
@@ -992,11 +1353,9 @@ struct TreeArgs {
   Counters* counters;
 };
 
-// Subtree sizes of one level's large nodes (their children are done already).
-__global__ void k_sizes(TreeArgs a, const int* tasks, int n) {
-  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= n) return;
-  const int t = tasks[i], l = a.left[t], r = a.right[t];
+// Subtree sizes of a node whose children have theirs.
+__device__ __forceinline__ void node_sizes(const TreeArgs& a, int t) {
+  const int l = a.left[t], r = a.right[t];
   if (l < 0) {
     a.size[t] = 1;
     a.isize[t] = 0;
@@ -1006,17 +1365,59 @@ __global__ void k_sizes(TreeArgs a, const int* tasks, int n) {
   }
 }
 
-// Depth-first indices (all nodes, and interior nodes only) of one level's
-// children: left follows its parent, right follows the left subtree.
-__global__ void k_dfs(TreeArgs a, const int* tasks, int n) {
-  const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= n) return;
-  const int t = tasks[i], l = a.left[t], r = a.right[t];
+// Of all large nodes, level by level: one block, since a level has few of them.
+__global__ void __launch_bounds__(512) k_sizes(TreeArgs a, const int* tasks, int levels) {
+  for (int k = levels - 1; k >= 0; --k) {
+    const LevelCount l = a.counters->lvl[k];
+    for (int i = threadIdx.x; i < l.tasks; i += blockDim.x) node_sizes(a, tasks[l.base + i]);
+    __syncthreads();
+  }
+}
+
+// Depth-first indices (all nodes, and interior nodes only) of a node's children:
+// left follows its parent, right follows the left subtree.
+__device__ __forceinline__ void child_indices(const TreeArgs& a, int t) {
+  const int l = a.left[t], r = a.right[t];
   if (l < 0) return;
   a.dfs[l] = a.dfs[t] + 1;
   a.dfs[r] = a.dfs[t] + 1 + a.size[l];
   a.idfs[l] = a.idfs[t] + 1;
   a.idfs[r] = a.idfs[t] + 1 + a.isize[l];
+}
+
+__global__ void __launch_bounds__(512) k_dfs(TreeArgs a, const int* tasks, int levels) {
+  for (int k = 0; k < levels; ++k) {
+    const LevelCount l = a.counters->lvl[k];
+    for (int i = threadIdx.x; i < l.tasks; i += blockDim.x) child_indices(a, tasks[l.base + i]);
+    __syncthreads();
+  }
+}
+
+// The same for the nodes that blocks built, one warp per block's list: levels from
+// the last up, then from the first down.
+__global__ void __launch_bounds__(128) k_mid_sizes(TreeArgs a, const int* mid_roots, const int* nodes, const int* ends) {
+  const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (w >= a.counters->mid_roots) return;
+  const int root = mid_roots[w];
+  nodes += a.first[root];
+  ends += static_cast<long long>(w) * kMaxLevels;
+  int n = 0;
+  while (n < kMaxLevels && ends[n] > 0) ++n;
+  for (int k = n - 1; k >= 0; --k) {
+    for (int i = (k ? ends[k - 1] : 0) + lane; i < ends[k]; i += 32) node_sizes(a, nodes[i]);
+    __syncwarp();
+  }
+}
+__global__ void __launch_bounds__(128) k_mid_dfs(TreeArgs a, const int* mid_roots, const int* nodes, const int* ends) {
+  const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (w >= a.counters->mid_roots) return;
+  const int root = mid_roots[w];
+  nodes += a.first[root];
+  ends += static_cast<long long>(w) * kMaxLevels;
+  for (int k = 0; k < kMaxLevels && ends[k] > 0; ++k) {
+    for (int i = (k ? ends[k - 1] : 0) + lane; i < ends[k]; i += 32) child_indices(a, nodes[i]);
+    __syncwarp();
+  }
 }
 
 // Nodes inside warp-built subtrees: offsets from their subtree root.
@@ -1284,7 +1685,9 @@ void gpu_bvh_preload() {
       reinterpret_cast<const void*>(k_bins),       reinterpret_cast<const void*>(k_decide),
       reinterpret_cast<const void*>(k_pcount),     reinterpret_cast<const void*>(k_pscan),
       reinterpret_cast<const void*>(k_pranks),     reinterpret_cast<const void*>(k_pswap),
-      reinterpret_cast<const void*>(k_small),      reinterpret_cast<const void*>(k_sizes),
+      reinterpret_cast<const void*>(k_small),      reinterpret_cast<const void*>(k_mid),
+      reinterpret_cast<const void*>(k_mid_sizes),  reinterpret_cast<const void*>(k_mid_dfs),
+      reinterpret_cast<const void*>(k_sizes),
       reinterpret_cast<const void*>(k_dfs),        reinterpret_cast<const void*>(k_small_dfs),
       reinterpret_cast<const void*>(k_finish),     reinterpret_cast<const void*>(k_wide_init),
       reinterpret_cast<const void*>(k_wide),       reinterpret_cast<const void*>(k_scan_block),
@@ -1323,7 +1726,7 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
   State& s = *st_;
   s.n = n;
   s.nn = 2 * n;
-  s.max_level_tasks = n / (kSmallItems + 1) + 2;
+  s.max_level_tasks = n / (kMidItems + 1) + 2;
   s.max_chunks = n / kChunk + s.max_level_tasks + 8;
 
   // Carve every scratch array out of one pool allocation.
@@ -1343,6 +1746,10 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
   add(s.first, nn);
   add(s.count, nn);
   add(s.small_roots, n);
+  const std::size_t max_mids = n / (kSmallItems + 1) + 1;
+  add(s.mid_roots, max_mids);
+  add(s.mid_nodes, n);
+  add(s.mid_ends, max_mids * kMaxLevels);
   for (int q = 0; q < 2; ++q) {
     add(s.bins[q], lt * kBinWords);
     for (int** p : {&s.task_chunk0[q], &s.task_nchunks[q], &s.need_part[q], &s.part_t[q], &s.part_m[q],
@@ -1353,6 +1760,7 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
     for (int** p : {&s.chunk_task[q], &s.cnt_lf[q], &s.cnt_rt[q], &s.base_lf[q], &s.base_rt[q]}) add(*p, mc);
     add(s.chunk_start[q], mc);
   }
+  add(s.moves, mc * (kChunk / 32));
   add(s.wide_list, n + 1);
   add(s.wide_kids, 4 * nn);
   add(s.wflag, nn);
@@ -1389,7 +1797,7 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
     if (host.error & 1) throw std::runtime_error("BVH leaf too large");
     if (host.error) throw std::runtime_error("device BVH build: inconsistent partition");
   };
-  auto level_args = [&](int parity, int lb, int nt, int nc) {
+  auto level_args = [&](int level) {
     LevelArgs a{};
     a.boxes = in.boxes;
     a.items = s.items;
@@ -1403,14 +1811,12 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
     a.depth = s.depth;
     a.axis = s.axis;
     a.sub = s.sub;
-    a.tasks_cur = s.tasks + lb;
-    a.tasks_next = s.tasks + lb + nt;
+    a.tasks = s.tasks;
+    a.mid_roots = s.mid_roots;
     a.small_roots = s.small_roots;
     a.counters = s.counters;
-    a.n_tasks = nt;
-    a.n_chunks = nc;
-    a.parity = parity;
-    const int p = parity, q = parity ^ 1;
+    a.level = level;
+    const int p = level & 1, q = p ^ 1;
     a.bins = s.bins[p];
     a.need_part = s.need_part[p];
     a.part_t = s.part_t[p];
@@ -1427,6 +1833,7 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
     a.cnt_rt = s.cnt_rt[p];
     a.base_lf = s.base_lf[p];
     a.base_rt = s.base_rt[p];
+    a.moves = s.moves;
     a.bins_next = s.bins[q];
     a.task_chunk0_next = s.task_chunk0[q];
     a.task_nchunks_next = s.task_nchunks[q];
@@ -1435,31 +1842,60 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
     return a;
   };
 
-  // The root lands in level 0 (parity 0) as a large node, or as a warp subtree.
-  k_init<<<1, 32, 0, stream_>>>(level_args(1, 0, 0, 0), n, s.dfs, s.idfs);
+  // Most tasks that a level can have, and their chunks.
+  auto level_tasks = [&](int level) {
+    return level < 30 ? std::min(1 << level, static_cast<int>(s.max_level_tasks)) : static_cast<int>(s.max_level_tasks);
+  };
+  auto level_chunks = [&](int level) {
+    return std::min(static_cast<int>(n / kChunk) + level_tasks(level), static_cast<int>(s.max_chunks));
+  };
+  // The root lands in level 0's arrays, which are an odd level's next.
+  k_init<<<1, 32, 0, stream_>>>(level_args(1), n, s.dfs, s.idfs);
   BVH_CK(cudaGetLastError());
-  read_counters();
-  int lb = 0, nt = host.lvl[0].tasks, nc = host.lvl[0].chunks;
-  for (int level = 0; nt > 0; ++level) {
-    if (level >= kMaxLevels) throw std::logic_error("device BVH build: too many levels");
-    const int p = level & 1;
-    const LevelArgs a = level_args(p, lb, nt, nc);
+  // A level has its largest node from at least n / 2^level primitives, so the first
+  // levels follow one another without a look at their sizes (a look costs 25 us).
+  int levels = 0, tasks = n > kMidItems ? 1 : 0;
+  while (tasks > 0) {
+    if (levels >= kMaxLevels - 1) throw std::logic_error("device BVH build: too many levels");
+    const LevelArgs a = level_args(levels);
+    const int nt = level_tasks(levels), nc = level_chunks(levels);
     k_bounds<<<blocks_for(32ll * nc, 128), 128, 0, stream_>>>(a);
     k_bins<<<blocks_for(nc, kWarpsPerBlock), kWarpsPerBlock * 32, 0, stream_>>>(a);
-    BVH_CK(cudaMemsetAsync(&s.counters->lvl[p ^ 1], 0, sizeof(LevelCount), stream_));
     k_decide<<<blocks_for(32ll * nt, 128), 128, 0, stream_>>>(a);
     k_pcount<<<blocks_for(32ll * nc, 128), 128, 0, stream_>>>(a);
     k_pscan<<<blocks_for(32ll * nt, 128), 128, 0, stream_>>>(a);
     k_pranks<<<blocks_for(32ll * nc, 128), 128, 0, stream_>>>(a);
     k_pswap<<<blocks_for(32ll * nc, 128), 128, 0, stream_>>>(a);
     BVH_CK(cudaGetLastError());
-    s.levels.push_back({lb, nt});
+    ++levels;
+    if (levels < 30 && (n >> levels) > static_cast<std::uint32_t>(kMidItems)) continue;
     read_counters();
-    lb += nt;
-    nt = host.lvl[p ^ 1].tasks;
-    nc = host.lvl[p ^ 1].chunks;
-    if (nt > static_cast<int>(s.max_level_tasks) || nc > static_cast<int>(s.max_chunks))
+    tasks = host.lvl[levels].tasks;
+    if (tasks > static_cast<int>(s.max_level_tasks) || host.lvl[levels].chunks > static_cast<int>(s.max_chunks))
       throw std::logic_error("device BVH build: level overflow");
+  }
+  const int mids = levels > 0 ? host.mid_roots : (n > kSmallItems ? 1 : 0);
+  if (mids > 0) {
+    MidArgs ma{};
+    ma.boxes = in.boxes;
+    ma.items = s.items;
+    ma.box = s.box;
+    ma.left = s.left;
+    ma.right = s.right;
+    ma.first = s.first;
+    ma.count = s.count;
+    ma.depth = s.depth;
+    ma.axis = s.axis;
+    ma.sub = s.sub;
+    ma.mid_roots = s.mid_roots;
+    ma.mid_nodes = s.mid_nodes;
+    ma.mid_ends = s.mid_ends;
+    ma.small_roots = s.small_roots;
+    ma.counters = s.counters;
+    // Set on every build: the attribute belongs to the device that is current.
+    BVH_CK(cudaFuncSetAttribute(k_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(MidBlock))));
+    k_mid<<<mids, kMidWarps * 32, sizeof(MidBlock), stream_>>>(ma);
+    BVH_CK(cudaGetLastError());
   }
 
   SmallArgs sa{};
@@ -1478,9 +1914,8 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
   sa.local = s.local;
   sa.ilocal = s.ilocal;
   sa.small_roots = s.small_roots;
-  sa.n_small = host.small_roots;
   sa.counters = s.counters;
-  if (sa.n_small > 0) k_small<<<blocks_for(sa.n_small, kWarpsPerBlock), kWarpsPerBlock * 32, 0, stream_>>>(sa);
+  k_small<<<std::min(blocks_for(n, kWarpsPerBlock), 148 * 6), kWarpsPerBlock * 32, 0, stream_>>>(sa);
 
   TreeArgs ta{};
   ta.box = s.box;
@@ -1497,9 +1932,12 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
   ta.local = s.local;
   ta.ilocal = s.ilocal;
   ta.counters = s.counters;
-  for (auto it = s.levels.rbegin(); it != s.levels.rend(); ++it)
-    k_sizes<<<blocks_for(it->second, 128), 128, 0, stream_>>>(ta, s.tasks + it->first, it->second);
-  for (const auto& lv : s.levels) k_dfs<<<blocks_for(lv.second, 128), 128, 0, stream_>>>(ta, s.tasks + lv.first, lv.second);
+  if (mids > 0) k_mid_sizes<<<blocks_for(32ll * mids, 128), 128, 0, stream_>>>(ta, s.mid_roots, s.mid_nodes, s.mid_ends);
+  if (levels > 0) {
+    k_sizes<<<1, 512, 0, stream_>>>(ta, s.tasks, levels);
+    k_dfs<<<1, 512, 0, stream_>>>(ta, s.tasks, levels);
+  }
+  if (mids > 0) k_mid_dfs<<<blocks_for(32ll * mids, 128), 128, 0, stream_>>>(ta, s.mid_roots, s.mid_nodes, s.mid_ends);
   k_small_dfs<<<blocks_for(s.nn, 256), 256, 0, stream_>>>(ta, static_cast<int>(s.nn));
   k_finish<<<1, 32, 0, stream_>>>(ta);
   BVH_CK(cudaGetLastError());
@@ -1527,7 +1965,7 @@ GpuBvhCounts GpuBvhBuilder::build(const GpuBvhInput& in) {
   counts_.leaves = host.leaves;
   counts_.max_leaf = host.max_leaf;
   counts_.max_depth = host.max_depth;
-  counts_.levels = static_cast<std::int32_t>(s.levels.size());
+  counts_.levels = levels;
   int wide = 0, depth4 = 0;
   for (int w = 0; w < kMaxLevels; ++w) {
     wide += host.wide_cnt[w];
