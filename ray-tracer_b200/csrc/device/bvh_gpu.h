@@ -38,6 +38,22 @@ struct GpuBvhInput {
   const std::uint32_t* material = nullptr; // 1 per primitive
 };
 
+// A primitive as the host stages it: a sphere's centre and, in v[3], radius; a triangle's
+// corners.
+struct RawPrim {
+  double v[9];
+  std::uint32_t material;  // top bit: the triangle has vertex normals
+  std::uint32_t sphere;
+};
+
+// The build's inputs for primitives first .. first + n - 1, from their records and, of
+// those that have them, vertex normals (9 floats each): boxes as Prim::bounds makes them,
+// the rest as slot_record (flatten.hpp) does, bit for bit. `items`, unless null, takes the
+// ids. The arrays written are indexed by primitive id; raw and normals by id - first.
+cudaError_t convert_prims(const RawPrim* raw, const float* normals, std::uint32_t first, std::uint32_t n, double* boxes,
+                          float4* rows, float4* row_normals, std::uint32_t* material, std::uint32_t* items,
+                          cudaStream_t stream);
+
 // What the build found; the caller sizes the layout arrays from it.
 struct GpuBvhCounts {
   std::int32_t interior = 0;  // DevNode records
@@ -70,8 +86,7 @@ class GpuBvhBuilder {
   GpuBvhBuilder(const GpuBvhBuilder&) = delete;
   GpuBvhBuilder& operator=(const GpuBvhBuilder&) = delete;
 
-  // Builds the tree and its four-wide collapse; synchronises the stream once per
-  // level of large nodes and at the end. Throws std::runtime_error on a leaf of
+  // Builds the tree and its four-wide collapse; synchronises the stream a few times. Throws std::runtime_error on a leaf of
   // more than 65535 primitives or a tree deeper than the traversal stack allows.
   GpuBvhCounts build(const GpuBvhInput& in);
 

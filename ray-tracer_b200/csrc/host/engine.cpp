@@ -442,77 +442,116 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
   FlatScene tables;
   flatten_tables(s, tables);
 
-  // Inputs in primitive order, converted on the host cores into one pinned buffer:
-  // boxes (double), slot rows, normals, material words, the ids of primitives
-  // with a usable box, then the tables. One copy takes them all to the GPU.
+  // The primitives' records, packed by the host's threads into pinned memory, and the
+  // tables. Pieces cross the bus, and are converted there, while the next are packed.
   auto pad = [](std::size_t bytes) { return (std::max<std::size_t>(bytes, 1) + 255) & ~std::size_t(255); };
-  const std::size_t in_bytes[8] = {np * 6 * sizeof(double), np * 3 * sizeof(float4), np * 3 * sizeof(float4),
-                                   np * sizeof(std::uint32_t), np * sizeof(std::uint32_t),
+  const std::size_t in_bytes[6] = {np * sizeof(RawPrim), np * 9 * sizeof(float), np * sizeof(std::uint32_t),
                                    tables.planes.size() * sizeof(DevPlane),
                                    tables.materials.size() * sizeof(DevMaterial),
                                    tables.lights.size() * sizeof(DevLight)};
-  std::size_t in_at[9];
+  std::size_t in_at[7];
   in_at[0] = 0;
-  for (int k = 0; k < 8; ++k) in_at[k + 1] = in_at[k] + pad(in_bytes[k]);
-  const std::size_t staged = in_at[8];
+  for (int k = 0; k < 6; ++k) in_at[k + 1] = in_at[k] + pad(in_bytes[k]);
+  const std::size_t staged = in_at[6];
   int b = 0;
   unsigned char* host = upload_staging(staged, b);
-  auto* boxes = reinterpret_cast<double*>(host + in_at[0]);
-  auto* rows = reinterpret_cast<float4*>(host + in_at[1]);
-  auto* normals = reinterpret_cast<float4*>(host + in_at[2]);
-  auto* material = reinterpret_cast<std::uint32_t*>(host + in_at[3]);
-  auto* items = reinterpret_cast<std::uint32_t*>(host + in_at[4]);
-  std::vector<std::uint8_t> usable(np);
-  {
-    const std::size_t workers = std::min<std::size_t>({16, std::max(1u, std::thread::hardware_concurrency()),
-                                                       (np + 16383) / 16384});
-    auto body = [&](std::size_t i0, std::size_t i1) {
-      for (std::size_t i = i0; i < i1; ++i) {
-        const Prim& p = s.prims[i];
-        const Box bx = p.bounds();
-        double* d = boxes + 6 * i;
-        d[0] = bx.lo.x; d[1] = bx.lo.y; d[2] = bx.lo.z;
-        d[3] = bx.hi.x; d[4] = bx.hi.y; d[5] = bx.hi.z;
-        usable[i] = !(bx.empty() || !bx.lo.finite() || !bx.hi.finite());
-        slot_record(p, static_cast<std::uint32_t>(i), rows + 3 * i, normals + 3 * i, material[i]);
-      }
-    };
-    std::vector<std::thread> pool;
-    const std::size_t chunk = workers > 1 ? (np + workers - 1) / workers : np;
-    for (std::size_t w = 1; w < workers; ++w)
-      pool.emplace_back(body, std::min(np, w * chunk), std::min(np, (w + 1) * chunk));
-    body(0, std::min(np, chunk));
-    for (auto& t : pool) t.join();
-  }
-  std::uint32_t n_items = 0;
-  for (std::size_t i = 0; i < np; ++i)
-    if (usable[i]) items[n_items++] = static_cast<std::uint32_t>(i);
-  std::memcpy(host + in_at[5], tables.planes.data(), in_bytes[5]);
-  std::memcpy(host + in_at[6], tables.materials.data(), in_bytes[6]);
-  std::memcpy(host + in_at[7], tables.lights.data(), in_bytes[7]);
+  auto* raw = reinterpret_cast<RawPrim*>(host + in_at[0]);
+  auto* normals = reinterpret_cast<float*>(host + in_at[1]);
+  auto* items = reinterpret_cast<std::uint32_t*>(host + in_at[2]);
 
-  // Device copy of the inputs plus room for the slot -> primitive map.
+  // Device copy of all that, and what the build takes: boxes (double), slot rows, normals,
+  // material words; then room for the slot -> primitive map.
+  const std::size_t made_bytes[5] = {np * 6 * sizeof(double), np * 3 * sizeof(float4), np * 3 * sizeof(float4),
+                                     np * sizeof(std::uint32_t), np * sizeof(std::uint32_t)};
+  std::size_t made_at[6];
+  made_at[0] = staged;
+  for (int k = 0; k < 5; ++k) made_at[k + 1] = made_at[k] + pad(made_bytes[k]);
   void* in_block = nullptr;
   count_allocation();
-  CK(cudaMallocFromPoolAsync(&in_block, staged + pad(np * sizeof(std::uint32_t)), pool_, build_stream_));
+  CK(cudaMallocFromPoolAsync(&in_block, made_at[5], pool_, build_stream_));
   struct FreeInput {
     void* p;
     cudaStream_t s;
     ~FreeInput() { cudaFreeAsync(p, s); }
   } free_input{in_block, build_stream_};
   auto* dev_in = static_cast<unsigned char*>(in_block);
-  CK(cudaMemcpyAsync(dev_in, host, staged, cudaMemcpyHostToDevice, build_stream_));
-  CK(cudaEventRecord(upload_ev_[b], build_stream_));
-  upload_pending_[b] = true;
-  auto* order = reinterpret_cast<std::uint32_t*>(dev_in + staged);
+  auto send = [&](std::size_t at, std::size_t bytes) {
+    if (!bytes) return;
+    CK(cudaMemcpyAsync(dev_in + at, host + at, bytes, cudaMemcpyHostToDevice, build_stream_));
+    CK(cudaEventRecord(upload_ev_[b], build_stream_));
+    upload_pending_[b] = true;
+  };
+  auto* boxes = reinterpret_cast<double*>(dev_in + made_at[0]);
+  auto* rows = reinterpret_cast<float4*>(dev_in + made_at[1]);
+  auto* row_normals = reinterpret_cast<float4*>(dev_in + made_at[2]);
+  auto* material = reinterpret_cast<std::uint32_t*>(dev_in + made_at[3]);
+  auto* order = reinterpret_cast<std::uint32_t*>(dev_in + made_at[4]);
+  auto* dev_items = reinterpret_cast<std::uint32_t*>(dev_in + in_at[2]);
+
+  std::vector<std::uint8_t> usable(np);
+  std::atomic<bool> all_usable{true};
+  constexpr std::size_t kPiece = 32768, kTask = 2048;
+  for (std::size_t p0 = 0; p0 < np; p0 += kPiece) {
+    const std::size_t count = std::min(kPiece, np - p0);
+    std::atomic<bool> smooth{false};
+    host_pool_.run((count + kTask - 1) / kTask, [&](std::size_t task) {
+      bool any_smooth = false, all = true;
+      const std::size_t end = p0 + std::min(count, (task + 1) * kTask);
+      for (std::size_t i = p0 + task * kTask; i < end; ++i) {
+        const Prim& p = s.prims[i];
+        const Box bx = p.bounds();
+        usable[i] = !(bx.empty() || !bx.lo.finite() || !bx.hi.finite());
+        all = all && usable[i];
+        const bool sphere = p.kind == Prim::kSphere, has_normals = !sphere && p.smooth;
+        RawPrim r;
+        const D3 corners[3] = {p.a, p.b, p.c};
+        for (int k = 0; k < 3; ++k) {
+          r.v[3 * k] = corners[k].x;
+          r.v[3 * k + 1] = corners[k].y;
+          r.v[3 * k + 2] = corners[k].z;
+        }
+        r.material = p.material | (has_normals ? 0x80000000u : 0u);
+        r.sphere = sphere ? 1u : 0u;
+        raw[i] = r;
+        if (has_normals) {
+          any_smooth = true;
+          const D3 n[3] = {p.n0, p.n1, p.n2};
+          for (int k = 0; k < 3; ++k) {
+            normals[9 * i + 3 * k] = float(n[k].x);
+            normals[9 * i + 3 * k + 1] = float(n[k].y);
+            normals[9 * i + 3 * k + 2] = float(n[k].z);
+          }
+        }
+      }
+      if (any_smooth) smooth.store(true, std::memory_order_relaxed);
+      if (!all) all_usable.store(false, std::memory_order_relaxed);
+    });
+    send(in_at[0] + p0 * sizeof(RawPrim), count * sizeof(RawPrim));
+    if (smooth.load()) send(in_at[1] + p0 * 9 * sizeof(float), count * 9 * sizeof(float));
+    CK(convert_prims(reinterpret_cast<const RawPrim*>(dev_in + in_at[0]) + p0,
+                     reinterpret_cast<const float*>(dev_in + in_at[1]) + 9 * p0, static_cast<std::uint32_t>(p0),
+                     static_cast<std::uint32_t>(count), boxes, rows, row_normals, material, dev_items, build_stream_));
+  }
+  std::uint32_t n_items = static_cast<std::uint32_t>(np);
+  if (!all_usable.load()) {
+    // The ids of primitives with a usable box.
+    n_items = 0;
+    for (std::size_t i = 0; i < np; ++i)
+      if (usable[i]) items[n_items++] = static_cast<std::uint32_t>(i);
+    send(in_at[2], n_items * sizeof(std::uint32_t));
+  }
+  std::memcpy(host + in_at[3], tables.planes.data(), in_bytes[3]);
+  std::memcpy(host + in_at[4], tables.materials.data(), in_bytes[4]);
+  std::memcpy(host + in_at[5], tables.lights.data(), in_bytes[5]);
+  send(in_at[3], staged - in_at[3]);
 
   GpuBvhInput in;
   in.n_items = n_items;
-  in.boxes = reinterpret_cast<const double*>(dev_in + in_at[0]);
-  in.rows = reinterpret_cast<const float4*>(dev_in + in_at[1]);
-  in.normals = reinterpret_cast<const float4*>(dev_in + in_at[2]);
-  in.material = reinterpret_cast<const std::uint32_t*>(dev_in + in_at[3]);
-  in.items = reinterpret_cast<const std::uint32_t*>(dev_in + in_at[4]);
+  in.boxes = boxes;
+  in.rows = rows;
+  in.normals = row_normals;
+  in.material = material;
+  in.items = dev_items;
   GpuBvhBuilder builder(build_stream_, pool_);
   const GpuBvhCounts c = builder.build(in);
 
@@ -579,7 +618,7 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
   const std::size_t part_bytes[kSceneParts] = {
       std::size_t(c.interior) * sizeof(DevNode), std::size_t(c.wide) * sizeof(DevNode4),
       std::size_t(n_items) * 3 * sizeof(float4), std::size_t(n_items) * sizeof(std::uint32_t),
-      std::size_t(n_items) * 3 * sizeof(float4), in_bytes[5], in_bytes[6], in_bytes[7],
+      std::size_t(n_items) * 3 * sizeof(float4), in_bytes[3], in_bytes[4], in_bytes[5],
       w8.nodes.size() * sizeof(DevNode8)};
   std::size_t at[kSceneParts], total = 0;
   for (int k = 0; k < kSceneParts; ++k) {
@@ -628,7 +667,7 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
         CK(cudaMemcpyAsync(dst + at[k], sb + sat[k], part_bytes[k], cudaMemcpyDeviceToDevice, build_stream_));
   }
   for (int k = 5; k < 8; ++k)
-    if (part_bytes[k]) CK(cudaMemcpyAsync(dst + at[k], dev_in + in_at[k], part_bytes[k], cudaMemcpyDeviceToDevice, build_stream_));
+    if (part_bytes[k]) CK(cudaMemcpyAsync(dst + at[k], dev_in + in_at[k - 2], part_bytes[k], cudaMemcpyDeviceToDevice, build_stream_));
   CK(cudaStreamSynchronize(build_stream_));
   gs->slot_prim.resize(n_items);
   for (std::size_t k = 0; k < n_items; ++k) gs->slot_prim[k] = prim_of_slot[w8.old_of[k]];
