@@ -350,6 +350,9 @@ class Engine {
   std::unique_ptr<Wave> wave_;
   std::vector<GpuFrame> frames_;  // frames of the last render / batch
   std::vector<int> rendering_;    // handles of the render / batch in progress (pass callbacks read these)
+  // Jobs one after the other instead of pass by pass: a batch of which nothing can be seen
+  // before its end (no callback, no cancel word).
+  bool job_order_ = false;
   std::vector<RenderSettings> frame_settings_;
   RenderStats stats_;
   std::map<int, Job> jobs_;        // open jobs by handle
