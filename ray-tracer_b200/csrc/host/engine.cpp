@@ -1537,7 +1537,9 @@ void Engine::read_moments(int job, double* sum, double* sumsq, std::uint32_t* co
     std::size_t bytes;
   };
   std::vector<Part> parts;
+  std::vector<std::pair<void*, std::size_t>> buffers;
   auto add = [&](void* to, const void* from, std::size_t bytes) {
+    if (to) buffers.emplace_back(to, bytes);
     for (std::size_t at = 0; to && at < bytes; at += kSlotBytes)
       parts.push_back({static_cast<unsigned char*>(to) + at, static_cast<const unsigned char*>(from) + at,
                        std::min(kSlotBytes, bytes - at)});
@@ -1548,6 +1550,7 @@ void Engine::read_moments(int job, double* sum, double* sumsq, std::uint32_t* co
   pieces(parts.size(),
          [&](std::size_t k, unsigned char* mem) {
            CK(cudaMemcpyAsync(mem, parts[k].from, parts[k].bytes, cudaMemcpyDeviceToHost, stream_));
+           if (k == 0) host_pool_.touch(buffers);
          },
          [&](std::size_t k, const unsigned char* mem) { host_pool_.copy(parts[k].to, mem, parts[k].bytes); });
 }
@@ -1567,6 +1570,7 @@ void Engine::read_mean_frame(const GpuFrame& f, double* rgb) {
            const std::size_t at = k * kPixels;
            CK(launch_resolve(f.sum + 4 * at, f.count + at, size(k), 0, 1.0, nullptr, reinterpret_cast<double*>(mem),
                              stream_));
+           if (k == 0) host_pool_.touch({{rgb, px * 3 * sizeof(double)}});
          },
          [&](std::size_t k, const unsigned char* mem) {
            host_pool_.copy(rgb + 3 * k * kPixels, mem, size(k) * 3 * sizeof(double));
@@ -1586,8 +1590,10 @@ void Engine::read_image_list(const std::vector<ImageRead>& list) {
   std::vector<std::vector<Part>> loads;
   static_assert(2 * kPixels * 3 + 256 <= kSlotBytes, "a piece fits its slot");
   std::size_t used = 0;
+  std::vector<std::pair<void*, std::size_t>> buffers;
   for (const ImageRead& r : list) {
     const std::size_t px = std::size_t(r.frame->width) * r.frame->height;
+    buffers.emplace_back(r.rgb, 3 * px);
     for (std::size_t first = 0; first < px;) {
       if (loads.empty() || used >= 3 * kPixels) {
         loads.emplace_back();
@@ -1604,6 +1610,7 @@ void Engine::read_image_list(const std::vector<ImageRead>& list) {
            for (const Part& p : loads[k])
              CK(launch_resolve(p.image->frame->sum + 4 * p.first, p.image->frame->count + p.first, p.pixels,
                                static_cast<int>(p.image->op), p.image->exposure, mem + p.at, nullptr, stream_));
+           if (k == 0) host_pool_.touch(buffers);
          },
          [&](std::size_t k, const unsigned char* mem) {
            if (loads[k].size() == 1) {

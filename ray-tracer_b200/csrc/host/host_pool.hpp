@@ -6,10 +6,12 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstddef>
+#include <cstdint>
 #include <cstring>
 #include <functional>
 #include <mutex>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace rtg {
@@ -61,6 +63,31 @@ class HostPool {
       const std::size_t at = k * kPiece;
       std::memcpy(static_cast<unsigned char*>(dst) + at, static_cast<const unsigned char*>(src) + at,
                   std::min(kPiece, bytes - at));
+    });
+  }
+
+  // Writes a byte to every page of buffers that are about to be filled, when they are
+  // large: fresh memory (an allocation that malloc maps anew each time) is then zeroed
+  // by all threads at once, each in huge pages of its own. Left to the copies, which work
+  // on a few megabytes at a time, two or three threads zero and the others wait (64 images,
+  // 58 MB: 9.2 ms, with this 5.0).
+  void touch(const std::vector<std::pair<void*, std::size_t>>& buffers) {
+    constexpr std::uintptr_t kHuge = std::uintptr_t(1) << 21, kPage = 4096;
+    std::size_t total = 0;
+    for (const auto& b : buffers) total += b.second;
+    if (total < (std::size_t(16) << 20)) return;
+    std::vector<std::pair<std::uintptr_t, std::uintptr_t>> parts;
+    for (const auto& b : buffers) {
+      const std::uintptr_t end = reinterpret_cast<std::uintptr_t>(b.first) + b.second;
+      for (std::uintptr_t at = reinterpret_cast<std::uintptr_t>(b.first); at < end;) {
+        const std::uintptr_t next = std::min(end, (at | (kHuge - 1)) + 1);
+        parts.emplace_back(at, next);
+        at = next;
+      }
+    }
+    run(parts.size(), [&parts](std::size_t k) {
+      for (std::uintptr_t at = parts[k].first; at < parts[k].second; at = (at | (kPage - 1)) + 1)
+        *reinterpret_cast<volatile unsigned char*>(at) = 0;
     });
   }
 
