@@ -249,9 +249,9 @@ int rtg_framebuffer_moments(rtg_context* ctx, int32_t job, double* sum, double* 
  * tone_map < 0 uses the render's settings (normals: clamp, exposure 1). */
 int rtg_image_rgb8(rtg_context* ctx, int32_t job, int32_t tone_map, double exposure, uint8_t* rgb);
 /* rtg_image_rgb8 for n jobs at once (no reference counterpart; Renderer::image
- * per job): image of jobs[k] into rgb[k]. All images are resolved on the device,
- * copied to the host in one transfer with one synchronisation, then copied out on
- * the host cores. tone_map and exposure as rtg_image_rgb8, for every job. */
+ * per job): image of jobs[k] into rgb[k]. The images are resolved on the device and
+ * cross in pieces through pinned buffers, from which the host cores copy them out
+ * while the next pieces are on their way. tone_map and exposure as rtg_image_rgb8, for every job. */
 int rtg_images_rgb8(rtg_context* ctx, int32_t n, const int32_t* jobs, int32_t tone_map, double exposure,
                     uint8_t* const* rgb);
 int rtg_render_stats(rtg_context* ctx, rtg_stats* out);
@@ -320,7 +320,8 @@ typedef struct rtg_tuning {
                               * (default 1); 0: the fp32 traversal's own t, the value the renderer's
                               * closest-hit stage hands to shading */
   int32_t closest_tree;      /* closest-hit walk: 2 the binary tree (default), 8 the compressed eight-wide tree */
-  int32_t shadow_tree;       /* any-hit walk: 4 the four-wide tree (default), 8 the compressed eight-wide tree.
+  int32_t shadow_tree;       /* any-hit walk: 4 (default) the four-wide tree for rtg_trace_any and small direct
+                              * renders, the binary tree for the rest; 8 the compressed eight-wide tree.
                               * Scenes get the eight-wide tree (and its slot order) when they are uploaded
                               * while either walk is 8; rendering or querying a scene without it with an
                               * eight-wide walk selected returns RTG_ERR_INVALID. */

@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
 // of every path moved some 300 bytes and every stage waited for its slowest warp
 // (36 us of fixed cost an iteration on the sphere field, 160 us on the mesh). On
 // B200, device time before and after, default pool: Cornell 256x256x64 2595 and
-// 1960 us, sphere field 640x360x64 4446 and 2850 us; pool of 2^23: sphere field
-// 512x512x128 8250 and 5970 us, mesh 1024x1024x64 52.9 and 50.5 ms, 16 scenes of the
-// mix 123.2 and 115.0 ms.
+// 1940 us, sphere field 640x360x64 4446 and 2790 us; pool of 2^23: sphere field
+// 512x512x128 8250 and 5970 us, mesh 1024x1024x64 52.9 and 50.2 ms, 16 scenes of the
+// mix 123.2 and 110.7 ms.
 //
 // What bounds it: instruction issue (73% of the slots on Cornell) under divergence
 // (11 to 16 of 32 lanes active in the walks), then the walks' dependent loads.
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kMaxGen) k_plan(WaveBuffers wb, int par) {
 // - Instruction cache: closest-hit and shadow rays share one copy of the walk, and
 //   what only some jobs need is in other instances. With a copy each (and the
 //   four-wide walk for shadow rays), warps in different steps evict each other's
-//   loops: 2.1 of 9.5 cycles per instruction went to fetching, now 0.4.
+//   loops: 2.1 of 9.5 cycles per instruction went to fetching, now 0.5 to 0.9.
 constexpr int kWarpPaths = 56;
 // Least paths a warp takes at once where there are too few for full batches: 4 and 8
 // measure alike, 16 loses half of the gain (mesh 64x64x1: 465 us with full batches only,

@@ -32,9 +32,10 @@ struct alignas(16) DevNode {
 // Four-child BVH node, collapsed from the binary tree (same leaves): the four
 // children's boxes as SoA float4s (component k is child k), then their links with
 // the same meaning as DevNode's; an unused child has kNoChild. One 128-byte node
-// replaces up to three binary nodes. Any-hit (shadow) queries walk this tree: they
-// stop at the first hit, so a wide node's four tests pay off; closest-hit queries
-// walk the binary tree, which measured faster for them.
+// replaces up to three binary nodes. Occlusion queries and small direct renders walk
+// this tree: they stop at the first hit, so a wide node's four tests pay off. The path
+// kernel and the warp-scheduled direct kernel take shadow rays through the binary walk
+// that their closest hits use: a second walk's code costs them more than it saves.
 struct alignas(16) DevNode4 {
   float4 lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;
   int4 link;

@@ -1,10 +1,11 @@
 // Closest-hit ray query for callers that must not allocate device memory.
 //
-// rtg_trace_closest stages its rays, its results and the scene descriptor in
-// buffers it cudaMallocs and cudaFrees on every call. Some callers cannot do
-// that: a render loop sharing the GPU with other streams (cudaFree synchronises
-// the whole device), or a host that reserves all device memory up front in its
-// own pool and forbids further allocations. This variant keeps every byte it
+// rtg_trace_closest stages its rays and results in pinned buffers that its context
+// allocates when they are first needed, takes the scene descriptor's memory from a
+// stream-ordered pool, and uploads the scene's double copy on its first query. Some
+// callers cannot have that in a call: a render loop sharing the GPU with other streams
+// (an allocation may synchronise the whole device), or a host that reserves all device
+// memory up front in its own pool and forbids further allocations. This variant keeps every byte it
 // needs in one file-scope device array, sized for kNoAllocMaxRays rays, that the
 // CUDA module reserves on each GPU where it is loaded (with lazy module loading:
 // at this file's first use on that GPU) and that stays until the process exits.

@@ -532,7 +532,7 @@ class Context:
 
     def images(self, jobs: Sequence[int], sizes: Sequence[tuple], tone_map: Optional[str] = None,
                exposure: float = 1.0) -> list:
-        """image() of several jobs at once (one device-to-host transfer): sizes[k] is
+        """image() of several jobs at once (resolved and read back together): sizes[k] is
         (width, height) of jobs[k]. The images are views into one allocation, which
         the library fills in one pass (many small arrays each fault in their own
         fresh pages: 9.1 against 5.6 ms for the 64 images of the mix)."""
