@@ -205,7 +205,9 @@ __device__ __forceinline__ float3 spawn_point(float3 p, float3 n) {
 }
 // Spawn for direction `dir` from a surface with geometric normal `gn`.
 __device__ __forceinline__ float3 spawn_towards(float3 p, float3 gn, float3 dir) {
-  return spawn_point(p, dot3(dir, gn) > 0.f ? gn : -gn);
+  // dot3p: a direction in the surface's plane (total reflection's edge) leaves on the side
+  // that this form's rounding says, as it always has.
+  return spawn_point(p, dot3p(dir, gn) > 0.f ? gn : -gn);
 }
 
 // The reference's shadow-ray shortening distance is 4 * 1.6e-6 * max(1, |p|inf)
