@@ -106,6 +106,7 @@ struct Engine::Wave {
   cudaEvent_t tev[10]{};
   std::uint64_t it = 0;                // iterations launched (the device's `iteration`)
   std::uint64_t seen = 0;              // next snapshot to read: the one plan(seen) wrote
+  std::uint64_t counters_it = 0;       // older snapshots than this iteration's lag behind last_counters_
   std::uint64_t rad_cap = 0;
   std::map<std::uint64_t, std::uint64_t> rad_free;  // free radiance ranges: begin -> length
   std::vector<int> free_jobs;          // descriptor slots, popped from the back
@@ -1031,7 +1032,7 @@ bool Engine::run_direct_passes(Job& j) {
         CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
         stats_.direct_ms += ms;
       }
-      CK(cudaMemcpy(&last_counters_, W.wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+      read_counters();
       if (last_counters_.error)
         throw CudaFailure("device error flag " + std::to_string(last_counters_.error) +
                           (last_counters_.error == 2 ? " (direct integrator branch stack overflow)" : ""));
@@ -1160,7 +1161,9 @@ void Engine::process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events
     throw CudaFailure("device error flag " + std::to_string(e) +
                       (e == 3 ? " (generation table names segment slot " + std::to_string(S.c.error_info) + ")" : ""));
   }
-  last_counters_ = S.c;
+  // A snapshot planned before the counters were last read from the device would take a
+  // direct launch's rays back.
+  if (iter >= W.counters_it) last_counters_ = S.c;
   std::uint64_t done_sum = 0;
   bool open = false;
   int max_depth = 1;
@@ -1288,19 +1291,26 @@ void Engine::abort_all() {
   write_gen_table();
 }
 
+// The counters as they are: for a stream without work in flight.
+void Engine::read_counters() {
+  CK(cudaMemcpy(&last_counters_, wave_->wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+  wave_->counters_it = wave_->it;
+}
+
 void Engine::begin_stats() {
   stats_ = RenderStats{};
   CK(cudaStreamSynchronize(stream_));
-  if (!counters_final_) CK(cudaMemcpy(&last_counters_, wave_->wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+  if (!counters_final_) read_counters();
   base_counters_ = last_counters_;
   CK(cudaEventRecord(ev_begin_, stream_));
 }
 
 void Engine::end_stats(bool cancelled) {
   finish_timing();
-  // Every path had ended when the last snapshot was taken, so its counters are final;
-  // only a cancelled render leaves paths behind it.
-  if (cancelled) CK(cudaMemcpy(&last_counters_, wave_->wb.cnt, sizeof(last_counters_), cudaMemcpyDeviceToHost));
+  // Every path had ended when the last snapshot was taken and direct launches are read
+  // after they ran, so the latest of the two is final; only a cancelled render leaves
+  // paths behind it.
+  if (cancelled) read_counters();
   counters_final_ = true;
   const WaveCounters& end = last_counters_;
   if (end.error) throw CudaFailure("device error flag " + std::to_string(end.error));

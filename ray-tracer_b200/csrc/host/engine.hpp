@@ -300,6 +300,7 @@ class Engine {
   void abort_all();                 // drop every open segment (after a cancel) and reset the pool
   void stage(void* dst, const void* src, std::size_t n);
   void write_gen_table();
+  void read_counters();
   void begin_stats();
   RtgSceneDev* upload_descriptor(const RtgSceneDev& d);
   void end_stats(bool cancelled);
@@ -363,7 +364,7 @@ class Engine {
   int mis_jobs_ = 0;               // open jobs with multiple importance sampling
   int brute_jobs_ = 0;             // open jobs without a BVH (use_bvh = false)
   bool gen_dirty_ = false;
-  WaveCounters last_counters_{};   // from the latest snapshot
+  WaveCounters last_counters_{};   // from the latest snapshot or direct launch
   WaveCounters base_counters_{};   // at the start of the current render
   const volatile std::int32_t* cancel_ = nullptr;  // of the render in progress
   bool counters_final_ = false;    // last_counters_ are the device's: nothing has run since
