@@ -224,13 +224,14 @@ constexpr std::uint32_t kMinBatch = 4;
 
 constexpr std::uint32_t kPathSpecular = 1u << 12;   // last bounce was specular (or the path is new)
 constexpr std::uint32_t kPathContinues = 1u << 13;  // goes on after its shadow ray
+constexpr std::uint32_t kPathApart = 1u << 14;      // its shadow ray has an origin of its own, in the radiance slot
 constexpr int kPathSegShift = 16;                   // low 12 bits: depth; 16 and up: segment slot
 static_assert(kMaxSegments <= 1 << 16, "the segment slot does not fit the path word");
 
 // One warp's path slots, one 4-byte column per field.
 template <bool kMis>
 struct alignas(16) WarpPaths {
-  float o[3][kWarpPaths];       // ray origin (and the shadow ray's: both leave the hit on the same side)
+  float o[3][kWarpPaths];       // ray origin (and the shadow ray's, unless the path is marked kPathApart)
   float d[3][kWarpPaths];
   float beta[3][kWarpPaths];    // throughput
   float light[3][kWarpPaths];   // radiance so far
@@ -366,7 +367,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
       on = lane < take;
       if (on) {
         p = S.lit[n_lit + lane];
-        o = get3(S.o, p);
+        o = S.meta[p] & kPathApart ? f3(wb.radiance[S.sample[p]]) : get3(S.o, p);
         d = get3(S.sh_d, p);
         tmax = S.sh_tmax[p];
         job = S.job[p];
@@ -493,6 +494,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
             // needs the registers.
             set3(S.o, p, spawn_towards(s.p, s.gn, sr.dir));
             set3(S.d, p, sr.dir);
+            std::uint32_t apart = 0;
             if (J.light_sampling && !sr.specular && J.n_lights > 0) {
               const std::uint32_t nl = static_cast<std::uint32_t>(J.n_lights);
               const LightSample ls = sample_light(J.lights + rng.below(nl), s, rng);
@@ -500,9 +502,17 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
                 // Only a Lambertian scatter is non-specular: its weight is the albedo.
                 const float3 f = lambert_cos(sr.weight, s, ls.wi);
                 if (!is_zero3(f) && !is_zero3(ls.li_over_pdf)) {
-                  // Its origin is the one stored above: a Lambertian scatter leaves,
-                  // and lambert_cos is non-zero, on the side of s.gn only.
+                  // Its origin is mostly the one stored above: a Lambertian scatter
+                  // leaves, and lambert_cos is non-zero, on the side of s.gn. But
+                  // spawn_towards rounds in another way than those tests: of a direction
+                  // in the surface's plane it may find the other side. The origin
+                  // then waits in the radiance slot, which is written when the path ends.
                   const ShadowRay sray = shadow_ray(s, ls);
+                  const float3 oo = get3(S.o, p);
+                  if (sray.o.x != oo.x || sray.o.y != oo.y || sray.o.z != oo.z) {
+                    apart = kPathApart;
+                    wb.radiance[S.sample[p]] = make_float4(sray.o.x, sray.o.y, sray.o.z, 0.f);
+                  }
                   float w = 1.f;  // a point light (pdf 0) cannot be hit by BSDF sampling
                   if (kMis && J.light_sampling == 2 && ls.pdf > 0.f)
                     w = power_heuristic(ls.pdf / static_cast<float>(nl), __fmul_rn(dot3(s.n, ls.wi), kInvPiF));
@@ -533,7 +543,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
               // Cosine-hemisphere pdf of this bounce, for the MIS weight at the next hit.
               if (kMis && J.light_sampling == 2 && !sr.specular) S.pdf[kMis ? p : 0] = __fmul_rn(dot3p(s.n, sr.dir), kInvPiF);
             }
-            S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u);
+            S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u) | apart;
           }
         }
       }
