@@ -978,9 +978,13 @@ bool Engine::run_direct_passes(Job& j) {
   // Passes of one launch: a progressive render's small ones go together, since the
   // serial chain of a launch's largest tree costs the same for one sample a pixel as
   // for many (mesh 256x256x16, depth 8, progressive: 22 ms pass by pass, 6 ms together).
+  // But one at a time where a caller can tell: a callback gets each pass as soon as it is
+  // traced, with the rays traced so far; a cancel takes effect after the pass it finds;
+  // and other requests wait for one pass.
+  const int most = j.on_pass || cancel_ || j.serving ? 1 : kMaxPassList;
   PassList passes;
   const std::uint32_t issued = j.issued;
-  while (j.issued < j.target && passes.n < kMaxPassList) {
+  while (j.issued < j.target && passes.n < most) {
     const std::uint32_t k = next_pass_size(j);
     const std::uint64_t count = j.pixels * k;
     if (passes.n && passes.samples() + count > kDirectSamples) break;
@@ -1017,39 +1021,31 @@ bool Engine::run_direct_passes(Job& j) {
   if (timed) CK(cudaEventRecord(W.tev[9], stream_));
   stats_.kernel_launches++;
   for (int k = 0; k < passes.n; ++k) W.rad_release(passes.seg[k].sample_base, passes.seg[k].count);
-  for (int p = 0; p < passes.n;) {
-    if (p > 0 && cancel_ && *cancel_) break;  // as between launches: the rest is dropped
-    // As in retire_segments: one by one where a callback may look.
-    PassList fold;
-    for (; fold.n < (j.on_pass ? 1 : passes.n); ++fold.n) fold.seg[fold.n] = passes.seg[p++];
-    CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, fold, W.wb.radiance, stream_));
-    stats_.kernel_launches++;
-    // Reported once it has run, so progress times are device-complete.
-    CK(cudaStreamSynchronize(stream_));
-    if (j.done == issued) {
-      if (timed) {
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
-        stats_.direct_ms += ms;
-      }
-      read_counters();
-      if (last_counters_.error)
-        throw CudaFailure("device error flag " + std::to_string(last_counters_.error) +
-                          (last_counters_.error == 2 ? " (direct integrator branch stack overflow)" : ""));
-    }
-    const WaveCounters& c = last_counters_;
-    for (int k = 0; k < fold.n; ++k) {
-      j.issued += fold.seg[k].pass_spp;
-      j.passes_issued++;
-      j.done += fold.seg[k].pass_spp;
-      j.prog.pass++;
-      j.prog.spp_done = j.done;
-      j.prog.finished = j.done >= j.target;
-      j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
-      j.prog.rays = (c.rays - base_counters_.rays) + (c.shadow_rays - base_counters_.shadow_rays);
-      stats_.passes++;
-      if (j.on_pass) j.on_pass(j.prog);
-    }
+  CK(launch_accumulate(W.jobs_dev + j.desc_slot, j.pixels, passes, W.wb.radiance, stream_));
+  stats_.kernel_launches++;
+  // Reported once it has run, so progress times are device-complete.
+  CK(cudaStreamSynchronize(stream_));
+  if (timed) {
+    float ms = 0;
+    CK(cudaEventElapsedTime(&ms, W.tev[8], W.tev[9]));
+    stats_.direct_ms += ms;
+  }
+  read_counters();
+  const WaveCounters& c = last_counters_;
+  if (c.error)
+    throw CudaFailure("device error flag " + std::to_string(c.error) +
+                      (c.error == 2 ? " (direct integrator branch stack overflow)" : ""));
+  for (int k = 0; k < passes.n; ++k) {
+    j.issued += passes.seg[k].pass_spp;
+    j.passes_issued++;
+    j.done += passes.seg[k].pass_spp;
+    j.prog.pass++;
+    j.prog.spp_done = j.done;
+    j.prog.finished = j.done >= j.target;
+    j.prog.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - j.t0).count();
+    j.prog.rays = (c.rays - base_counters_.rays) + (c.shadow_rays - base_counters_.shadow_rays);
+    stats_.passes++;
+    if (j.on_pass) j.on_pass(j.prog);
   }
   return true;
 }
