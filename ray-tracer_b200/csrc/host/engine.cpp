@@ -77,14 +77,20 @@ constexpr std::size_t kStagePiece = std::size_t(1) << 20;  // batch upload: byte
 constexpr int kJobSlots = 4096;  // job descriptors resident at once
 // Paths of one iteration. A render's iterations take four pools, since every iteration
 // ends with a wait for its slowest warps (0.03 ms on the sphere field, 0.1 ms on the
-// mix, 0.2 ms on the mesh). While requests are open they take half a pool (or a pool of
-// up to 2^20, whose iterations are short), so that a preview waits less for its turn:
-// with 8,388,608 paths, half a pool serves 3573 Msamples/s with previews at 7.7 ms
-// (median) and 15 ms (p99), a whole one 3687 at 13 and 22.5 ms, a third 3446 at 6.2 and
-// 13 ms.
+// mix, 0.2 ms on the mesh). While someone waits for them they take half a pool (or a pool
+// of up to 2^20, whose iterations are short): requests are open, or the render has a
+// callback or a cancel word, which are looked after between iterations.
+// - Requests, with 8,388,608 paths: half a pool serves 3573 Msamples/s with previews at
+//   7.7 ms (median) and 15 ms (p99), a whole one 3687 at 13 and 22.5 ms, a third 3446 at
+//   6.2 and 13 ms.
+// - A watched render of the mesh, 1024x1024x64, with 8,388,608 paths: half a pool takes
+//   53.2 ms and returns 8.0 ms (median) after a cancel, a whole one 51.5 and 11.9 ms, a
+//   third 54.6 and 5.0 ms, four 50.1 and 25 ms and more; progressive, the first pass is
+//   seen after 6.8 ms (50 with four pools). With 2^20 paths: 63 ms and 1.3 ms (four: 53
+//   and 11 ms).
 constexpr std::uint32_t kRenderPools = 4;
-std::uint32_t iteration_paths(std::uint32_t pool, bool serving) {
-  return serving ? std::min(pool, std::max(1u << 20, pool / 2)) : pool * kRenderPools;
+std::uint32_t iteration_paths(std::uint32_t pool, bool awaited) {
+  return awaited ? std::min(pool, std::max(1u << 20, pool / 2)) : pool * kRenderPools;
 }
 constexpr std::uint64_t kDirectSamples = std::uint64_t(1) << 22;  // of the passes the direct integrator traces together
 
@@ -1059,7 +1065,7 @@ void Engine::refill() {
     if (!s.used || s.complete || s.abandoned) continue;
     backlog[jobs_.at(s.job).priority] += s.d.count - std::min<std::uint64_t>(s.done, s.d.count);
   }
-  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 ? 1u : kRenderPools);
+  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 || watched_ ? 1u : kRenderPools);
   while (true) {
     Job* best = nullptr;
     for (auto& kv : jobs_) {
@@ -1199,7 +1205,7 @@ void Engine::launch_one_iteration(bool look) {
   const int par = static_cast<int>(W.it & 1);
   const int r = static_cast<int>(W.it % kRing);
   const bool timed = cfg_.time_kernels;
-  W.wb.capacity = iteration_paths(cfg_.pool_paths, serve_open_ > 0);
+  W.wb.capacity = iteration_paths(cfg_.pool_paths, serve_open_ > 0 || watched_);
   LaunchShape shape = cfg_.shape;
   shape.mis = mis_jobs_ > 0;
   shape.general = cfg_.count_traversal || brute_jobs_ > 0 || shape.closest_tree == 8 || shape.shadow_tree == 8;
@@ -1249,11 +1255,14 @@ void Engine::drain(const volatile std::int32_t* cancel, std::vector<PassEvent>* 
       W.ungenerated = W.left = 0;
       return;
     }
-    launch_one_iteration(false);
+    // A watched render looks at every iteration as soon as the next one starts, which
+    // leaves one queued behind it and not two (a cancel of the mesh render above returns
+    // after 12.4 ms otherwise).
+    launch_one_iteration(watched_);
     // Nothing to run ahead of: look at once instead of two empty iterations later.
     const bool idle_next = W.ungenerated == 0 && W.left == 0;
     if (idle_next) launch_one_iteration(true);
-    const std::uint64_t lag = idle_next ? 0 : kLag;
+    const std::uint64_t lag = idle_next || watched_ ? 0 : kLag;
     while (W.seen + lag < W.it) process_snapshot(W.seen++, events);
     if (return_on_event && events && events->size() > events0) return;
     if (budget_ms < std::numeric_limits<double>::infinity() &&
@@ -1353,14 +1362,15 @@ std::vector<RenderProgress> Engine::render_batch(const std::vector<BatchJob>& ba
   // Job by job, an iteration's warps share fewer scenes' nodes, and a job's passes finish
   // together and are folded together: the 64-scene mix takes 436.7 ms on the device
   // (449.3 pass by pass; of that accumulate 10.1 and 15.6), 16 of its scenes 110.7 (112.7).
-  job_order_ = !cancel && !on_pass;
+  watched_ = cancel || on_pass;
+  job_order_ = !watched_;
   bool cancelled = false;
   try {
     drain(cancel, nullptr, std::numeric_limits<double>::infinity(), false);
     cancelled = cancel && *cancel && !all_jobs_drained();
-    job_order_ = false;
+    job_order_ = watched_ = false;
   } catch (...) {
-    job_order_ = false;
+    job_order_ = watched_ = false;
     rendering_.clear();
     abort_all();
     for (int h : handles) {

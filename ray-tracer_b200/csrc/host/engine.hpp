@@ -354,6 +354,7 @@ class Engine {
   // Jobs one after the other instead of pass by pass: a batch of which nothing can be seen
   // before its end (no callback, no cancel word).
   bool job_order_ = false;
+  bool watched_ = false;           // the render in progress has a callback or a cancel word
   std::vector<RenderSettings> frame_settings_;
   RenderStats stats_;
   std::map<int, Job> jobs_;        // open jobs by handle
