@@ -77,21 +77,19 @@ constexpr std::size_t kStagePiece = std::size_t(1) << 20;  // batch upload: byte
 constexpr int kJobSlots = 4096;  // job descriptors resident at once
 // Paths of one iteration. A render's iterations take four pools, since every iteration
 // ends with a wait for its slowest warps (0.03 ms on the sphere field, 0.1 ms on the
-// mix, 0.2 ms on the mesh). While someone waits for them they take half a pool (or a pool
-// of up to 2^20, whose iterations are short): requests are open, or the render has a
-// callback or a cancel word, which are looked after between iterations.
-// - Requests, with 8,388,608 paths: half a pool serves 3573 Msamples/s with previews at
-//   7.7 ms (median) and 15 ms (p99), a whole one 3687 at 13 and 22.5 ms, a third 3446 at
-//   6.2 and 13 ms.
-// - A watched render of the mesh, 1024x1024x64, with 8,388,608 paths: half a pool takes
-//   53.2 ms and returns 8.0 ms (median) after a cancel, a whole one 51.5 and 11.9 ms, a
-//   third 54.6 and 5.0 ms, four 50.1 and 25 ms and more; progressive, the first pass is
-//   seen after 6.8 ms (50 with four pools). With 2^20 paths: 63 ms and 1.3 ms (four: 53
-//   and 11 ms).
+// mix, 0.2 ms on the mesh). Shorter where someone waits for their end:
+// - While requests are open they take half a pool (or a pool of up to 2^20, whose
+//   iterations are short), so that a preview waits less for its turn. With 8,388,608
+//   paths, half a pool serves 3573 Msamples/s with previews at 7.7 ms (median) and 15 ms
+//   (p99), a whole one 3687 at 13 and 22.5 ms, a third 3446 at 6.2 and 13 ms.
+// - A render with a callback or a cancel word, which are looked after between iterations,
+//   takes half a pool or 2^20 paths, whichever is more. The mesh, 1024x1024x64, with
+//   8,388,608 paths: half a pool takes 53.2 ms and returns 8.0 ms (median) after a cancel,
+//   a whole one 51.5 and 11.9 ms, a third 54.6 and 5.0 ms, four 50.1 and 25 ms and more;
+//   progressive, the first pass is seen after 6.8 ms (50 with four pools). With 1,048,576:
+//   63 ms and 1.3 ms (four: 53 and 11 ms).
 constexpr std::uint32_t kRenderPools = 4;
-std::uint32_t iteration_paths(std::uint32_t pool, bool awaited) {
-  return awaited ? std::min(pool, std::max(1u << 20, pool / 2)) : pool * kRenderPools;
-}
+constexpr std::uint32_t kShortIteration = 1u << 20;
 constexpr std::uint64_t kDirectSamples = std::uint64_t(1) << 22;  // of the passes the direct integrator traces together
 
 }  // namespace
@@ -1065,7 +1063,7 @@ void Engine::refill() {
     if (!s.used || s.complete || s.abandoned) continue;
     backlog[jobs_.at(s.job).priority] += s.d.count - std::min<std::uint64_t>(s.done, s.d.count);
   }
-  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * cfg_.pool_paths * (serve_open_ > 0 || watched_ ? 1u : kRenderPools);
+  const std::uint64_t target = std::uint64_t(cfg_.backlog_pools) * std::max(cfg_.pool_paths, iteration_size());
   while (true) {
     Job* best = nullptr;
     for (auto& kv : jobs_) {
@@ -1198,6 +1196,11 @@ void Engine::process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events
   for (auto& kv : jobs_) retire_segments(kv.second, events);
 }
 
+std::uint32_t Engine::iteration_size() const {
+  const std::uint32_t pool = cfg_.pool_paths, most = serve_open_ > 0 ? pool : pool * kRenderPools;
+  return serve_open_ > 0 || watched_ ? std::min(most, std::max(kShortIteration, pool / 2)) : most;
+}
+
 void Engine::launch_one_iteration(bool look) {
   Wave& W = *wave_;
   counters_final_ = false;
@@ -1205,7 +1208,7 @@ void Engine::launch_one_iteration(bool look) {
   const int par = static_cast<int>(W.it & 1);
   const int r = static_cast<int>(W.it % kRing);
   const bool timed = cfg_.time_kernels;
-  W.wb.capacity = iteration_paths(cfg_.pool_paths, serve_open_ > 0 || watched_);
+  W.wb.capacity = iteration_size();
   LaunchShape shape = cfg_.shape;
   shape.mis = mis_jobs_ > 0;
   shape.general = cfg_.count_traversal || brute_jobs_ > 0 || shape.closest_tree == 8 || shape.shadow_tree == 8;

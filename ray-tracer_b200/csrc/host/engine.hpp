@@ -294,6 +294,7 @@ class Engine {
   bool run_direct_passes(Job& j);   // false if no radiance space is free now
   void process_snapshot(std::uint64_t iter, std::vector<PassEvent>* events);
   void retire_segments(Job& j, std::vector<PassEvent>* events);
+  std::uint32_t iteration_size() const;  // paths of the next iteration
   void launch_one_iteration(bool look);  // look: its snapshot is waited for at once
   void drain(const volatile std::int32_t* cancel, std::vector<PassEvent>* events, double budget_ms,
              bool return_on_event);

@@ -1,5 +1,6 @@
-"""A render with a callback or a cancel word goes in iterations of at most a pool, with at most
-two of them under way when a cancel is seen, so that neither waits for long."""
+"""A render with a callback or a cancel word goes in iterations of at most 2^20 paths (half of a
+larger pool), with at most two of them under way when a cancel is seen, so that neither
+waits for long."""
 import ctypes as C
 import json
 
@@ -10,8 +11,8 @@ import workloads
 
 pytestmark = pytest.mark.gpu
 
-POOL, SIZE, SPP = 1 << 16, 512, 16
-PASS = SIZE * SIZE  # samples of the first pass: four pools
+POOL, SIZE, SPP = 1 << 20, 1024, 16
+PASS = SIZE * SIZE  # samples of the first pass: an iteration's
 
 
 @pytest.fixture
@@ -28,7 +29,7 @@ def render(ctx):
 
 
 @pytest.mark.parametrize("how", ["callback", "cancel word", "both"])
-def test_iterations_take_a_pool(ctx, render, how):
+def test_iterations_are_short(ctx, render, how):
     render()
     plain = [x.tobytes() for x in ctx.framebuffer_moments(-1, SIZE, SIZE)]
     seen = []
@@ -41,7 +42,10 @@ def test_iterations_take_a_pool(ctx, render, how):
 
 def test_a_cancel_leaves_little_behind(ctx, render):
     """The callback's progress has the rays of the iterations before the one under way. That one ends, and at most
-    one queued behind it; a path of so small a pool is traced once or twice in an iteration."""
+    one queued behind it; together they trace the rays of 2 x 2^20 samples, or a few more where paths are left over."""
+    render()
+    st = ctx.stats()
+    rays_a_sample = (st["rays"] + st["shadow_rays"]) / (PASS * SPP)
     cancel, seen = C.c_int32(0), []
 
     def stop(p):
@@ -49,6 +53,6 @@ def test_a_cancel_leaves_little_behind(ctx, render):
         seen.append(p.rays)
 
     p = render(stop, cancel)
-    assert p.cancelled and p.spp_done == 1
+    assert p.cancelled and 1 <= p.spp_done < SPP
     st = ctx.stats()
-    assert 0 <= st["rays"] + st["shadow_rays"] - seen[0] <= 4 * POOL
+    assert 0 <= st["rays"] + st["shadow_rays"] - seen[0] <= 2.2 * POOL * rays_a_sample
