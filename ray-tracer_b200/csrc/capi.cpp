@@ -525,8 +525,6 @@ int rtg_scene_get_info(rtg_context* ctx, rtg_scene_id scene, rtg_scene_info* out
     out->device_bytes = g.device_bytes;
     out->bvh_build_ms = b.build_ms;
     out->bvh_sah_cost = b.sah_cost;
-    if (g.host_stats)  // the GPU build does not add the cost up; it has the host tree's
-      if (const rtg::BinaryBvh* tree = rtg::host_tree(*g.host, true)) out->bvh_sah_cost = tree->stats.sah_cost;
     return RTG_OK;
   });
 }

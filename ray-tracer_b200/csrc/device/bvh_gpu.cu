@@ -1609,6 +1609,16 @@ __global__ void k_emit_nodes(EmitArgs a) {
   if (at >= 0 && at < a.t.counters->interior) a.nodes[at] = d;
 }
 
+// BinaryBvh::build's cost terms (host/bvh_build.cpp), a node's at its depth-first index.
+__global__ void k_node_costs(TreeArgs t, int n, double* out) {
+  const int id = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+  if (id >= n) return;
+  const double root = box_area(t.box, t.box + 3), area = box_area(t.box + 6ll * id, t.box + 6ll * id + 3);
+  const double term = area / (root < 1e-30 ? 1e-30 : root) * (t.left[id] < 0 ? double(t.count[id]) : 1.0);
+  const int at = t.dfs[id];
+  if (at >= 0 && at < n) out[at] = term;
+}
+
 // Slots in leaf order, gathered from the per-primitive records.
 __global__ void k_emit_slots(EmitArgs a, std::uint32_t n) {
   const std::uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1750,6 +1760,7 @@ void gpu_bvh_preload() {
   cudaFuncAttributes a;
   const void* kernels[] = {
       reinterpret_cast<const void*>(k_convert),    reinterpret_cast<const void*>(k_init),
+      reinterpret_cast<const void*>(k_node_costs),
       reinterpret_cast<const void*>(k_bounds),
       reinterpret_cast<const void*>(k_bins),       reinterpret_cast<const void*>(k_decide),
       reinterpret_cast<const void*>(k_pcount),     reinterpret_cast<const void*>(k_pscan),
@@ -2088,6 +2099,17 @@ void GpuBvhBuilder::emit(const GpuBvhInput& in, DevNode* nodes, DevNode4* nodes4
   if (counts_.interior > 0) k_emit_nodes<<<blocks_for(counts_.nodes, 256), 256, 0, stream_>>>(e);
   k_emit_slots<<<blocks_for(s.n, 256), 256, 0, stream_>>>(e, s.n);
   if (counts_.wide > 0) k_emit_wide<<<blocks_for(counts_.wide, 256), 256, 0, stream_>>>(e, counts_.wide);
+  BVH_CK(cudaGetLastError());
+}
+
+void GpuBvhBuilder::node_costs(double* out) {
+  if (!st_ || counts_.nodes == 0) return;
+  TreeArgs t{};
+  t.box = st_->box;
+  t.left = st_->left;
+  t.count = st_->count;
+  t.dfs = st_->dfs;
+  k_node_costs<<<blocks_for(counts_.nodes, 256), 256, 0, stream_>>>(t, counts_.nodes, out);
   BVH_CK(cudaGetLastError());
 }
 

@@ -86,8 +86,9 @@ class GpuBvhBuilder {
   GpuBvhBuilder(const GpuBvhBuilder&) = delete;
   GpuBvhBuilder& operator=(const GpuBvhBuilder&) = delete;
 
-  // Builds the tree and its four-wide collapse; synchronises the stream a few times. Throws std::runtime_error on a leaf of
-  // more than 65535 primitives or a tree deeper than the traversal stack allows.
+  // Builds the tree and its four-wide collapse; synchronises the stream a few times.
+  // Throws std::runtime_error on a leaf of more than 65535 primitives or a tree deeper
+  // than the traversal stack allows.
   GpuBvhCounts build(const GpuBvhInput& in);
 
   // Writes the device layout: counts.interior nodes, counts.wide four-wide nodes
@@ -95,6 +96,11 @@ class GpuBvhBuilder {
   // order = slot -> primitive id). Stream-ordered; no synchronisation.
   void emit(const GpuBvhInput& in, DevNode* nodes, DevNode4* nodes4, float4* prims, std::uint32_t* slot_material,
             float4* slot_normals, std::uint32_t* order);
+
+  // Each node's share of the tree's SAH cost, in depth-first order (counts.nodes
+  // doubles): summed in that order, they give BvhStats::sah_cost as the host build has
+  // it. Stream-ordered; no synchronisation.
+  void node_costs(double* out);
 
  private:
   void* alloc(std::size_t bytes);

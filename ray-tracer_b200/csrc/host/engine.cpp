@@ -236,9 +236,9 @@ void Engine::reset_wave() {
 int Engine::add_scene(std::shared_ptr<const CompiledScene> scene) {
   if (!scene->bvh_built) {
     if (scene->prims.size() >= kGpuBuildMinPrims) {
-      const int id = add_scene_gpu_bvh(std::move(scene));
-      scenes_.at(id)->host_stats = true;
-      return id;
+      // Its information is the same as with a host-built tree, up to where it always was.
+      const bool with_cost = scene->prims.size() < kHostTreePrims;
+      return add_scene_gpu_bvh(std::move(scene), with_cost);
     }
     // Small scene: the host builds the same tree faster than the GPU build's
     // level-by-level passes can start and finish.
@@ -440,7 +440,7 @@ unsigned char* Engine::upload_staging(std::size_t bytes, int& b, int want) {
   return upload_host_[b];
 }
 
-int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
+int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene, bool with_cost) {
   CK(cudaSetDevice(device_));
   const CompiledScene& s = *scene;
   if (s.prims.size() > kIdMask) throw std::runtime_error("too many primitives for the device layout");
@@ -564,12 +564,13 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
   // The layout in the binary tree's leaf order, in scratch first: the
   // eight-wide tree is built from it on the host (the same function as for a
   // host-built scene, so the bytes agree) and sets the final slot order.
-  const std::size_t scratch_bytes[7] = {std::size_t(c.interior) * sizeof(DevNode), std::size_t(c.wide) * sizeof(DevNode4),
+  const std::size_t cost_bytes = with_cost ? static_cast<std::size_t>(c.nodes) * sizeof(double) : 0;
+  const std::size_t scratch_bytes[8] = {std::size_t(c.interior) * sizeof(DevNode), std::size_t(c.wide) * sizeof(DevNode4),
                                         std::size_t(n_items) * 3 * sizeof(float4), std::size_t(n_items) * sizeof(std::uint32_t),
                                         std::size_t(n_items) * 3 * sizeof(float4), std::size_t(n_items) * sizeof(std::uint32_t),
-                                        std::size_t(n_items) * sizeof(std::uint32_t)};
-  std::size_t sat[7], scratch_total = 0;
-  for (int k = 0; k < 7; ++k) {
+                                        std::size_t(n_items) * sizeof(std::uint32_t), cost_bytes};
+  std::size_t sat[8], scratch_total = 0;
+  for (int k = 0; k < 8; ++k) {
     sat[k] = scratch_total;
     scratch_total += pad(scratch_bytes[k]);
   }
@@ -590,6 +591,13 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
   auto* s_old_of = reinterpret_cast<std::uint32_t*>(sb + sat[5]);
   auto* s_new_of = reinterpret_cast<std::uint32_t*>(sb + sat[6]);
   builder.emit(in, s_nodes, s_nodes4, s_prims, s_material, s_normals, order);
+  static_assert(2 * kHostTreePrims * sizeof(double) <= kSlotBytes, "a node's cost each fits a slot");
+  const double* costs = nullptr;
+  if (cost_bytes) {
+    costs = reinterpret_cast<const double*>(slot(0).mem);
+    builder.node_costs(reinterpret_cast<double*>(sb + sat[7]));
+    CK(cudaMemcpyAsync(slot(0).mem, sb + sat[7], cost_bytes, cudaMemcpyDeviceToHost, build_stream_));
+  }
   const bool want8 = wants_wide8();
   std::vector<DevNode> bin_nodes;
   std::vector<std::uint32_t> row0_w, prim_of_slot(n_items);
@@ -694,6 +702,7 @@ int Engine::add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene) {
   gs->bvh.max_depth = static_cast<std::size_t>(c.max_depth);
   gs->bvh.max_leaf = static_cast<std::size_t>(c.max_leaf);
   gs->bvh.build_ms = c.build_ms;
+  for (std::size_t k = 0; costs && k < gs->bvh.nodes; ++k) gs->bvh.sah_cost += costs[k];
   gs->device_built = true;
   free_block.p = nullptr;
   gs->host = std::move(scene);

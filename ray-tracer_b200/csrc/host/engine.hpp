@@ -92,7 +92,6 @@ struct GpuScene {
   int jobs_open = 0;           // jobs in the wavefront that use this scene
   BvhStats bvh;                // of the tree on the device (host or device build)
   bool device_built = false;   // the BVH was built on the GPU
-  bool host_stats = false;     // ... because the scene is large enough, not by request
 };
 
 // Per-job device framebuffer.
@@ -151,8 +150,9 @@ class Engine {
   // is the same.
   int add_scene(std::shared_ptr<const CompiledScene> scene);
   // Builds the scene's BVH on the GPU (device/bvh_gpu.h), whether or not the host
-  // compile holds one, and derives the device layout there.
-  int add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene);
+  // compile holds one, and derives the device layout there. with_cost: adds up the tree's
+  // SAH cost too (scenes of under kHostTreePrims primitives).
+  int add_scene_gpu_bvh(std::shared_ptr<const CompiledScene> scene, bool with_cost = false);
   // Several scenes at once: flattened in parallel on the host, then copied.
   std::vector<int> add_scenes(const std::vector<std::shared_ptr<const CompiledScene>>& scenes);
   void release_scene(int id);
