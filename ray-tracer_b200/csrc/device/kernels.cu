@@ -634,8 +634,8 @@ __device__ __forceinline__ CameraSample listed_sample(const RtgSceneDev& J, cons
 // tree with a stack of pending refraction branches, which keeps the reference's RNG
 // draw order.
 //
-// Two kernels. From kDirectWarpSamples samples a launch up, k_direct schedules them like
-// the path kernel: each warp holds kDirectPaths samples in shared memory; `ready` ones
+// Two kernels. From kDirectWarpSamples samples a launch up, unless the branches below
+// have no memory, k_direct schedules them like the path kernel: each warp holds kDirectPaths samples in shared memory; `ready` ones
 // have a ray to trace, `lit` ones the next light of a diffuse hit to sample and test
 // (its surface is made again from the hit for each light, which costs less than
 // keeping it). Pending branches are in device memory: at most one per level, so
@@ -1245,8 +1245,9 @@ namespace {
 constexpr int kDirectBlock = 128;
 template <bool kGeneral>
 cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance,
-                                   WaveCounters* cnt, float4* pending, int pending_depth, int tree, cudaStream_t stream) {
-  if (passes.samples() < kDirectWarpSamples) {
+                                   WaveCounters* cnt, bool by_warp, float4* pending, int pending_depth, int tree,
+                                   cudaStream_t stream) {
+  if (!by_warp) {
     constexpr int kMaxPerSm = 2048 / kDirectBlock;
     static GridTable grids;
     const Grid grid = grids.get(k_direct_sample<kDirectBlock, kGeneral>, kDirectBlock, 0, kMaxPerSm);
@@ -1267,18 +1268,18 @@ cudaError_t launch_direct_instance(const RtgSceneDev* job_dev, const PassList& p
 }
 }  // namespace
 
-int direct_pending_depth(int max_depth, std::uint64_t samples) {
-  return samples < kDirectWarpSamples ? 0 : (max_depth < kDirectStack ? max_depth : kDirectStack);
-}
+bool direct_by_warp(std::uint64_t samples) { return samples >= kDirectWarpSamples; }
+
+int direct_pending_depth(int max_depth) { return max_depth < kDirectStack ? max_depth : kDirectStack; }
 
 std::size_t direct_pending_bytes(int sms, int pending_depth) {
   return static_cast<std::size_t>(sms) * (kPathThreads / 32) * kDirectPaths * pending_depth * kPendingRows * sizeof(float4);
 }
 
 cudaError_t launch_direct(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance, WaveCounters* cnt,
-                          float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream) {
-  return general ? launch_direct_instance<true>(job_dev, passes, radiance, cnt, pending, pending_depth, tree, stream)
-                 : launch_direct_instance<false>(job_dev, passes, radiance, cnt, pending, pending_depth, tree, stream);
+                          bool by_warp, float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream) {
+  return general ? launch_direct_instance<true>(job_dev, passes, radiance, cnt, by_warp, pending, pending_depth, tree, stream)
+                 : launch_direct_instance<false>(job_dev, passes, radiance, cnt, by_warp, pending, pending_depth, tree, stream);
 }
 
 cudaError_t launch_resolve(const double* fb_sum, const std::uint32_t* fb_count, std::uint64_t pixels, int tone_map,

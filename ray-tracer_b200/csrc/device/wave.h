@@ -56,14 +56,18 @@ cudaError_t launch_paths(const WaveBuffers& wb, int parity, const LaunchShape& s
 cudaError_t launch_accumulate(const RtgSceneDev* job_dev, std::uint64_t pixels, const PassList& passes,
                               const float4* radiance, cudaStream_t stream);
 
-// Direct (Whitted) integrator over whole passes. Writes each sample's radiance slot. `pending` holds direct_pending_bytes(SMs, pending_depth) bytes for the
-// samples' pending refraction branches, pending_depth of them a sample
-// (direct_pending_depth of the job's maximum depth and the passes' samples; 0 for a
-// scene without dielectrics, whose samples have none). `general`: an eight-wide walk (tree 8) or brute force.
-int direct_pending_depth(int max_depth, std::uint64_t samples);
+// Direct (Whitted) integrator over whole passes. Writes each sample's radiance slot.
+// `by_warp` takes the kernel that schedules samples by warps, which is the faster one
+// where direct_by_warp says so; else a thread traces a sample. The former's `pending`
+// holds direct_pending_bytes(SMs, pending_depth) bytes for the samples' pending refraction
+// branches, pending_depth of them a sample (direct_pending_depth of the job's maximum
+// depth; 0 for a scene without dielectrics, whose samples have none).
+// `general`: an eight-wide walk (tree 8) or brute force.
+bool direct_by_warp(std::uint64_t samples);
+int direct_pending_depth(int max_depth);
 std::size_t direct_pending_bytes(int sms, int pending_depth);
 cudaError_t launch_direct(const RtgSceneDev* job_dev, const PassList& passes, float4* radiance, WaveCounters* cnt,
-                          float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream);
+                          bool by_warp, float4* pending, int pending_depth, bool general, int tree, cudaStream_t stream);
 
 // Framebuffer means (mean_out, 3 doubles per pixel) and/or their tone-mapped
 // sRGB encoding (rgb8, 3 bytes per pixel), each 16-byte aligned, in device or pinned

@@ -123,8 +123,6 @@ struct Engine::Wave {
   std::uint32_t snapshot_slots = 0;
   std::uint32_t hi_slot = 0;           // segment slots ever used are below this
   int sms = 0;
-  float4* direct_pending = nullptr;    // pending branches of the direct integrator (grown on demand)
-  std::size_t direct_pending_bytes = 0;
   std::uint64_t stall = 0;             // snapshots without a finished sample while work is open
   std::uint64_t last_done_sum = 0;
 
@@ -222,7 +220,7 @@ void Engine::reset_wave() {
     for (int i = 0; i < 2; ++i) { dev_free(b.st_a[i]); dev_free(b.st_b[i]); dev_free(b.st_c[i]); dev_free(b.st_d[i]); dev_free(b.st_e[i]); }
     dev_free(b.radiance); dev_free(b.cnt);
     dev_free(wave_->jobs_dev); dev_free(wave_->segs_dev); dev_free(wave_->prog_dev);
-    dev_free(wave_->gen_dev); dev_free(wave_->plan_dev); dev_free(wave_->direct_pending);
+    dev_free(wave_->gen_dev); dev_free(wave_->plan_dev);
     if (wave_->ring) cudaFreeHost(wave_->ring);
     if (wave_->staging) cudaFreeHost(wave_->staging);
     for (auto& e : wave_->plan_ev) if (e) cudaEventDestroy(e);
@@ -1014,22 +1012,39 @@ bool Engine::run_direct_passes(Job& j) {
   }
   j.issued = issued;  // counted pass by pass below
   if (!passes.n) return false;  // retried once radiance space frees up
+  // The kernel that schedules samples by warps keeps their pending branches in device
+  // memory (9.5 MB a level of depth, 458 MB at most): from the pool, for this launch only.
+  // Requests have admission by footprint, which does not count that memory, and go
+  // without it, as a render does that cannot get it: a thread a sample, 1.1 to 1.3 times
+  // slower in launches this large.
+  bool by_warp = !j.serving && direct_by_warp(passes.samples());
+  struct Branches {
+    float4* mem = nullptr;
+    cudaStream_t s;
+    ~Branches() {
+      if (mem) cudaFreeAsync(mem, s);
+    }
+  } pending{nullptr, stream_};
   int pending_depth = 0;
-  for (const Material& m : scene(j.scene_id).host->materials)
-    if (std::holds_alternative<Dielectric>(m))
-      pending_depth = direct_pending_depth(j.settings.max_depth, passes.samples());
-  const std::size_t pending_bytes = direct_pending_bytes(W.sms, pending_depth);
-  if (W.direct_pending_bytes < pending_bytes) {
-    CK(cudaStreamSynchronize(stream_));
-    dev_free(W.direct_pending);
-    W.direct_pending = nullptr;
-    W.direct_pending_bytes = 0;
-    W.direct_pending = dev_alloc<float4>(pending_bytes / sizeof(float4));
-    W.direct_pending_bytes = pending_bytes;
+  if (by_warp)
+    for (const Material& m : scene(j.scene_id).host->materials)
+      if (std::holds_alternative<Dielectric>(m)) pending_depth = direct_pending_depth(j.settings.max_depth);
+  if (pending_depth > 0) {
+    void* mem = nullptr;
+    count_allocation();
+    const cudaError_t e = cudaMallocFromPoolAsync(&mem, direct_pending_bytes(W.sms, pending_depth), pool_, stream_);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      by_warp = false;
+      pending_depth = 0;
+    } else {
+      CK(e);
+    }
+    pending.mem = static_cast<float4*>(mem);
   }
   const bool timed = cfg_.time_kernels;
   if (timed) CK(cudaEventRecord(W.tev[8], stream_));
-  CK(launch_direct(W.jobs_dev + j.desc_slot, passes, W.wb.radiance, W.wb.cnt, W.direct_pending, pending_depth,
+  CK(launch_direct(W.jobs_dev + j.desc_slot, passes, W.wb.radiance, W.wb.cnt, by_warp, pending.mem, pending_depth,
                    !j.settings.use_bvh || cfg_.shape.closest_tree == 8, cfg_.shape.closest_tree, stream_));
   if (timed) CK(cudaEventRecord(W.tev[9], stream_));
   stats_.kernel_launches++;
