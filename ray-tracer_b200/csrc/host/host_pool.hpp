@@ -10,6 +10,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -96,7 +97,11 @@ class HostPool {
     if (!threads_.empty()) return;
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
     const unsigned workers = std::min(7u, cores > 1 ? cores - 1 : 0u);
-    for (unsigned w = 0; w < workers; ++w) threads_.emplace_back([this] { work(); });
+    try {
+      for (unsigned w = 0; w < workers; ++w) threads_.emplace_back([this] { work(); });
+    } catch (const std::system_error&) {
+      // No more threads to be had: those there are, or the caller alone, do the work.
+    }
   }
   void work() {
     std::size_t seen = 0;
