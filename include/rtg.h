@@ -70,7 +70,7 @@ typedef struct rtg_progress {
 typedef struct rtg_stats {
   uint64_t camera_samples, rays, shadow_rays, rr_terminated, invalid_samples, passes;
   uint64_t iterations, node_visits, prim_tests, sphere_tests, extend_launches; /* closest-hit walks */
-  uint64_t shadow_node_visits, shadow_prim_tests, shadow_sphere_tests;         /* any-hit kernel */
+  uint64_t shadow_node_visits, shadow_prim_tests, shadow_sphere_tests;         /* any-hit walks */
   uint64_t kernel_launches; /* every kernel of this library launched by the render */
   double elapsed_ms;        /* host wall time of the render call */
   double device_ms;         /* CUDA-event time on the context's stream, first to last launch */
@@ -120,13 +120,14 @@ int rtg_compile(const char* scene_json, const char* base_dir, rtg_host_scene** o
  * compile (Bvh::build, src/geometry/bvh.cpp:133-163, is skipped; the view below
  * then has no nodes): rtg_scene_upload builds the same tree at upload, on the GPU
  * for scenes of 1,024 primitives or more and on the host below that, where the
- * host is faster. */
+ * build takes a millisecond at most. */
 #define RTG_COMPILE_DEFER_BVH 1u
 /* RTG_COMPILE_AUTO_BVH: the compile builds the tree itself for scenes under 1,024
  * primitives and defers it to the GPU build for larger ones, so the host work stays
- * on the compiling thread (not on the thread that uploads). The view and the host
- * layout of a deferred scene under 32,768 primitives still have the tree: it is
- * built on the host when one of them is first asked for. */
+ * on the compiling thread (not on the thread that uploads). The GPU build is part of
+ * every upload: a scene that is uploaded again and again is better compiled with its
+ * tree. The view and the host layout of a deferred scene under 32,768 primitives still
+ * have the tree: it is built on the host when one of them is first asked for. */
 #define RTG_COMPILE_AUTO_BVH 2u
 int rtg_compile_flags(const char* scene_json, const char* base_dir, uint32_t flags, rtg_host_scene** out, char* err,
                       size_t err_cap);
@@ -230,7 +231,8 @@ int rtg_scene_release(rtg_context* ctx, rtg_scene_id scene);
 
 /* Blocking progressive render. `cancel` may be set to non-zero from any thread;
  * the render stops at the next wavefront iteration, drops the partial pass and
- * reports cancelled. `settings` may be NULL (use the scene's); `opts` may be NULL
+ * reports cancelled. With on_pass or cancel, iterations are kept short (rtg_tuning.pool_paths)
+ * and direct renders go pass by pass, so that neither waits for long. `settings` may be NULL (use the scene's); `opts` may be NULL
  * (progressive, 32). */
 int rtg_render(rtg_context* ctx, rtg_scene_id scene, const rtg_settings* settings, const rtg_render_options* opts,
                rtg_pass_fn on_pass, void* user, const volatile int32_t* cancel, rtg_progress* out);
@@ -304,8 +306,10 @@ int rtg_probe_read_bandwidth(rtg_context* ctx, uint64_t bytes, int32_t reps, int
 
 /* ---- engine tuning (no reference counterpart) ---- */
 typedef struct rtg_tuning {
-  uint32_t pool_paths;       /* a render's wavefront iterations trace up to four times as many paths, with
-                              * requests open half as many, or the whole pool up to 2^20 (default 1 << 20) */
+  uint32_t pool_paths;       /* a render's wavefront iterations trace up to four times as many paths (default
+                              * 1 << 20). Half as many, or 2^20 if that is more, in a render with a callback
+                              * or a cancel word; the same, but never more than the pool, while requests are
+                              * open */
   uint32_t block;            /* threads per block of the path kernel: 64, 128, 256 */
   uint64_t max_pass_samples; /* radiance slots shared by all passes in flight (default 1 << 27) */
   int32_t extend_blocks; /* grid of the path kernel; 0 = every resident block */

@@ -76,10 +76,13 @@ struct CompiledScene {
   BuildInfo info;
 };
 
-// Scenes from this many primitives up build their BVH faster on the GPU: its level
-// passes cost some 1.1 ms however few primitives they have (2.7 ms for 25k, 6.4 ms for
-// 174k, upload included), the host 1.2 to 1.6 us a primitive below 34k (2.5 ms for 2,053,
-// 38 ms for 25k), where it runs on one thread.
+// Scenes from this many primitives up build their BVH faster on the GPU, upload
+// included: 0.35 ms for 200 spheres, 0.48 for 1,000, 0.64 for 2,500, 1.7 for 32,000, 3.6
+// for 174k triangles. The host takes 1.0 to 1.6 us a primitive below 34k, where it runs on
+// one thread (0.27 ms for 200 with its upload, 1.05 for 1,000, 3.3 for 2,500, 52 for
+// 32,000). The two are equal at some 300 primitives. The line lies above that because
+// below it the build is the compile's, which may run on another thread, and there is at
+// most 0.6 ms to gain.
 constexpr std::size_t kGpuBuildMinPrims = 1024;
 // Scenes of fewer primitives than this that the rule above sends to the GPU still have
 // their tree where a caller asks for it on the host (host_tree).
