@@ -1511,6 +1511,9 @@ void Engine::reserve_pool(std::size_t bytes) {
     gpu_bvh_preload();
     bvh_preloaded_ = true;
   }
+  // The slots that reads go through: pinned allocations wait for the driver too (1 ms each,
+  // and on a busy host one in ten or so of 20 MB took 80 to 660 ms).
+  for (std::size_t k = 0; k < kSlots; ++k) slot(k);
   if (bytes <= pool_reserved_) return;
   void* p = nullptr;
   count_allocation();
