@@ -442,6 +442,11 @@ unsigned char* Engine::upload_staging(std::size_t bytes, int& b, int want) {
   if (upload_pending_[b]) CK(cudaEventSynchronize(upload_ev_[b]));
   upload_pending_[b] = false;
   if (upload_cap_[b] < bytes) {
+    // A quarter more than is asked for. Freeing and allocating pinned memory waits for the
+    // GPU and for the driver (12 ms for 20 MB, up to 660 on a busy host), and scenes of
+    // about one size, or one scene in its two forms (records for the GPU build, and
+    // flattened, which is some 15% more), should not do it again and again.
+    bytes += bytes / 4;
     if (upload_host_[b]) CK(cudaFreeHost(upload_host_[b]));
     upload_host_[b] = nullptr;
     upload_cap_[b] = 0;
