@@ -203,11 +203,13 @@ __device__ __forceinline__ float3 spawn_point(float3 p, float3 n) {
   const float3 near = kNearScale * n;  // exact: a power of two
   return f3(ulp_step(p.x, n.x, near.x), ulp_step(p.y, n.y, near.y), ulp_step(p.z, n.z, near.z));
 }
-// Spawn for direction `dir` from a surface with geometric normal `gn`.
+// Whether direction `dir` leaves a surface with geometric normal `gn` on that side. dot3p:
+// one in the surface's plane (total reflection's edge) leaves on the side that this form's
+// rounding says, as it always has.
+__device__ __forceinline__ bool leaves_outside(float3 gn, float3 dir) { return dot3p(dir, gn) > 0.f; }
+// Spawn for direction `dir` from there.
 __device__ __forceinline__ float3 spawn_towards(float3 p, float3 gn, float3 dir) {
-  // dot3p: a direction in the surface's plane (total reflection's edge) leaves on the side
-  // that this form's rounding says, as it always has.
-  return spawn_point(p, dot3p(dir, gn) > 0.f ? gn : -gn);
+  return spawn_point(p, leaves_outside(gn, dir) ? gn : -gn);
 }
 
 // The reference's shadow-ray shortening distance is 4 * 1.6e-6 * max(1, |p|inf)

@@ -224,14 +224,13 @@ constexpr std::uint32_t kMinBatch = 4;
 
 constexpr std::uint32_t kPathSpecular = 1u << 12;   // last bounce was specular (or the path is new)
 constexpr std::uint32_t kPathContinues = 1u << 13;  // goes on after its shadow ray
-constexpr std::uint32_t kPathApart = 1u << 14;      // its shadow ray has an origin of its own, in the radiance slot
 constexpr int kPathSegShift = 16;                   // low 12 bits: depth; 16 and up: segment slot
 static_assert(kMaxSegments <= 1 << 16, "the segment slot does not fit the path word");
 
 // One warp's path slots, one 4-byte column per field.
 template <bool kMis>
 struct alignas(16) WarpPaths {
-  float o[3][kWarpPaths];       // ray origin (and the shadow ray's, unless the path is marked kPathApart)
+  float o[3][kWarpPaths];       // ray origin (and the shadow ray's, unless sh_tmax is negative)
   float d[3][kWarpPaths];
   float beta[3][kWarpPaths];    // throughput
   float light[3][kWarpPaths];   // radiance so far
@@ -239,7 +238,7 @@ struct alignas(16) WarpPaths {
   std::uint32_t sample[kWarpPaths];  // radiance slot
   std::uint32_t meta[kWarpPaths];
   float sh_d[3][kWarpPaths];    // shadow ray direction, length, contribution
-  float sh_tmax[kWarpPaths];
+  float sh_tmax[kWarpPaths];    // negative: the shadow ray's origin is in the radiance slot
   float sh_c[3][kWarpPaths];
   float pdf[kMis ? kWarpPaths : 1];  // pdf of the last diffuse bounce
   std::uint16_t job[kWarpPaths];
@@ -367,9 +366,13 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
       on = lane < take;
       if (on) {
         p = S.lit[n_lit + lane];
-        o = S.meta[p] & kPathApart ? f3(wb.radiance[S.sample[p]]) : get3(S.o, p);
+        o = get3(S.o, p);
         d = get3(S.sh_d, p);
         tmax = S.sh_tmax[p];
+        if (tmax < 0.f) {
+          o = f3(wb.radiance[S.sample[p]]);
+          tmax = -tmax;
+        }
         job = S.job[p];
       }
     } else if (step == kBounce) {
@@ -492,9 +495,9 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
           if (scatter(m, d, s, rng, sr)) {
             // The next ray goes to shared memory before the light sample, which
             // needs the registers.
-            set3(S.o, p, spawn_towards(s.p, s.gn, sr.dir));
+            const bool outside = leaves_outside(s.gn, sr.dir);
+            set3(S.o, p, spawn_point(s.p, outside ? s.gn : -s.gn));
             set3(S.d, p, sr.dir);
-            std::uint32_t apart = 0;
             if (J.light_sampling && !sr.specular && J.n_lights > 0) {
               const std::uint32_t nl = static_cast<std::uint32_t>(J.n_lights);
               const LightSample ls = sample_light(J.lights + rng.below(nl), s, rng);
@@ -504,20 +507,19 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
                 if (!is_zero3(f) && !is_zero3(ls.li_over_pdf)) {
                   // Its origin is mostly the one stored above: a Lambertian scatter
                   // leaves, and lambert_cos is non-zero, on the side of s.gn. But
-                  // spawn_towards rounds in another way than those tests: of a direction
-                  // in the surface's plane it may find the other side. The origin
-                  // then waits in the radiance slot, which is written when the path ends.
+                  // leaves_outside rounds in another way than those tests: of a direction
+                  // in the surface's plane it may find the other side. The origin then
+                  // waits in the radiance slot, which is written when the path ends.
                   const ShadowRay sray = shadow_ray(s, ls);
-                  const float3 oo = get3(S.o, p);
-                  if (sray.o.x != oo.x || sray.o.y != oo.y || sray.o.z != oo.z) {
-                    apart = kPathApart;
+                  S.sh_tmax[p] = sray.tmax;
+                  if (leaves_outside(s.gn, ls.wi) != outside) {
+                    S.sh_tmax[p] = -sray.tmax;
                     wb.radiance[S.sample[p]] = make_float4(sray.o.x, sray.o.y, sray.o.z, 0.f);
                   }
                   float w = 1.f;  // a point light (pdf 0) cannot be hit by BSDF sampling
                   if (kMis && J.light_sampling == 2 && ls.pdf > 0.f)
                     w = power_heuristic(ls.pdf / static_cast<float>(nl), __fmul_rn(dot3(s.n, ls.wi), kInvPiF));
                   set3(S.sh_d, p, sray.d);
-                  S.sh_tmax[p] = sray.tmax;
                   set3(S.sh_c, p, get3(S.beta, p) * (f * ls.li_over_pdf) * __fmul_rn(static_cast<float>(nl), w));
                   shadow = true;
                 }
@@ -543,7 +545,7 @@ k_path(WaveBuffers wb, int par, int closest_tree, int shadow_tree) {
               // Cosine-hemisphere pdf of this bounce, for the MIS weight at the next hit.
               if (kMis && J.light_sampling == 2 && !sr.specular) S.pdf[kMis ? p : 0] = __fmul_rn(dot3p(s.n, sr.dir), kInvPiF);
             }
-            S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u) | apart;
+            S.meta[p] = (meta & ~0xFFFFu) | depth | (sr.specular ? kPathSpecular : 0u) | (cont ? kPathContinues : 0u);
           }
         }
       }
